@@ -233,58 +233,136 @@ __device__ __forceinline__ bool sphere_cube_rn(double px, double py, double pz, 
   return dmin <= r2;
 }
 
+// A node in cell order for the scan: its position relative to its cell's corner, in units of the
+// radius (FP32), and its index.
+struct __align__(16) ScanNode {
+  float x, y, z;
+  int id;
+};
+
+__global__ void k_scan_nodes(int n, const int* __restrict__ order, const int* __restrict__ hash,
+                             const double* __restrict__ x, const double* __restrict__ y,
+                             const double* __restrict__ z, double x0, double y0, double z0, double cx, double cy,
+                             double cz, int mx, int my, double inv_r, ScanNode* out) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int i = order[k], m = hash[i];
+    ScanNode v;
+    v.x = (float)((x[i] - (x0 + (double)(m % mx) * cx)) * inv_r);
+    v.y = (float)((y[i] - (y0 + (double)((m / mx) % my) * cy)) * inv_r);
+    v.z = (float)((z[i] - (z0 + (double)(m / mx / my) * cz)) * inv_r);
+    v.id = i;
+    out[k] = v;
+  }
+}
+
 // Warp per node.  Visits the cells within one cell of the sphere's bounding box in
 // ascending hash order, keeps those that pass the reference's sphere-cube test, and
 // appends the members of each (in the sorted order) that pass the horizon test, so the
 // list equals the reference's scan over all cells (grid.h:157-196).  Pass FILL=false
 // counts (lengths without self), FILL=true writes the CSR columns.
+//
+// Both tests are decided in FP32 on positions relative to the cells' corners in units of r,
+// where the squared distance is off by less than eps (see scan_eps): below 1 - eps a test
+// passes, above 1 + eps it fails, and only in between (or for a NaN) it is evaluated in FP64 with
+// the reference's rounding.  The tests of the ~4,000 candidates and 27-64 cells a node has with
+// the reference's cells of ten spacings are ~1,500 FP64 instructions a warp, which at 64 cycles
+// each took 53 ms a pass at 512k nodes; in FP32, four candidates a lane in flight and a cell a
+// lane, a pass takes 3.4 ms.  Nodes in cell order: the warps of a CTA scan the same cells.
 template <bool FILL>
 __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, double x0, double y0, double z0,
                             double cx, double cy, double cz, int mx, int my, int max_hash,
-                            double r, const int* __restrict__ start,
-                            const int* __restrict__ order, int max_node_no, int* len,
+                            double r, float eps, const int* __restrict__ start,
+                            const ScanNode* __restrict__ nodes, int max_node_no, int* len,
                             const int* __restrict__ row_ptr, int* cols, int* err) {
+  constexpr int U = 4;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const double r2 = __dmul_rn(r, r);
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+  const double r2 = __dmul_rn(r, r), inv_r = 1.0 / r;
+  const float wx = (float)(cx * inv_r), wy = (float)(cy * inv_r), wz = (float)(cz * inv_r);
+  const float in2 = 1.0f - eps, out2 = 1.0f + eps;
+  for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += warps) {
+    const int i = nodes[q].id;
     const double px = x[i], py = y[i], pz = z[i];
     int lo[3], hi[3];
-    const double q[3] = {px, py, pz}, o[3] = {x0, y0, z0}, w[3] = {cx, cy, cz};
+    const double qp[3] = {px, py, pz}, o[3] = {x0, y0, z0}, w[3] = {cx, cy, cz};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      lo[d] = (int)floor((q[d] - r - o[d]) / w[d]) - 1;
-      hi[d] = (int)floor((q[d] + r - o[d]) / w[d]) + 1;
+      lo[d] = (int)floor((qp[d] - r - o[d]) / w[d]) - 1;
+      hi[d] = (int)floor((qp[d] + r - o[d]) / w[d]) + 1;
       if (lo[d] < 0) lo[d] = 0;
     }
     if (hi[0] > mx - 1) hi[0] = mx - 1;
     if (hi[1] > my - 1) hi[1] = my - 1;
+    const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1;
+    // planes of cells up to max_hash
+    long long cells = 0;
+    if (nx > 0 && ny > 0 && hi[2] >= lo[2]) cells = (long long)nx * ny * (hi[2] - lo[2] + 1);
     int fill = 0;
     const int rbase = FILL ? row_ptr[i] : 0;
     const int cap = max_node_no - 1;
-    for (int kz = lo[2]; kz <= hi[2]; ++kz) {
-      const int mzo = mx * my * kz;
-      if (mzo >= max_hash) break;
-      for (int ky = lo[1]; ky <= hi[1]; ++ky)
-        for (int kx = lo[0]; kx <= hi[0]; ++kx) {
-          const int m = kx + mx * ky + mzo;
-          if (m >= max_hash) continue;
-          const double bx = __dadd_rn(x0, __dmul_rn((double)kx, cx));
-          const double by = __dadd_rn(y0, __dmul_rn((double)ky, cy));
-          const double bz = __dadd_rn(z0, __dmul_rn((double)kz, cz));
-          if (!sphere_cube_rn(px, py, pz, r2, bx, by, bz, cx, cy, cz)) continue;
-          const int s = start[m], e = start[m + 1];
-          for (int base = s; base < e; base += 32) {
-            const int k = base + lane;
+    for (long long c0 = 0; c0 < cells; c0 += 32) {
+      // a cell a lane, in ascending hash order
+      const long long c = c0 + lane;
+      int s = 0, e = 0;
+      float ax = 0.0f, ay = 0.0f, az = 0.0f;
+      long long mfirst = 0;
+      {
+        const int kz0 = lo[2] + (int)(c0 / nx / ny);
+        mfirst = (long long)mx * my * kz0;
+      }
+      if (mfirst >= max_hash) break;  // warp-uniform: this round's and all later cells lie beyond
+      if (c < cells) {
+        const int kx = lo[0] + (int)(c % nx), ky = lo[1] + (int)(c / nx % ny), kz = lo[2] + (int)(c / nx / ny);
+        const long long m = kx + (long long)mx * ky + (long long)mx * my * kz;
+        if (m < max_hash) {
+          s = start[m];
+          e = start[m + 1];
+          if (s < e) {
+            const double bx = __dadd_rn(x0, __dmul_rn((double)kx, cx));
+            const double by = __dadd_rn(y0, __dmul_rn((double)ky, cy));
+            const double bz = __dadd_rn(z0, __dmul_rn((double)kz, cz));
+            ax = (float)((px - bx) * inv_r);
+            ay = (float)((py - by) * inv_r);
+            az = (float)((pz - bz) * inv_r);
+            const float gx = fmaxf(fmaxf(-ax, ax - wx), 0.0f), gy = fmaxf(fmaxf(-ay, ay - wy), 0.0f),
+                        gz = fmaxf(fmaxf(-az, az - wz), 0.0f);
+            const float g2 = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+            bool touch = g2 < in2;
+            if (!touch && !(g2 > out2)) touch = sphere_cube_rn(px, py, pz, r2, bx, by, bz, cx, cy, cz);
+            if (!touch) e = s;
+          }
+        }
+      }
+      unsigned int todo = __ballot_sync(0xffffffffu, s < e);
+      while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int cs = __shfl_sync(0xffffffffu, s, l), ce = __shfl_sync(0xffffffffu, e, l);
+        const float cax = __shfl_sync(0xffffffffu, ax, l), cay = __shfl_sync(0xffffffffu, ay, l),
+                    caz = __shfl_sync(0xffffffffu, az, l);
+        for (int base = cs; base < ce; base += 32 * U) {
+          float4 v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int k = base + 32 * u + lane;
+            if (k < ce) v[u] = __ldg(reinterpret_cast<const float4*>(nodes) + k);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int k = base + 32 * u + lane;
             bool pass = false;
-            int cand = -1;
-            if (k < e) {
-              cand = order[k];
-              const double d2 = __dadd_rn(__dadd_rn(sqr_rn(__dsub_rn(px, x[cand])),
-                                                    sqr_rn(__dsub_rn(py, y[cand]))),
-                                          sqr_rn(__dsub_rn(pz, z[cand])));
-              pass = (d2 <= r2) && (cand != i);
+            const int cand = __float_as_int(v[u].w);
+            if (k < ce) {
+              const float dx = cax - v[u].x, dy = cay - v[u].y, dz = caz - v[u].z;
+              const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+              pass = d2 < in2;
+              if (!pass && !(d2 > out2)) {
+                const double e2 = __dadd_rn(__dadd_rn(sqr_rn(__dsub_rn(px, x[cand])), sqr_rn(__dsub_rn(py, y[cand]))),
+                                            sqr_rn(__dsub_rn(pz, z[cand])));
+                pass = e2 <= r2;
+              }
+              pass = pass && cand != i;
             }
             const unsigned int bal = __ballot_sync(0xffffffffu, pass);
             if (FILL && pass) {
@@ -294,6 +372,7 @@ __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* _
             fill += __popc(bal);
           }
         }
+      }
     }
     if (!FILL && lane == 0) {
       len[i] = fill;
@@ -474,6 +553,18 @@ nnpp_status check_hash_grid(const double bb[6], double cx, double cy, double cz,
   return NNPP_OK;
 }
 
+// Bound of the error of k_cell_scan's squared distances (units of r) near 1.  With cells of c
+// radii, the node's position relative to a visited cell's corner is at most 1 + 3 c, a
+// candidate's at most c, their difference is rounded once more: each coordinate is off by less
+// than u (3 + 7 c), u = 2^-24; 2 sqrt(3) of that, its square and the square sum's own three
+// roundings bound the squared distance's error (with a factor of about two to spare).  Large
+// cells make it exceed 1: every test is then the FP64 one.
+float scan_eps(double r, double cx, double cy, double cz) {
+  const double c = std::max(cx, std::max(cy, cz)) / r;
+  const double u = 1.0 / 16777216.0, d = u * (4.0 + 14.0 * c);
+  return (float)std::min(1e6, 4.0 * d + 4.0 * d * d + 16.0 * u);
+}
+
 int grid_for(long long n, int block, int cap = 152 * 16) {
   long long g = (n + block - 1) / block;
   if (g < 1) g = 1;
@@ -574,8 +665,13 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
     return set_error(NNPP_ERR_NOMEM, "scan buffers");
   NNPP_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
   const int warps_grid = grid_for((long long)N * 32, 256, 152 * 64);
+  DBuf<ScanNode> nodes;
+  if (!nodes.alloc(N)) return set_error(NNPP_ERR_NOMEM, "scan buffers");
+  k_scan_nodes<<<grid_for(N, 256), 256, 0, st>>>(N, order.get(), hash.get(), x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
+                                                 1.0 / r, nodes.get());
+  const float eps = scan_eps(r, cx, cy, cz);
   k_cell_scan<false><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
-                                                 max_hash, r, start.get(), order.get(),
+                                                 max_hash, r, eps, start.get(), nodes.get(),
                                                  max_node_no, len.get(), nullptr, nullptr,
                                                  err.get());
   NNPP_CUDA(cudaGetLastError());
@@ -590,7 +686,7 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
     return set_error(NNPP_ERR_UNSUPPORTED, "build: more than 2^31-1 bonds");
   if (!out.col.alloc(nnz > 0 ? nnz : 1)) return set_error(NNPP_ERR_NOMEM, "neighbour columns");
   k_cell_scan<true><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
-                                                max_hash, r, start.get(), order.get(),
+                                                max_hash, r, eps, start.get(), nodes.get(),
                                                 max_node_no, nullptr, out.ptr.get(),
                                                 out.col.get(), err.get());
   NNPP_CUDA(cudaGetLastError());

@@ -1,0 +1,47 @@
+"""The neighbour scan's FP32 decisions with their FP64 fallback: nodes exactly on the horizon
+(lattices of a spacing that FP64 holds, r a whole number of spacings: every tie is decided by the
+reference's FP64 test), cells much smaller and much larger than the radius (larger than about 10^5
+radii every test is the FP64 one) and flat extents, against the oracle's lists, order included."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu(nn):
+    if nn.device_count() < 1:
+        pytest.skip("no CUDA device")
+    return nn
+
+
+def _oracle_lists(nn, orc, nodes, r, cell):
+    N = nodes.shape[1]
+    inp = nn.synth(0, 4, 1)
+    o = orc.Oracle(inp["params"], nodes, np.ones(N, dtype=np.int32), -np.ones((5, N)), np.zeros((5, N)),
+                   np.zeros(N, dtype=np.int32))
+    ml = o.build_neighbours(1024, r, cell)
+    lengths, ptr, cols = o.clouds()
+    expect = -np.ones((N, 1024), dtype=np.int32)
+    for i in range(N):
+        expect[i, :lengths[i]] = cols[ptr[i]:ptr[i + 1]]
+    return ml, lengths, expect
+
+
+@pytest.mark.parametrize("shape,r_cells,cell_factor", [
+    ((11, 10, 9), 3.0, 3.25),       # ties, cells a little wider than the radius
+    ((11, 10, 9), 3.0, 0.5),        # ties, a dozen cells along the diameter
+    ((17, 31, 1), 2.0, 10.0),       # a flat extent
+    ((12, 11, 7), 3.0, 1.0e7),      # one cell: every test falls back to FP64
+])
+def test_scan_ties_and_cells(gpu, orc, shape, r_cells, cell_factor):
+    nn = gpu
+    dx = 0.125
+    g = np.stack(np.meshgrid(*[np.arange(n) for n in shape], indexing="ij")).reshape(3, -1).astype(np.float64) * dx
+    g = np.ascontiguousarray(g[:, np.random.default_rng(4).permutation(g.shape[1])])
+    cell = (cell_factor * dx, cell_factor * dx * 1.5, cell_factor * dx)
+    clouds, lengths, ml = nn.build_clouds_hash(1024, r_cells * dx, *cell, g)
+    ml_o, len_o, expect = _oracle_lists(nn, orc, g, r_cells * dx, cell)
+    assert ml == ml_o
+    assert np.array_equal(lengths, len_o)
+    assert np.array_equal(clouds, expect)
