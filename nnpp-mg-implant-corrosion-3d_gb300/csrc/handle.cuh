@@ -4,6 +4,7 @@
 
 #include <vector>
 
+#include "coarse_inverse.cuh"
 #include "common.cuh"
 #include "dbuf.cuh"
 #include "neighbours.cuh"
@@ -136,14 +137,20 @@ struct Coarse {
   DBuf<int> ap_col;   // A P off its diagonal term (27 N capacity, ap_k used): see KParams
   DBuf<float> ap_val;
   int ap_k = 1;
-  DBuf<float> rowabs; // n: row sums of |A_c| (Newton-Schulz scaling)
-  DBuf<float> a, t, x, y; // n x n: A_c and the Newton-Schulz work matrices
+  DBuf<float> rowabs; // n: row sums of |A_c| (Newton-Schulz scaling; -1: no unknown)
+  DBuf<float> st27;   // 27 n: A_c's rows, entry q the neighbour (q % 3, q / 3 % 3, q / 9) - 1
+  DBuf<unsigned int> tag, mask;  // N: the bond walk's node words, the aggregates a node's bonds reach
+  DBuf<float> dn;          // N: the sum of a node's liquid bonds
+  CoarseBlocks blocks;     // the direct inverse's work arrays
+  DBuf<float> x;           // n x n work matrix of either inverse
+  DBuf<float> a, t, y;     // n x n: A_c and the Newton-Schulz work matrices
   DBuf<double> nrm;        // block partials of ||I - A_c X_0||_F^2 (warm-started rebuilds)
   size_t inv_elems() const { return (size_t)n * ld; }
   DBuf<unsigned char> snap;  // N: phases (internal order) the inverse was computed from
   DBuf<int> count;           // phase changes since (coarse_check)
   void* cublas = nullptr;
   bool valid = false; // inv holds an inverse
+  bool ns_valid = false;  // inv came from the Newton-Schulz iteration (its warm start)
   bool stale = true;  // the phases changed since inv was computed
   long long rebuilds = 0;  // inverses computed since the handle was built
   long long warm_rebuilds = 0;  // of which Newton-Schulz started from the previous inverse
