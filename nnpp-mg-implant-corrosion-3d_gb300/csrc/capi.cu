@@ -350,6 +350,7 @@ nnpp_status nnpp_build_neighbours(nnpp_handle* hp, int max_node_no, double r, do
     h.engine = nullptr;
   }
   h.built = false;
+  h.implicit_work.reset();
   NNPP_TRY(build_ref_lists(h.st, h.N, h.ux.get(), h.uy.get(), h.uz.get(), max_node_no, r, cx, cy, cz,
                            order_mode, h.ref));
   h.max_node_no = max_node_no;
