@@ -40,6 +40,11 @@ namespace nnpp {
 namespace {
 
 constexpr int kSp = 10;  // species; field kSp is the potential
+// groups of 32 nodes below which four warps share a group's bonds (see k_residuals_grouped):
+// 152 SMs of 16 resident warps three times over.  Measured, four parts
+// against one (ms): 8k nodes 0.222 against 0.462, 64k 0.911 against 1.140; 262k (above the line)
+// 3.47 either way
+constexpr int kSplitGroups = 152 * 48;
 
 // The reference's parameter object from its data arrays (utils.h:2343-2484): data2 (51
 // values), per species k the datac_k array (z, D_solid, D_liquid, s_k1, s_k2, K_kprop1,
@@ -64,6 +69,10 @@ struct ChemParams {
   // not zero, q[0] / q[1] = the liquid-solid / solid-solid factor over sg
   double sg1[kSp], sg2[kSp], q1[2][kSp], q2[2][kSp];
   int on1[kSp], on2[kSp];
+  double rdt;               // 1 / dt, 0 where it is out of range
+  // k_residuals_grouped: beta = bc0 - rdx xi; rho of the charge groups; whether it applies
+  double rdx, bc0, rho[5];
+  int grouped;
 };
 
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
@@ -89,6 +98,104 @@ __device__ __forceinline__ double rpow(double rs, double xi, double e, int ie) {
     return p;
   }
   return dvd(1.0, pow(xi, e));
+}
+
+// a / dt: the quotient from the reciprocal and one correction by its remainder (three FP64
+// instructions against the two dozen of a division; the correction leaves it within a rounding
+// of the quotient), the division itself where dt's reciprocal is out of range
+__device__ __forceinline__ double over_dt(double a, const ChemParams& c) {
+  if (c.rdt == 0.0) return dvd(a, c.dt);
+  const double q = mul(a, c.rdt);
+  if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;  // infinite or NaN: no remainder
+  return fma(fma(-q, c.dt, a), c.rdt, q);
+}
+
+// The fields of node i from its bond sums (sums[k] = sum_KRk1 + sum_KRk2, s11 the potential's): the
+// time term, the reactions, the interface's H+ source and the potential's row.
+__device__ __forceinline__ void finish_node(const ChemParams& c, int N, int i, int pi, bool iface, bool flag,
+                                            const double (&sums)[kSp], double s11, const double* __restrict__ Un1,
+                                            const double* __restrict__ Un, double* __restrict__ F) {
+  const double phi_i = Un[(size_t)kSp * N + i];
+  double u1[kSp], u0[kSp];
+  // the fields' values at the node
+#pragma unroll
+  for (int k = 0; k < kSp; ++k) {
+    u1[k] = Un1[(size_t)k * N + i];
+    u0[k] = Un[(size_t)k * N + i];
+  }
+  const bool liq = pi == 0;
+  const bool act = iface || liq;  // solid nodes with a liquid neighbour, liquid nodes
+  double R[kSp];
+#pragma unroll
+  for (int k = 0; k < kSp; ++k) R[k] = 0.0;
+  // Mg (utils.h:162-174)
+  if (act) {
+    double t = mul(-c.k1b, pos(sub(mul(mul(u1[0], u0[2]), u0[2]), c.pMgOH2)));
+    t = sub(t, mul(c.k2b, pos(sub(mul(u1[0], u0[4]), c.pMgCO3))));
+    t = sub(t, mul(c.k3b, pos(sub(mul(u1[0], u0[4]), c.pMgHCO3))));
+    t = sub(t, mul(c.k4b, pos(sub(mul(mul(mul(mul(u0[0], u0[0]), u0[0]), u0[5]), u0[5]), c.pMgPO4))));
+    R[0] = t;
+  }
+  // H+ (utils.h:241-253): the interface's Butler-Volmer source, the liquid's equilibria
+  if (iface) {
+    const double phic = mul(dvd(mul(c.R, c.T), mul(c.F, c.z[0])), log(dvd(u0[0], dvd(c.CSat, c.CSolid))));
+    const double eta = sub(sub(add(c.phim, c.phimse), phi_i), phic);
+    R[1] = add(0.0, mul(dvd(c.JHp, mul(mul(c.z[1], c.F), c.CSolid)),
+                        exp(dvd(mul(mul(-c.alphaC, c.F), eta), mul(c.R, c.T)))));
+  } else if (liq) {
+    double t = mul(c.k7b, sub(c.pH2O, mul(u1[1], u0[2])));
+    t = add(t, mul(c.k8b, sub(c.pHCO3, mul(u1[1], u0[4]))));
+    t = add(t, mul(c.k9b, sub(c.pHPO4, mul(u1[1], u0[6]))));
+    R[1] = t;
+  }
+  // OH- (utils.h:321-330)
+  if (act) {
+    double t = mul(-c.k1b, pos(sub(mul(mul(u0[2], u0[2]), u0[0]), c.pMgOH2)));
+    t = sub(t, mul(c.k6b, pos(sub(ca5ohpo4(u1[2], u0[7], u0[6]), c.pCa5OHPO4))));
+    if (liq) t = add(t, mul(c.k7b, sub(c.pH2O, mul(u1[2], u0[1]))));
+    R[2] = t;
+  }
+  // species 4 (utils.h:396-401): the liquid's HCO3 equilibrium
+  if (liq) R[3] = mul(c.k8b, sub(c.pHCO3, mul(u1[3], u0[1])));
+  // species 5 (utils.h:466-476)
+  if (act) {
+    double t = mul(-c.k2b, pos(sub(mul(u1[4], u0[0]), c.pMgCO3)));
+    t = sub(t, mul(c.k3b, pos(sub(mul(u1[4], u0[0]), c.pMgHCO3))));
+    t = sub(t, mul(c.k5b, pos(sub(mul(u1[4], u0[7]), c.pCaCO3))));
+    if (liq) t = add(t, mul(c.k8b, sub(c.pHCO3, mul(u0[1], u1[4]))));
+    R[4] = t;
+  }
+  // species 6 (utils.h:541-547)
+  if (act) {
+    double t = mul(-c.k4b, pos(sub(mul(mul(mul(mul(u0[0], u0[0]), u0[0]), u0[5]), u0[5]), c.pMgPO4)));
+    if (liq) t = add(t, mul(c.k9b, add(-c.pHPO4, mul(u0[6], u0[1]))));
+    R[5] = t;
+  }
+  // species 7 (utils.h:612-618)
+  if (act) {
+    double t = mul(-c.k6b, pos(sub(ca5ohpo4(u0[2], u0[7], u0[6]), c.pCa5OHPO4)));
+    if (liq) t = add(t, mul(c.k9b, sub(c.pHPO4, mul(u1[6], u0[1]))));
+    R[6] = t;
+  }
+  // species 8 (utils.h:683-690)
+  if (act) {
+    double t = mul(-c.k5b, pos(sub(mul(u1[7], u0[4]), c.pCaCO3)));
+    t = sub(t, mul(c.k6b, pos(sub(ca5ohpo4(u0[2], u0[7], u0[6]), c.pCa5OHPO4))));
+    R[7] = t;
+  }
+#pragma unroll
+  for (int k = 0; k < kSp; ++k)
+    F[(size_t)k * N + i] = sub(add(over_dt(sub(u1[k], u0[k]), c), sums[k]), R[k]);
+  // potential (utils.h:801-841)
+  double f11 = 0.0;
+  if (flag) {
+    double r11 = mul(c.z[0], u0[0]);
+#pragma unroll
+    for (int k = 1; k < kSp; ++k) r11 = add(r11, mul(c.z[k], u0[k]));
+    const double inv = dvd(1.0, mul(c.K11, c.sigma1));
+    f11 = sub(mul(inv, s11), mul(mul(mul(inv, c.F), c.CSolid), r11));
+  }
+  F[(size_t)kSp * N + i] = f11;
 }
 
 template <bool kOneExp, bool kAllOn>
@@ -170,93 +277,125 @@ __global__ void k_residuals_full(ChemParams c, int N, const double* __restrict__
         flag = 1;
       }
     }
-    double s1[kSp], s2[kSp];
+    double sums[kSp];
 #pragma unroll
-    for (int k = 0; k < kSp; ++k) {
-      s1[k] = -mul(c.sg1[k], S1[k]);
-      s2[k] = -mul(c.sg2[k], S2[k]);
-    }
-    const double s11 = -mul(c.KS11, S11);
-    // the fields' values at the node
-    double u1[kSp], u0[kSp];
+    for (int k = 0; k < kSp; ++k) sums[k] = -add(mul(c.sg1[k], S1[k]), mul(c.sg2[k], S2[k]));
+    finish_node(c, N, i, pi, iface != 0, flag != 0, sums, -mul(c.KS11, S11), Un1, Un, F);
+  }
+}
+
+// 1 / sqrt(x) from a single-precision start y0 (22 bits) and Householder's third-order step
+// y0 + y0 e (1/2 + 3/8 e), e = 1 - x y0^2: the error falls to e^3 and stays at the FP64 rounding.
+// The conversions move bits, so that only the step's five operations use the FP64 pipe; values
+// that FP32 does not hold take CUDA's rsqrt.
+__device__ __forceinline__ double rsqrt_step(double x) {
+  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
+  const unsigned int ex = hi >> 20;  // the sign is clear
+  if (ex < 1023u - 100u || ex > 1023u + 100u) return rsqrt(x);
+  const float f = __uint_as_float(((ex - 1023u + 127u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const unsigned int g = __float_as_uint(rsqrtf(f));
+  const double y = __hiloint2double((int)((((g >> 23) - 127u + 1023u) << 20) | ((g & 0x7fffffu) >> 3)), (int)(g << 29));
+  const double e = fma(-mul(x, y), y, 1.0);
+  return fma(mul(e, fma(e, 0.375, 0.5)), y, y);
+}
+
+// The residual for s = 0 and liquid diffusivities that are not zero, charges in the model's groups
+// (2, 1, -1, -2, -3: kGroup): the reference's data.  In units of a species' liquid-liquid
+// diffusion factor a liquid-liquid bond adds (w + rho v) d + rho v U_i, with w = beta / xi^3,
+// v = w dphi, d = U_n - U_i and rho = K_k2 z_k F / (K_k1 R T): the weight w + rho v is one FMA a
+// group, the rest of the migration one sum of v a node, so that a species costs a bond a
+// subtraction and an FMA (26 FP64 instructions for the ten species where the separate sums
+// take 40).  Mixed bonds carry their factor's ratio.  K warps share 32 nodes' bonds and meet in
+// shared memory: with K = 4 while a thread a node would leave SMs idle.
+constexpr int kGroups = 5;
+__host__ __device__ constexpr int species_group(int k) {
+  constexpr int g[kSp] = {0, 1, 2, 2, 3, 3, 4, 0, 1, 2};
+  return g[k];
+}
+template <int K>
+__global__ void __launch_bounds__(128) k_residuals_grouped(ChemParams c, int N, const double* __restrict__ xyz,
+                                                           const int* __restrict__ hz, const int* __restrict__ hl,
+                                                           const double* __restrict__ Un1, const double* __restrict__ Un,
+                                                           const int* __restrict__ phase, double* __restrict__ F) {
+  constexpr int NV = kSp + 2;
+  __shared__ double sm[K > 1 ? (K - 1) * NV * 32 : 1];
+  __shared__ int s_flags[K > 1 ? K * 32 : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int part = K > 1 ? warp : 0;
+  constexpr int per = 4 / K;  // groups of 32 nodes a block
+  const double one = 1.0;
+  for (int g0 = blockIdx.x * per; 32 * g0 < N; g0 += gridDim.x * per) {
+    const int i = 32 * (g0 + (K > 1 ? 0 : warp)) + lane;
+    const bool live = i < N;
+    double t[NV];  // the species' sums, the potential's, the sum of v over liquid-liquid bonds
 #pragma unroll
-    for (int k = 0; k < kSp; ++k) {
-      u1[k] = ui[k];
-      u0[k] = Un[(size_t)k * N + i];
-    }
-    const bool liq = pi == 0;
-    const bool act = iface || liq;  // solid nodes with a liquid neighbour, liquid nodes
-    double R[kSp];
+    for (int q = 0; q < NV; ++q) t[q] = 0.0;
+    int pi = 0, flags = 0;  // 1: a liquid neighbour, 2: a solid one
+    if (live) {
+      pi = phase[i];
+      const int len = hl[i];
+      const double xi0 = xyz[i], yi0 = xyz[N + i], zi0 = xyz[2 * N + i];
+      const double phi_i = Un[(size_t)kSp * N + i], phi1_i = Un1[(size_t)kSp * N + i];
+      double ui[kSp];
 #pragma unroll
-    for (int k = 0; k < kSp; ++k) R[k] = 0.0;
-    // Mg (utils.h:162-174)
-    if (act) {
-      double t = mul(-c.k1b, pos(sub(mul(mul(u1[0], u0[2]), u0[2]), c.pMgOH2)));
-      t = sub(t, mul(c.k2b, pos(sub(mul(u1[0], u0[4]), c.pMgCO3))));
-      t = sub(t, mul(c.k3b, pos(sub(mul(u1[0], u0[4]), c.pMgHCO3))));
-      t = sub(t, mul(c.k4b, pos(sub(mul(mul(mul(mul(u0[0], u0[0]), u0[0]), u0[5]), u0[5]), c.pMgPO4))));
-      R[0] = t;
-    }
-    // H+ (utils.h:241-253): the interface's Butler-Volmer source, the liquid's equilibria
-    if (iface) {
-      const double phic = mul(dvd(mul(c.R, c.T), mul(c.F, c.z[0])), log(dvd(u0[0], dvd(c.CSat, c.CSolid))));
-      const double eta = sub(sub(add(c.phim, c.phimse), phi_i), phic);
-      R[1] = add(0.0, mul(dvd(c.JHp, mul(mul(c.z[1], c.F), c.CSolid)),
-                          exp(dvd(mul(mul(-c.alphaC, c.F), eta), mul(c.R, c.T)))));
-    } else if (liq) {
-      double t = mul(c.k7b, sub(c.pH2O, mul(u1[1], u0[2])));
-      t = add(t, mul(c.k8b, sub(c.pHCO3, mul(u1[1], u0[4]))));
-      t = add(t, mul(c.k9b, sub(c.pHPO4, mul(u1[1], u0[6]))));
-      R[1] = t;
-    }
-    // OH- (utils.h:321-330)
-    if (act) {
-      double t = mul(-c.k1b, pos(sub(mul(mul(u0[2], u0[2]), u0[0]), c.pMgOH2)));
-      t = sub(t, mul(c.k6b, pos(sub(ca5ohpo4(u1[2], u0[7], u0[6]), c.pCa5OHPO4))));
-      if (liq) t = add(t, mul(c.k7b, sub(c.pH2O, mul(u1[2], u0[1]))));
-      R[2] = t;
-    }
-    // species 4 (utils.h:396-401): the liquid's HCO3 equilibrium
-    if (liq) R[3] = mul(c.k8b, sub(c.pHCO3, mul(u1[3], u0[1])));
-    // species 5 (utils.h:466-476)
-    if (act) {
-      double t = mul(-c.k2b, pos(sub(mul(u1[4], u0[0]), c.pMgCO3)));
-      t = sub(t, mul(c.k3b, pos(sub(mul(u1[4], u0[0]), c.pMgHCO3))));
-      t = sub(t, mul(c.k5b, pos(sub(mul(u1[4], u0[7]), c.pCaCO3))));
-      if (liq) t = add(t, mul(c.k8b, sub(c.pHCO3, mul(u0[1], u1[4]))));
-      R[4] = t;
-    }
-    // species 6 (utils.h:541-547)
-    if (act) {
-      double t = mul(-c.k4b, pos(sub(mul(mul(mul(mul(u0[0], u0[0]), u0[0]), u0[5]), u0[5]), c.pMgPO4)));
-      if (liq) t = add(t, mul(c.k9b, add(-c.pHPO4, mul(u0[6], u0[1]))));
-      R[5] = t;
-    }
-    // species 7 (utils.h:612-618)
-    if (act) {
-      double t = mul(-c.k6b, pos(sub(ca5ohpo4(u0[2], u0[7], u0[6]), c.pCa5OHPO4)));
-      if (liq) t = add(t, mul(c.k9b, sub(c.pHPO4, mul(u1[6], u0[1]))));
-      R[6] = t;
-    }
-    // species 8 (utils.h:683-690)
-    if (act) {
-      double t = mul(-c.k5b, pos(sub(mul(u1[7], u0[4]), c.pCaCO3)));
-      t = sub(t, mul(c.k6b, pos(sub(ca5ohpo4(u0[2], u0[7], u0[6]), c.pCa5OHPO4))));
-      R[7] = t;
-    }
+      for (int k = 0; k < kSp; ++k) ui[k] = Un1[(size_t)k * N + i];
+      for (int j = 1 + part; j < len; j += K) {
+        const int n = hz[(size_t)j * N + i];
+        const double ex = sub(xyz[n], xi0), ey = sub(xyz[N + n], yi0), ez = sub(xyz[2 * N + n], zi0);
+        const double x2 = fma(ex, ex, fma(ey, ey, mul(ez, ez)));
+        const double rs = rsqrt_step(x2);
+        // beta (utils.h:17-25) = (delta + dx / 2 - xi) / dx between 0 and 1, by its bits
+        double beta = fma(mul(x2, rs), -c.rdx, c.bc0);
+        if (__double2hiint(beta) >= __double2hiint(one)) beta = one;
+        if (__double2hiint(beta) < 0) beta = 0.0;
+        const double w = mul(mul(mul(rs, rs), rs), beta);
+        const double v = mul(w, sub(Un[(size_t)kSp * N + n], phi_i));
+        const int pn = phase[n];
+        flags |= pn == 0 ? 1 : 2;
+        if (pi == 0 && pn == 0) {
+          double wg[kGroups];
 #pragma unroll
-    for (int k = 0; k < kSp; ++k)
-      F[(size_t)k * N + i] = sub(add(add(dvd(sub(u1[k], u0[k]), c.dt), s1[k]), s2[k]), R[k]);
-    // potential (utils.h:801-841)
-    double f11 = 0.0;
-    if (flag) {
-      double r11 = mul(c.z[0], u0[0]);
+          for (int q = 0; q < kGroups; ++q) wg[q] = fma(c.rho[q], v, w);
 #pragma unroll
-      for (int k = 1; k < kSp; ++k) r11 = add(r11, mul(c.z[k], u0[k]));
-      const double inv = dvd(1.0, mul(c.K11, c.sigma1));
-      f11 = sub(mul(inv, s11), mul(mul(mul(inv, c.F), c.CSolid), r11));
+          for (int k = 0; k < kSp; ++k) t[k] = fma(wg[species_group(k)], sub(Un1[(size_t)k * N + n], ui[k]), t[k]);
+          t[kSp] = fma(w, sub(Un1[(size_t)kSp * N + n], phi1_i), t[kSp]);
+          t[kSp + 1] = add(t[kSp + 1], v);
+        } else {
+          const int cls = pi != 0 && pn != 0 ? 1 : 0;
+#pragma unroll
+          for (int k = 0; k < kSp; ++k) {
+            if (k > 0 && cls) continue;  // solid-solid bonds carry only Mg
+            const double un = Un1[(size_t)k * N + n];
+            const double m = fma(mul(c.rho[species_group(k)], v), un, mul(w, sub(un, ui[k])));
+            t[k] = fma(c.q1[cls][k], m, t[k]);
+          }
+        }
+      }
     }
-    F[(size_t)kSp * N + i] = f11;
+    if (K > 1) {
+      if (part > 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sm[((part - 1) * NV + q) * 32 + lane] = t[q];
+      s_flags[part * 32 + lane] = flags;
+      __syncthreads();
+      if (part == 0)
+        for (int h = 0; h < K - 1; ++h) {
+#pragma unroll
+          for (int q = 0; q < NV; ++q) t[q] += sm[(h * NV + q) * 32 + lane];
+          flags |= s_flags[(h + 1) * 32 + lane];
+        }
+    }
+    if (live && part == 0) {
+      double sums[kSp];
+#pragma unroll
+      for (int k = 0; k < kSp; ++k) {
+        const double m = mul(c.rho[species_group(k)], t[kSp + 1]);
+        sums[k] = -mul(mul(c.sg1[k], c.dxyz), fma(m, Un1[(size_t)k * N + i], t[k]));
+      }
+      finish_node(c, N, i, pi, pi == 1 && (flags & 1), pi == 0 && (flags & 1), sums, -mul(mul(c.KS11, c.dxyz), t[kSp]),
+                  Un1, Un, F);
+    }
+    if (K > 1) __syncthreads();
   }
 }
 
@@ -344,10 +483,23 @@ ChemParams make_chem_params(const double* d2, const double* dc, const double* d1
       c.q2[q][k] = c.a2[q + 1][k] / c.sg2[k];
     }
   }
+  c.rdt = std::fabs(c.dt) > 1e-150 && std::fabs(c.dt) < 1e150 ? 1.0 / c.dt : 0.0;
+  c.rdx = 1.0 / c.dx;
+  c.bc0 = (c.delta + c.dx / 2.0) / c.dx;
   c.one_exp = c.e11 == c.e1[0];
   for (int k = 0; k < kSp; ++k) c.one_exp = c.one_exp && c.e1[k] == c.e1[0] && c.e2[k] == c.e1[0];
   c.ie = 0;
   if (c.one_exp && c.e1[0] >= 1.0 && c.e1[0] <= 8.0 && c.e1[0] == std::floor(c.e1[0])) c.ie = (int)c.e1[0];
+  // the charge groups' migration over diffusion factors; equal within a group by their inputs
+  c.grouped = c.one_exp && c.ie == 3 && std::isfinite(c.rdx) && c.dx > 0.0 && c.delta > c.dx / 2.0;
+  bool seen[kGroups] = {};
+  for (int k = 0; k < kSp; ++k) {
+    const int g = species_group(k);
+    const double rho = c.K2[k] * c.z[k] * c.F / (c.K1[k] * c.R * c.T);
+    if (!seen[g]) c.rho[g] = rho;
+    seen[g] = true;
+    c.grouped = c.grouped && c.on1[k] && std::isfinite(rho) && rho == c.rho[g];
+  }
   return c;
 }
 
@@ -375,13 +527,18 @@ nnpp_status nnpp_residuals_full_device(int n_nodes, const double* d_nodes, const
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   bool all_on = true;
   for (int k = 0; k < kSp; ++k) all_on = all_on && c.on1[k] && c.on2[k];
-  auto go = [&](auto kern) {
-    kern<<<blocks, 128, 0, st>>>(c, n_nodes, d_nodes, d_clouds, d_lengths, d_U_n1, d_U_n, d_phase, d_F);
+  auto go = [&](auto kern, int grid) {
+    kern<<<grid, 128, 0, st>>>(c, n_nodes, d_nodes, d_clouds, d_lengths, d_U_n1, d_U_n, d_phase, d_F);
   };
-  if (c.one_exp)
-    all_on ? go(k_residuals_full<true, true>) : go(k_residuals_full<true, false>);
+  const int groups = (n_nodes + 31) / 32;
+  if (c.grouped && groups < kSplitGroups)
+    go(k_residuals_grouped<4>, std::min(groups, 152 * 64));
+  else if (c.grouped)
+    go(k_residuals_grouped<1>, std::min((groups + 3) / 4, 152 * 64));
+  else if (c.one_exp)
+    all_on ? go(k_residuals_full<true, true>, blocks) : go(k_residuals_full<true, false>, blocks);
   else
-    all_on ? go(k_residuals_full<false, true>) : go(k_residuals_full<false, false>);
+    all_on ? go(k_residuals_full<false, true>, blocks) : go(k_residuals_full<false, false>, blocks);
   NNPP_CUDA(cudaGetLastError());
   return NNPP_OK;
 }
