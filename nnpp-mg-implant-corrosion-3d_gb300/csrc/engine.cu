@@ -49,6 +49,19 @@ nnpp_status sync_members(Engine& e) {
   return NNPP_OK;
 }
 
+// slots a value of the partials takes: the items, or the groups of slices (slice_group0)
+int partial_stride(const Engine& e) {
+  return std::max(std::max(e.ntiles, e.nchunks), std::max(e.nslices, e.ncslices)) + (int)e.members.size() + 1;
+}
+
+// the members' FP64 weights for the current lists (FP64 runs)
+nnpp_status ensure_sell64(Engine& e) {
+  const int M = (int)e.members.size();
+  for (int i = 0; i < M; ++i)
+    NNPP_TRY(build_sell64(*e.members[i], e.d_slices.get() + e.h_meta[4 * M + i], e.h_meta[5 * M + i]));
+  return NNPP_OK;
+}
+
 // Work lists for bins-per-tile T (rebuilds every member's slots).
 nnpp_status build_lists(Engine& e, int T) {
   const int M = (int)e.members.size();
@@ -110,11 +123,12 @@ nnpp_status build_lists(Engine& e, int T) {
   e.halo_max = hm;
   e.bond_max = bmax;
   e.T = T;
-  const int stride = std::max(std::max(e.ntiles, e.nchunks), std::max(e.nslices, e.ncslices));
+  const int stride = partial_stride(e);
+  e.h_meta = meta;
   if (!e.d_tiles.alloc(tiles.size()) || !e.d_chunks.alloc(chunks.size()) || !e.d_meta.alloc(meta.size()) ||
       !e.d_slices.alloc(std::max<size_t>(slices.size(), 1)) || !e.d_htiles.alloc(std::max<size_t>(htiles.size(), 1)) ||
       !e.d_cslices.alloc(std::max<size_t>(cslices.size(), 1)) ||
-      !e.d_ticket.alloc(M + 4) ||
+      !e.d_ticket.alloc(M + 4) || !e.d_gcount.alloc((size_t)stride) ||
       !e.d_partials.alloc((size_t)kReduceSlots * stride) ||
       !e.d_inst[0].alloc(M) || !e.d_inst[1].alloc(M))
     return set_error(NNPP_ERR_NOMEM, "engine work lists");
@@ -128,6 +142,7 @@ nnpp_status build_lists(Engine& e, int T) {
   if (!cslices.empty())
     NNPP_CUDA(cudaMemcpyAsync(e.d_cslices.get(), cslices.data(), sizeof(SliceDesc) * cslices.size(), cudaMemcpyHostToDevice, e.st));
   NNPP_CUDA(cudaMemsetAsync(e.d_ticket.get(), 0, e.d_ticket.bytes(), e.st));
+  NNPP_CUDA(cudaMemsetAsync(e.d_gcount.get(), 0, e.d_gcount.bytes(), e.st));
   NNPP_CUDA(cudaStreamSynchronize(e.st));
   engine_destroy_graphs(e);
   return NNPP_OK;
@@ -147,22 +162,39 @@ nnpp_status set_active(Engine& e, int outer, int inner) {
   return NNPP_OK;
 }
 
-// Autotuner: bins per tile T and lanes per node W that minimise the CG operator on the
-// current state (run tens of times per step) plus, for the mixed path, one FP64 tile
-// operator (the refinement residual and the prep use the W lanes per node).
+// Autotuner: the FP32 CG operator's variant and the bins per tile T that minimise the share of a
+// step they decide on the current state: kTuneCg launches of the operator and kTunePrep of the prep
+// (whose slices, like the transport's, are cut at the tiles' ends).  Variants 1 and 8 depend on the
+// tiles and are timed for each T; the others run on the CG slices, the same for every T.  The FP64
+// path has one operator: T alone is chosen.  The lanes per node of the residual entry points' tile
+// kernels stay at their default.
+constexpr int kTuneCg = 15, kTunePrep = 3;
 nnpp_status tune(Engine& e, int prec) {
   std::vector<DevState> saved(e.members.size());
   NNPP_CUDA(cudaStreamSynchronize(e.st));
   for (size_t i = 0; i < e.members.size(); ++i)
     NNPP_CUDA(cudaMemcpy(&saved[i], e.members[i]->dstate.get(), sizeof(DevState), cudaMemcpyDeviceToHost));
-  const int Ts[4] = {2, 4, 8, 16};
-  const int Ws[3] = {4, 8, 16};
+  const int Ts[3] = {2, 4, 8};
+  const int W = 8;
   float best = 1e30f;
-  int bT = 4, bW = 8;
-  int bS = 0;
+  int bT = 4, bS = 0;
   cudaEvent_t e0, e1;
   NNPP_CUDA(cudaEventCreate(&e0));
   NNPP_CUDA(cudaEventCreate(&e1));
+  // milliseconds a launch (after one to warm up)
+  auto timed = [&](int reps, float* ms, auto launch) -> nnpp_status {
+    NNPP_TRY(launch());
+    cudaEventRecord(e0, e.st);
+    for (int r = 0; r < reps; ++r) NNPP_TRY(launch());
+    cudaEventRecord(e1, e.st);
+    NNPP_CUDA(cudaEventSynchronize(e1));
+    cudaEventElapsedTime(ms, e0, e1);
+    *ms /= reps;
+    return NNPP_OK;
+  };
+  float t_var[kSpmvVariants];
+  bool have_var[kSpmvVariants] = {};
+  e.W = W;
   for (int T : Ts) {
     const nnpp_status bs = build_lists(e, T);
     if (bs == NNPP_ERR_UNSUPPORTED) {
@@ -170,35 +202,33 @@ nnpp_status tune(Engine& e, int prec) {
       continue;
     }
     NNPP_TRY(bs);
+    if (prec == NNPP_FP64) NNPP_TRY(ensure_sell64(e));
     NNPP_TRY(refresh_params(e));
-    for (int W : Ws) {
-      e.W = W;
-      if (prepare_kernels(e.halo_max, e.bond_max, W) != NNPP_OK) continue;
-      EngineView v = make_view(e, 0, 0);
-      NNPP_TRY(set_active(e, 1, 1));
-      NNPP_TRY(launch_prep_b(e, v, prec, e.st, 0, nullptr));
-      const bool win = prec == NNPP_MIXED && spmv_staged_fits(e);
-      const int nvar = prec == NNPP_MIXED ? kSpmvVariants : 1;
-      for (int var = 0; var < nvar; ++var) {
-        if (!win && spmv_needs_windows(var)) continue;
-        if (var == kSpmvHalo && !spmv_halo_fits(e)) continue;
-        e.spmv_variant = var;
+    if (prepare_kernels(e.halo_max, e.bond_max, W) != NNPP_OK) {
+      clear_error();
+      continue;
+    }
+    EngineView v = make_view(e, 0, 0);
+    NNPP_TRY(set_active(e, 1, 1));
+    float t_prep = 0.0f;
+    // the warm-up launch forms the mask sums, the timed ones are a step's
+    NNPP_TRY(timed(4, &t_prep, [&] { return launch_prep_b(e, v, prec, e.st, 0, nullptr); }));
+    const bool win = prec == NNPP_MIXED && spmv_staged_fits(e);
+    const int nvar = prec == NNPP_MIXED ? kSpmvVariants : 1;
+    for (int var = 0; var < nvar; ++var) {
+      if (!win && spmv_needs_windows(var)) continue;
+      if (var == kSpmvHalo && !spmv_halo_fits(e)) continue;
+      e.spmv_variant = var;
+      if (!have_var[var] || var == 1 || var == kSpmvHalo) {
+        have_var[var] = true;
         NNPP_TRY(set_active(e, 1, 1));
-        NNPP_TRY(launch_cg_spmv_b(e, v, prec, e.st));
-        cudaEventRecord(e0, e.st);
-        // the CG operator dominates; the FP64 tile kernels (residual, prep) follow the lanes
-        for (int r = 0; r < 5; ++r) NNPP_TRY(launch_cg_spmv_b(e, v, prec, e.st));
-        if (prec == NNPP_MIXED) NNPP_TRY(launch_cg_spmv_b(e, v, NNPP_FP64, e.st));
-        cudaEventRecord(e1, e.st);
-        NNPP_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best) {
-          best = ms;
-          bT = T;
-          bW = W;
-          bS = e.spmv_variant;
-        }
+        NNPP_TRY(timed(5, &t_var[var], [&] { return launch_cg_spmv_b(e, v, prec, e.st); }));
+      }
+      const float ms = kTuneCg * t_var[var] + kTunePrep * t_prep;
+      if (ms < best) {
+        best = ms;
+        bT = T;
+        bS = var;
       }
     }
   }
@@ -208,9 +238,8 @@ nnpp_status tune(Engine& e, int prec) {
   for (size_t i = 0; i < e.members.size(); ++i)
     NNPP_CUDA(cudaMemcpy(e.members[i]->dstate.get(), &saved[i], sizeof(DevState), cudaMemcpyHostToDevice));
   NNPP_TRY(build_lists(e, bT));
-  e.W = bW;
   e.spmv_variant = bS;
-  NNPP_TRY(prepare_kernels(e.halo_max, e.bond_max, bW));
+  NNPP_TRY(prepare_kernels(e.halo_max, e.bond_max, W));
   e.tuned = true;
   return NNPP_OK;
 }
@@ -341,6 +370,7 @@ nnpp_status prepare_run(Engine& e, int prec) {
         break;
       }
   }
+  if (prec == NNPP_FP64) NNPP_TRY(ensure_sell64(e));
   // two-level preconditioner of single-instance engines: recompute the coarse inverse when the
   // state was replaced; the captured graphs follow whether the coarse correction is applied
   for (Handle* hp : e.members) {
@@ -411,7 +441,8 @@ EngineView make_view(Engine& e, int parity, int in_graph) {
   v.nchunks = e.nchunks;
   v.M = M;
   v.in_graph = in_graph;
-  v.stride = std::max(std::max(e.ntiles, e.nchunks), std::max(e.nslices, e.ncslices));
+  v.gcount = e.d_gcount.get();
+  v.stride = partial_stride(e);
   v.halo_max = e.halo_max;
   v.bond_max = e.bond_max;
   return v;

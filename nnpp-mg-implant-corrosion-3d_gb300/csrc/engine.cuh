@@ -92,11 +92,12 @@ struct EngineView {
   const int* cslice_count;
   unsigned int* ticket;     // per instance completion counters, + [M] global, + [M+1] grid,
                             // + [M+2] slice claims, + [M+3] the next-guess pass
+  unsigned int* gcount;     // FP64 slice groups: slices done (zero between kernels)
   double* partials;         // kReduceSlots * stride
   int ntiles, nchunks, M, in_graph;
   int nslices;
   int ncslices;
-  int stride;               // max(ntiles, nchunks, nslices, ncslices): slot stride of partials
+  int stride;               // slot stride of partials: at least the largest item count + M + 1
   int halo_max;             // largest halo (dynamic shared memory sizing)
   int bond_max;             // largest staged bond range of a tile (bond1 - bond0)
   int hcode_max16;          // largest code block of a tile (16-byte units, variant 8)
@@ -138,6 +139,8 @@ struct Engine {
   DBuf<SliceDesc> d_cslices;
   DBuf<HTile> d_htiles;
   DBuf<unsigned int> d_ticket;
+  DBuf<unsigned int> d_gcount;
+  std::vector<int> h_meta;  // host copy of d_meta
   DBuf<double> d_partials;
   int ntiles = 0, nchunks = 0, nslices = 0, ncslices = 0;
   cudaStream_t st = nullptr, st_b1 = nullptr, st_b2 = nullptr;
@@ -166,6 +169,9 @@ nnpp_status build_tiles(Handle& h, int T, std::vector<TileDesc>& tiles, std::vec
 // value, 32 a slice, with their windows) and its compacted arrays (filled by the prep); the
 // slices are appended to cslices; false in *windows_fit when a window exceeds kWinCap
 nnpp_status build_cg_slices(Handle& h, std::vector<SliceDesc>& cslices, int inst, bool* windows_fit);
+// the FP64 weights of the instance's slices (device descriptors, count) in sell's order, and room for
+// the CG slices' (the FP64 prep fills them); nothing to do while sell64_ok
+nnpp_status build_sell64(Handle& h, const SliceDesc* slices, int count);
 // the variant 8 layout of one instance (after build_tiles, same T): its HTile entries are
 // appended to htiles (parallel to the instance's tiles); false in *ok when the layout does
 // not apply (a kernel exponent s != 0, a halo of 65535 nodes or more)

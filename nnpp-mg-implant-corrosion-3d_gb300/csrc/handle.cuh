@@ -32,16 +32,18 @@ struct KParams {
   const int* col;
   const unsigned short* slot16;  // per bond: halo slot of the neighbour within its tile
   // sliced layout (32 consecutive rows of a tile per slice, bonds column-major within a
-  // slice, rows padded to the slice's longest): per bond column 32 FP32 weights then 32
-  // 16-bit slot codes (window row << 12 | offset)
+  // slice, rows padded to the slice's longest, whole quads): per quad of bond columns 32 lanes'
+  // four FP32 weights, then their four 16-bit slot codes (window row << 12 | offset)
   const float* sell;
-  const float* sell_lo;          // sliced like sell's weights: wlo32 (32 floats per column)
+  const float* sell_lo;          // wlo32, per quad 32 lanes' four values (32 floats a column)
   // the CG operator (and the refinement's residual update) on its own slices: 32 of a bin
   // row's nodes without a potential Dirichlet value a slice; each row holds its bonds to
   // columns that can be unknowns (liquid, no potential Dirichlet value) in bond order,
   // interleaved like sell (weights, codes relative to the CG slice's windows) and sell_lo
   float* sell_cg;
   float* sell_cg_lo;
+  const double* sell64;          // FP64 path: the slices' FP64 weights, ordered like sell_lo
+  double* sell_cg64;             // and the CG slices' (filled by the FP64 prep)
   int* cg_width;                 // per CG slice of the handle: its longest row (the shorter
                                  // rows are zero-padded to the slice's capacity)
   const int* cg_rows;            // per slot: the node, -1 for padding
@@ -83,6 +85,8 @@ struct KParams {
   double dt, csat, c_floor, k_diss, sw, vol_red, lam;
   float csat_hi, csat_lo, cfl_hi, cfl_lo;  // CSat/CSolid and c_floor as FP32 pairs
   double K1[S], K2zF[S], DL[S], DSo[S], z[S];
+  // their FP32 roundings, for the FP32 bond sums (a conversion from FP64 holds the FP64 pipe)
+  float K1f[S], K2zFf[S], DLf[S], DSof[S], dtf;
   int sub_step_no;
   int dissolve_count;            // 1: count the dissolution source into the diagnostics
   int extrapolate;               // 1: warm start phi = 2 phi^n - phi^{n-1}
@@ -182,6 +186,8 @@ struct Handle {
   DBuf<float> sell_lo;
   DBuf<float> sell_cg;          // the CG operator's slices (see KParams)
   DBuf<float> sell_cg_lo;
+  DBuf<double> sell64, sell_cg64;  // FP64 weights of both slicings, made by the first FP64 run
+  bool sell64_ok = false;          // they belong to the current slices
   DBuf<int> cg_width, cg_rows, cg_pos, xrow;
   DBuf<float4> phi4;
   DBuf<float4> posrec;

@@ -228,6 +228,44 @@ __device__ __forceinline__ void reduce_dot_items(const double* partials, int str
     reduce_pair_items<NV>(partials, stride, first, count, out, sm);
 }
 
+// FP64 slice partials: a warp stores its slice's values (lane 0 holds them) and the warp that
+// completes a group of 32 of the instance's slices sums the group, so that the last CTA is
+// left with a thirty-second of the FP64 additions (one SM's FP64 pipe takes microseconds for
+// the slices of a 512k-node pass).  Groups are fixed, so the sums do not depend on timing.
+// `first`, `count`: the instance's slices; group sums at partials[(NV + k) * stride + slot].
+__device__ __forceinline__ int slice_group0(int first, int inst) { return (first >> 5) + inst; }
+template <int NV>
+__device__ __forceinline__ void slice_partials64(const EngineView& v, int inst, int first, int count, int sg,
+                                                 const double (&val)[NV]) {
+  const int lane = threadIdx.x & 31;
+  const int gi = (sg - first) >> 5, members = min(32, count - 32 * gi);
+  const int slot = slice_group0(first, inst) + gi;
+  unsigned int t = 0;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v.partials[(size_t)k * v.stride + sg] = val[k];
+    __threadfence();
+    t = atomicAdd(&v.gcount[slot], 1u);
+  }
+  t = __shfl_sync(0xffffffffu, t, 0);
+  if (t != (unsigned int)(members - 1)) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    double x = lane < members ? __ldcg(&v.partials[(size_t)k * v.stride + first + 32 * gi + lane]) : 0.0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+    if (lane == 0) v.partials[(size_t)(NV + k) * v.stride + slot] = x;
+  }
+  if (lane == 0) v.gcount[slot] = 0;
+}
+// the last CTA's sum of an instance's groups
+template <int NV>
+__device__ __forceinline__ void reduce_slices64(const EngineView& v, int inst, int first, int count, double (&out)[NV],
+                                                double* sm) {
+  reduce_items<NV>(v.partials + (size_t)NV * v.stride, v.stride, slice_group0(first, inst), (count + 31) >> 5, out, sm);
+}
+
 // Item partials of per-thread dot accumulators: FP64 block sums on the FP64 path; on the
 // FP32 path FP32-pair warp sums, then warp 0 sums the warps' pairs (sm: NV * kBlock / 32
 // doubles, reused as pairs) and stores the pair partials (reduce_dot_items sums them).
@@ -334,17 +372,14 @@ __device__ __forceinline__ double seg_reduce_pair(float h, float l) {
   return (double)h + (double)l;
 }
 
-// ------------------------------------------------------------------- potential: prep ----
-// Per node: K11 diagonal (sum of liquid-liquid weights), unknown mask, right-hand side
-// b = (1/(K sigma)) F CSolid sum_k z_k c_k and the FP64 residual r = b - A phi.  With F11_out
-// (single instance), writes the reference's F11 (utils.h:798-841) for every node instead.
+// ------------------------------------------------------------------- potential: F11 ------
+// The reference's F11 (utils.h:798-841) for every node of one instance: the sum of liquid-liquid
+// weights times the potential's differences against b = (1/(K sigma)) F CSolid sum_k z_k c_k,
+// zero on nodes without such a bond.  CTA per tile, its halo staged in shared memory.
 template <typename P, int W>
-__global__ void __launch_bounds__(kBlock) k_prep(EngineView v, cudaGraphConditionalHandle hc,
-                                                 double* F11_out) {
+__global__ void __launch_bounds__(kBlock) k_f11(EngineView v, double* F11_out) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ TileSmem ts;
-  __shared__ double sm[2 * kBlock / 32];
-  __shared__ int s_last;
   const int sub = threadIdx.x % W, seg = threadIdx.x / W, nseg = kBlock / W;
   for (int item = blockIdx.x; item < v.ntiles; item += gridDim.x) {
     const TileDesc t = v.tiles[item];
@@ -355,159 +390,63 @@ __global__ void __launch_bounds__(kBlock) k_prep(EngineView v, cudaGraphConditio
     float2* sphi2 = reinterpret_cast<float2*>(dsm);
     unsigned char* sfl = dsm + sizeof(double) * (size_t)t.halo;
     const unsigned short* sslot = stage_slots(k.slot16, t, dsm + align16(sizeof(double) * (size_t)t.halo + t.halo));
-    const double* phi64 = k.phi64;
-    const unsigned char* dm = k.dirmask;
     for (int s = threadIdx.x; s < t.halo; s += kBlock) {
       const int n = halo_node(ts, s);
-      const double ph = phi64[n];
+      const double ph = k.phi64[n];
       if (kPair) {
         const float hi = (float)ph;
         sphi2[s] = make_float2(hi, (float)(ph - (double)hi));
       } else {
         sphi[s] = ph;
       }
-      sfl[s] = (unsigned char)((phase_of<P>(k, n) == 0.0f ? 1 : 0) | (((dm[n] >> S) & 1) ? 2 : 0));
+      sfl[s] = phase_of<P>(k, n) == 0.0f ? 1 : 0;
     }
     __syncthreads();
-    double part[2] = {0.0, 0.0};
     const int* row = k.row;
-    const double* w64 = k.w64;
     const int own0 = ts.off[4] + (t.own_begin - t.hb[4]);
-    // the mask-only sums (diagonal, Dirichlet coupling, unknown flag) are kept from the
-    // last prep while no phase changed: only sum_j w phi_j is formed then
-    const bool cached = F11_out == nullptr && k.ds->op_valid != 0;
     for (int a0 = t.own_begin; a0 < t.own_end; a0 += nseg) {
       const int a = a0 + seg;
       const bool act = a < t.own_end;
       const int so = own0 + (a - t.own_begin);
-      const unsigned char fa = act ? sfl[so] : 0;
-      const bool scan = act && (fa & 1) && (F11_out != nullptr || !(fa & 2));
-      double dsum = 0.0, swphi = 0.0, cpl = 0.0;
+      const bool scan = act && sfl[so];
+      double dsum = 0.0, swphi = 0.0;
       int anyll = 0;
-      if (cached) {
-        if (kPair) {
-          float sh = 0.f, sl = 0.f;
-          if (scan && k.freem[a]) {
-            for (int j = row[a] + sub; j < row[a + 1]; j += W) {
-              const int s = sslot[j - t.bond0];
-              if (sfl[s] & 1) {
-                const float2 ph = sphi2[s];
-                float ph_, pl_;
-                pair_mul(k.w32[j], k.wlo32[j], ph.x, ph.y, ph_, pl_);
-                pair_add(sh, sl, ph_, pl_);
-              }
-            }
-          }
-          swphi = seg_reduce_pair<W>(sh, sl);
-        } else {
-          if (scan && k.freem[a]) {
-            for (int j = row[a] + sub; j < row[a + 1]; j += W) {
-              const int s = sslot[j - t.bond0];
-              if (sfl[s] & 1) swphi += w64[j] * sphi[s];
-            }
-          }
-          swphi = seg_reduce_d<W>(swphi);
-        }
-      } else if (kPair) {
-        float dh = 0.f, dl = 0.f, sh = 0.f, sl = 0.f, ch = 0.f, cl = 0.f;
-        if (scan) {
+      if (kPair) {
+        float dh = 0.f, dl = 0.f, sh = 0.f, sl = 0.f;
+        if (scan)
           for (int j = row[a] + sub; j < row[a + 1]; j += W) {
             const int s = sslot[j - t.bond0];
-            const unsigned char f = sfl[s];
-            if (f & 1) {
-              const float wh = k.w32[j], wl = k.wlo32[j];
-              const float2 ph = sphi2[s];
-              float ph_, pl_;
-              pair_mul(wh, wl, ph.x, ph.y, ph_, pl_);
-              pair_add(dh, dl, wh, wl);
-              pair_add(sh, sl, ph_, pl_);
-              anyll = 1;
-              if (f & 2) pair_add(ch, cl, ph_, pl_);
-            }
+            if (!sfl[s]) continue;
+            const float wh = k.w32[j], wl = k.wlo32[j];
+            const float2 ph = sphi2[s];
+            float ph_, pl_;
+            pair_mul(wh, wl, ph.x, ph.y, ph_, pl_);
+            pair_add(dh, dl, wh, wl);
+            pair_add(sh, sl, ph_, pl_);
+            anyll = 1;
           }
-        }
         dsum = seg_reduce_pair<W>(dh, dl);
         swphi = seg_reduce_pair<W>(sh, sl);
-        cpl = seg_reduce_pair<W>(ch, cl);
       } else {
-        if (scan) {
+        if (scan)
           for (int j = row[a] + sub; j < row[a + 1]; j += W) {
             const int s = sslot[j - t.bond0];
-            const unsigned char f = sfl[s];
-            if (f & 1) {
-              const double w = w64[j];
-              const double ph = sphi[s];
-              dsum += w;
-              swphi += w * ph;
-              anyll = 1;
-              if (f & 2) cpl += w * ph;
-            }
+            if (!sfl[s]) continue;
+            const double w = k.w64[j];
+            dsum += w;
+            swphi += w * sphi[s];
+            anyll = 1;
           }
-        }
         dsum = seg_reduce_d<W>(dsum);
         swphi = seg_reduce_d<W>(swphi);
-        cpl = seg_reduce_d<W>(cpl);
       }
       anyll = seg_or<W>(anyll);
       if (act && sub == 0) {
-        double b;
-        if (k.b_override) {
-          b = k.b_override[a];
-        } else {
-          double R11 = 0.0;
-          for (int s = 0; s < S; ++s) R11 += k.z[s] * conc_of<P>(k, a, s);
-          b = k.lam * R11;
-        }
+        double R11 = 0.0;
+        for (int s = 0; s < S; ++s) R11 += k.z[s] * conc_of<P>(k, a, s);
+        const double b = k.b_override ? k.b_override[a] : k.lam * R11;
         const double pha = kPair ? (double)sphi2[so].x + (double)sphi2[so].y : sphi[so];
-        if (F11_out) {
-          F11_out[a] = anyll ? (dsum * pha - swphi) - b : 0.0;
-        } else {
-          bool fr;
-          if (cached) {
-            fr = k.freem[a] != 0;
-            dsum = k.dsum64[a];
-            cpl = k.cpl64[a];
-          } else {
-            fr = !(fa & 2) && (fa & 1) && anyll;
-            k.freem[a] = fr ? 1 : 0;
-            k.dsum64[a] = fr ? dsum : 1.0;
-            k.cpl64[a] = fr ? cpl : 0.0;
-            k.dinv64[a] = fr ? 1.0 / dsum : 0.0;
-            k.d32[a] = fr ? (float)dsum : 1.0f;
-            k.dinv32[a] = fr ? (float)(1.0 / dsum) : 0.0f;
-          }
-          const double bb = fr ? b : 0.0;
-          const double r = fr ? bb - (dsum * pha - swphi) : 0.0;
-          k.b64[a] = bb;
-          k.r64[a] = r;
-          const double be = bb + (fr ? cpl : 0.0);
-          part[0] += be * be;
-          part[1] += r * r;
-        }
-      }
-    }
-    if (!F11_out) {
-      write_partials<2>(v, item, part, sm);
-      if (item_done(&v.ticket[t.inst], v.tile_count[t.inst], &s_last)) {
-        double tot[2];
-        reduce_items<2>(v.partials, v.stride, v.tile_first[t.inst], v.tile_count[t.inst], tot, sm);
-        if (threadIdx.x == 0) {
-          DevState* ds = k.ds;
-          ds->op_valid = 1;
-          const double bn = tot[0] > 0.0 ? tot[0] : 1.0;
-          ds->bnorm2 = bn;
-          ds->rnorm2 = tot[1];
-          ds->outer_it = 0;
-          ds->solve_iters = 0;
-          const bool go = tot[1] > ds->tol * ds->tol * bn && ds->max_outer > 0;
-          if (!go) {
-            ds->cg_solves += 1;
-            ds->last_relres = sqrt(tot[1] / bn);
-          }
-          ds->outer_active = go ? 1 : 0;
-          ds->inner_active = 0;
-          instance_finished(v, t.inst, 0, hc);
-        }
+        F11_out[a] = anyll ? (dsum * pha - swphi) - b : 0.0;
       }
     }
     __syncthreads();
@@ -619,23 +558,19 @@ __device__ __forceinline__ double warp_sum_d(double x) {
 }
 
 
-// Interleaved sliced operator: bond column c of a slice holds 32 FP32 weights then 32 16-bit
-// slot codes (kSellW floats = 192 bytes), so one contiguous copy moves both.
-constexpr int kSellW = 48;      // stride of a column in floats
-constexpr int kSellC = 96;      // stride of a column in 16-bit codes
+// Interleaved sliced operator: a quad of bond columns of a slice holds, per lane, the four FP32
+// weights of its row's bonds (32 x 16 bytes), then per lane their four 16-bit slot codes (32 x 8
+// bytes): one 16-byte and one 8-byte load a lane bring four bonds, and one contiguous copy
+// moves both.  A column takes 48 floats (192 bytes) on average; widths are padded to quads.
+constexpr int kSellW = 48;              // floats a column
+constexpr int kQuadW = 4 * kSellW;      // floats a quad
 __device__ __forceinline__ const float* sell_w(const KParams& k, const SliceDesc& d) {
   return k.sell + (size_t)(d.off >> 5) * kSellW;
-}
-__device__ __forceinline__ const unsigned short* sell_code(const KParams& k, const SliceDesc& d) {
-  return reinterpret_cast<const unsigned short*>(sell_w(k, d) + 32);
 }
 
 // the CG operator's compacted copy (same layout and offsets; columns in use: cg_width)
 __device__ __forceinline__ const float* sell_cg_w(const KParams& k, const SliceDesc& d) {
   return k.sell_cg + (size_t)(d.off >> 5) * kSellW;
-}
-__device__ __forceinline__ const unsigned short* sell_cg_code(const KParams& k, const SliceDesc& d) {
-  return reinterpret_cast<const unsigned short*>(sell_cg_w(k, d) + 32);
 }
 
 // the inner-loop flag of a slice's instance (constant while the operator runs)
@@ -652,15 +587,39 @@ __device__ __forceinline__ uint64_t stream_policy() {
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
-__device__ __forceinline__ float ld_stream(const float* p) {
-  float v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(stream_policy()));
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(p), "l"(stream_policy()));
   return v;
 }
-__device__ __forceinline__ unsigned int ld_stream(const unsigned short* p) {
-  unsigned short v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(stream_policy()));
+__device__ __forceinline__ uint2 ld_stream(const uint2* p) {
+  uint2 v;
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
+      : "=r"(v.x), "=r"(v.y)
+      : "l"(p), "l"(stream_policy()));
   return v;
+}
+// a lane's view of a slice's operator: quad q's weights and codes
+struct QuadPtr {
+  const float4* w;
+  const uint2* c;
+  __device__ __forceinline__ QuadPtr(const float* base, int lane)
+      : w(reinterpret_cast<const float4*>(base) + lane), c(reinterpret_cast<const uint2*>(base + 128) + lane) {}
+  __device__ __forceinline__ float4 weights(int q) const { return ld_stream(w + (kQuadW / 4) * q); }
+  __device__ __forceinline__ uint2 codes(int q) const { return ld_stream(c + (kQuadW / 2) * q); }
+};
+// the FP64 weights of a quad: 32 bytes a lane
+__device__ __forceinline__ void ld_stream_d4(const double* p, double (&w)[4]) {
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+      : "=d"(w[0]), "=d"(w[1]), "=d"(w[2]), "=d"(w[3])
+      : "l"(p), "l"(stream_policy()));
+}
+__device__ __forceinline__ float quad_weight(const float4& w, int u) { return u == 0 ? w.x : u == 1 ? w.y : u == 2 ? w.z : w.w; }
+__device__ __forceinline__ unsigned int quad_code(const uint2& c, int u) {
+  const unsigned int v = u < 2 ? c.x : c.y;
+  return u & 1 ? v >> 16 : v & 0xffffu;
 }
 
 __device__ __forceinline__ int code_node(const int* hb, unsigned int code) {
@@ -753,54 +712,46 @@ __global__ void __launch_bounds__(kBlock, MINB) k_cg_spmv32(EngineView v) {
       // code 0, weight 0), so that lane 0 can issue the prefetches
       if (PF > 0 ? __any_sync(0xffffffffu, live) : live) {
         const int* hb = s_hb[warp];
-        const float* ws = sell_cg_w(k, d) + lane;
-        const unsigned short* cs16 = sell_cg_code(k, d) + lane;
+        const QuadPtr op(sell_cg_w(k, d), lane);
         const float* z = k.z32;
-        // B columns per batch; PIPE: the next batch of streamed columns is in flight while
-        // the current batch's neighbour values are gathered (more registers, fewer warps)
+        // QB quads (B columns) per batch; PIPE: the next batch of streamed quads is in flight
+        // while the current batch's neighbour values are gathered (more registers, fewer warps).
+        // The last batch's missing quads take weight 0 and code 0 (a valid node).
+        constexpr int QB = B / 4;
+        const int nq = (width + 3) >> 2;
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        const int nb = width / B;
-        float w[B];
-        unsigned int code[B];
-        if (PIPE && nb > 0) {
+        float4 w[QB];
+        uint2 code[QB];
+        auto load = [&](int q0) {
 #pragma unroll
-          for (int u = 0; u < B; ++u) {
-            w[u] = ld_stream(ws + kSellW * u);
-            code[u] = ld_stream(cs16 + kSellC * u);
+          for (int u = 0; u < QB; ++u) {
+            w[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            code[u] = make_uint2(0u, 0u);
+            if (q0 + u < nq) {
+              w[u] = op.weights(q0 + u);
+              code[u] = op.codes(q0 + u);
+            }
           }
-        }
-        for (int b = 0; b < nb; ++b) {
+        };
+        if (PIPE) load(0);
+        for (int q0 = 0; q0 < nq; q0 += QB) {
           if (PF > 0 && lane == 0 && pf_next < pf_end) {
             bulk_prefetch_l2(pf_next, (unsigned)min((size_t)B * kSellW * 4, (size_t)(pf_end - pf_next)));
             pf_next += B * kSellW * 4;
           }
-          if (!PIPE) {
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-              w[u] = ld_stream(ws + kSellW * (b * B + u));
-              code[u] = ld_stream(cs16 + kSellC * (b * B + u));
-            }
-          }
+          if (!PIPE) load(q0);
           float zv[B];
 #pragma unroll
-          for (int u = 0; u < B; ++u) zv[u] = WIN ? zw[code[u] & 4095u] : __ldg(z + code_node(hb, code[u]));
-          float wc[B];
-#pragma unroll
-          for (int u = 0; u < B; ++u) wc[u] = w[u];
-          if (PIPE && b + 1 < nb) {
-            const int c1 = (b + 1) * B;
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-              w[u] = ld_stream(ws + kSellW * (c1 + u));
-              code[u] = ld_stream(cs16 + kSellC * (c1 + u));
-            }
+          for (int u = 0; u < B; ++u) {
+            const unsigned int cd = quad_code(code[u >> 2], u & 3);
+            zv[u] = WIN ? zw[cd & 4095u] : __ldg(z + code_node(hb, cd));
           }
+          float4 wc[QB];
 #pragma unroll
-          for (int u = 0; u < B; ++u) acc[u & 3] = fmaf(wc[u], zv[u], acc[u & 3]);
-        }
-        for (int c = nb * B; c < width; ++c) {
-          const unsigned int cc = ld_stream(cs16 + kSellC * c);
-          acc[0] = fmaf(ld_stream(ws + kSellW * c), WIN ? zw[cc & 4095u] : __ldg(z + code_node(hb, cc)), acc[0]);
+          for (int u = 0; u < QB; ++u) wc[u] = w[u];
+          if (PIPE && q0 + QB < nq) load(q0 + QB);
+#pragma unroll
+          for (int u = 0; u < B; ++u) acc[u & 3] = fmaf(quad_weight(wc[u >> 2], u & 3), zv[u], acc[u & 3]);
         }
         if (live) {
           const float za = z[a];
@@ -834,6 +785,116 @@ __global__ void __launch_bounds__(kBlock, MINB) k_cg_spmv32(EngineView v) {
       v.ticket[v.M + 1] = 0;
       v.ticket[v.M + 2] = 0;
     }
+  }
+}
+
+// The warp's share of a slice that K warps of a CTA split: part p of K takes the quads p, p + K,
+// ...; the parts' sums meet in shared memory and part 0 finishes the row.  For sizes at which a
+// warp a slice leaves most of the chip's warps empty and a pass is one slice's chain of loads
+// (8,000 nodes: 110 slices of unknowns on 152 SMs).
+template <int K>
+struct SplitSlice {
+  static constexpr int kSlices = (kBlock / 32) / K;  // slices of a CTA at a time
+  int sg, part;
+  __device__ __forceinline__ SplitSlice(int base) : sg(base + (threadIdx.x >> 5) / K), part((threadIdx.x >> 5) % K) {}
+};
+// the parts' sums of NV values a lane: part 0 gets the totals, in part order (sm: kBlock * NV)
+template <int K, int NV, typename T>
+__device__ __forceinline__ void split_sum(T (&v)[NV], T* sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp % K)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sm[(warp * NV + q) * 32 + lane] = v[q];
+  __syncthreads();
+  if (warp % K == 0)
+#pragma unroll
+    for (int h = 1; h < K; ++h)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[q] += sm[((warp + h) * NV + q) * 32 + lane];
+}
+
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_cg_spmv32k(EngineView v) {
+  constexpr int QB = 4;
+  __shared__ float s_acc[kBlock];
+  __shared__ double sm[kBlock / 32];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.ncslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.cslices[have ? ss.sg : 0];
+    const int inst = __ldg(&d.inst);
+    const KParams& k = v.inst[inst];
+    const bool run = have && __ldg(&k.ds->inner_active) != 0;
+    float sum[1] = {0.0f};
+    int a = -1;
+    bool live = false;
+    if (run) {
+      const int width = k.cg_width[ss.sg - __ldg(&v.cslice_first[inst])];
+      a = k.cg_rows[__ldg(&d.row0) + lane];
+      live = a >= 0 && k.freem[a];
+      if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+      __syncwarp();
+      const int* hb = s_hb[warp];
+      const QuadPtr op(sell_cg_w(k, d), lane);
+      const float* z = k.z32;
+      const int nq = (width + 3) >> 2;
+      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (live)
+        for (int q0 = ss.part; q0 < nq; q0 += QB * K) {
+          float4 w[QB];
+          uint2 code[QB];
+#pragma unroll
+          for (int u = 0; u < QB; ++u) {
+            w[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            code[u] = make_uint2(0u, 0u);
+            if (q0 + u * K < nq) {
+              w[u] = op.weights(q0 + u * K);
+              code[u] = op.codes(q0 + u * K);
+            }
+          }
+          float zv[4 * QB];
+#pragma unroll
+          for (int u = 0; u < 4 * QB; ++u) zv[u] = __ldg(z + code_node(hb, quad_code(code[u >> 2], u & 3)));
+#pragma unroll
+          for (int u = 0; u < 4 * QB; ++u) acc[u & 3] = fmaf(quad_weight(w[u >> 2], u & 3), zv[u], acc[u & 3]);
+        }
+      sum[0] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    }
+    split_sum<K, 1>(sum, s_acc);
+    if (have && ss.part == 0) {
+      DotAcc<float> part;
+      if (live) {
+        const float za = k.z32[a];
+        const float sa = k.d32[a] * za - sum[0];
+        const float beta = (float)k.ds->beta;
+        const float qn = sa + beta * k.q32[a];
+        const float pn = za + beta * k.p32[a];
+        k.q32[a] = qn;
+        k.p32[a] = pn;
+        part.add(pn, qn);
+      }
+      part.warp_sum();
+      if (lane == 0) store_pair(v.partials, ss.sg, part.hi, part.lo);
+    }
+    __syncthreads();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
+      double tot[1];
+      reduce_pair_items<1>(v.partials, v.stride, v.cslice_first[i], v.cslice_count[i], tot, sm);
+      if (threadIdx.x == 0) {
+        DevState* ds = v.inst[i].ds;
+        if (ds->inner_active) {
+          ds->alpha = (tot[0] > 0.0 && isfinite(tot[0])) ? ds->rz / tot[0] : 0.0;
+          ds->pq = tot[0];
+        }
+      }
+    }
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
   }
 }
 
@@ -1155,6 +1216,14 @@ __device__ __forceinline__ void win_copy(const EngineView& v, int* ws, int s1, f
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// quad q of a staged chunk (shared memory) times the window values
+__device__ __forceinline__ void staged_quad(const float* stage, int q, int lane, const float* zw, float (&acc)[4]) {
+  const float4 w = reinterpret_cast<const float4*>(stage + kQuadW * q)[lane];
+  const uint2 c = reinterpret_cast<const uint2*>(stage + kQuadW * q + 128)[lane];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc[u] = fmaf(quad_weight(w, u), zw[quad_code(c, u) & 4095u], acc[u]);
+}
+
 template <int W>
 __global__ void __launch_bounds__(kBlock, 1) k_cg_spmv32t(EngineView v) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1207,20 +1276,13 @@ __global__ void __launch_bounds__(kBlock, 1) k_cg_spmv32t(EngineView v) {
         uint64_t* bar = bars + warp * kTmaStages + stage;
         if (!mbar_wait_bounded(bar, (phases >> stage) & 1u, kWaitPolls)) timed_out = d.inst;
         phases ^= 1u << stage;
-        const float* sw = reinterpret_cast<const float*>(ring + (size_t)(warp * kTmaStages + stage) * kStageBytes) + lane;
-        const unsigned short* sc = reinterpret_cast<const unsigned short*>(sw - lane + 32) + lane;
-        const int cc = min(kTmaCol, width - ch * kTmaCol);
+        const float* sw = reinterpret_cast<const float*>(ring + (size_t)(warp * kTmaStages + stage) * kStageBytes);
+        const int cc = min(kTmaCol, width - ch * kTmaCol);  // a multiple of 4
         if (cc == kTmaCol) {
-#pragma unroll 8
-          for (int c = 0; c < kTmaCol; ++c) {
-            const unsigned q = sc[kSellC * c];
-            acc[c & 3] = fmaf(sw[kSellW * c], zw[q & 4095u], acc[c & 3]);
-          }
+#pragma unroll 2
+          for (int q = 0; q < kTmaCol / 4; ++q) staged_quad(sw, q, lane, zw, acc);
         } else {
-          for (int c = 0; c < cc; ++c) {
-            const unsigned q = sc[kSellC * c];
-            acc[c & 3] = fmaf(sw[kSellW * c], zw[q & 4095u], acc[c & 3]);
-          }
+          for (int q = 0; q < cc / 4; ++q) staged_quad(sw, q, lane, zw, acc);
         }
         __syncwarp();
         if (lane == 0) tma_produce(v, pc, s1, warp, stage, ring, bars, pol);
@@ -1378,20 +1440,13 @@ __global__ void __launch_bounds__(kBlock, 1) k_cg_spmv32s(EngineView v, int stag
           phases ^= 1u << stage;
           ready = true;
         }
-        const float* sw = reinterpret_cast<const float*>(myring + (size_t)stage * SB) + lane;
-        const unsigned short* sc = reinterpret_cast<const unsigned short*>(sw - lane + 32) + lane;
-        const int n = min(COL - cis, width - c);
+        const float* sw = reinterpret_cast<const float*>(myring + (size_t)stage * SB);
+        const int n = min(COL - cis, width - c);  // widths, and so cis and n, are multiples of 4
         if (n == COL) {
-#pragma unroll 8
-          for (int q = 0; q < COL; ++q) {
-            const unsigned code = sc[kSellC * q];
-            acc[q & 3] = fmaf(sw[kSellW * q], zw[code & 4095u], acc[q & 3]);
-          }
+#pragma unroll 2
+          for (int q = 0; q < COL / 4; ++q) staged_quad(sw, q, lane, zw, acc);
         } else {
-          for (int q = cis; q < cis + n; ++q) {
-            const unsigned code = sc[kSellC * q];
-            acc[q & 3] = fmaf(sw[kSellW * q], zw[code & 4095u], acc[q & 3]);
-          }
+          for (int q = cis / 4; q < (cis + n) / 4; ++q) staged_quad(sw, q, lane, zw, acc);
         }
         c += n;
         cis += n;
@@ -1445,65 +1500,103 @@ __global__ void __launch_bounds__(kBlock, 1) k_cg_spmv32s(EngineView v, int stag
   }
 }
 
-// FP64 operator: stored FP64 weights, staged FP64 vector values
-template <int W>
-__global__ void __launch_bounds__(kBlock) k_cg_spmv64(EngineView v) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ TileSmem ts;
-  __shared__ double sm[kBlock / 32];
-  __shared__ int s_last;
-  const int sub = threadIdx.x % W, seg = threadIdx.x / W, nseg = kBlock / W;
-  for (int item = blockIdx.x; item < v.ntiles; item += gridDim.x) {
-    const TileDesc t = v.tiles[item];
-    const KParams& k = v.inst[t.inst];
-    const bool active = *((volatile int*)&k.ds->inner_active) != 0;
-    double part[1] = {0.0};
-    if (active) {
-      load_tile(t, ts);
-      double* hs = reinterpret_cast<double*>(dsm);
-      const unsigned short* sslot = stage_slots(k.slot16, t, dsm + align16(sizeof(double) * (size_t)t.halo));
-      const double* z = k.z64;
-      for (int s = threadIdx.x; s < t.halo; s += kBlock) hs[s] = z[halo_node(ts, s)];
-      __syncthreads();
-      const int* row = k.row;
-      const double* w64 = k.w64;
-      const unsigned char* freem = k.freem;
-      double* p = k.p64;
-      double* q = k.q64;
-      const double beta = k.ds->beta;
-      const int own0 = ts.off[4] + (t.own_begin - t.hb[4]);
-      for (int a0 = t.own_begin; a0 < t.own_end; a0 += nseg) {
-        const int a = a0 + seg;
-        const bool act = a < t.own_end && freem[a];
-        double acc = 0.0;
-        if (act)
-          for (int j = row[a] + sub; j < row[a + 1]; j += W) acc = fma(w64[j], hs[sslot[j - t.bond0]], acc);
-        acc = seg_reduce_d<W>(acc);
-        if (act && sub == 0) {
-          const double za = hs[own0 + (a - t.own_begin)];
-          const double s = k.dsum64[a] * za - acc;
-          const double qn = s + beta * q[a];
-          const double pn = za + beta * p[a];
-          q[a] = qn;
-          p[a] = pn;
-          part[0] += pn * qn;
-        }
-      }
+// The FP64 operator's row sums on the CG slices: sum over this part's quads of w x[node] (FP64
+// weights, 32 bytes a lane and quad, next to the codes of the FP32 operator), two quads in flight.
+template <int K>
+__device__ __forceinline__ double cg_row64(const KParams& k, const SliceDesc& d, int width, int lane, int part,
+                                           const int* hb, const double* x) {
+  constexpr int QB = 2;
+  const double* w64 = k.sell_cg64 + (size_t)(d.off >> 5) * 32 + 4 * lane;
+  const QuadPtr op(sell_cg_w(k, d), lane);
+  const int nq = (width + 3) >> 2;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  int q0 = part;
+  for (; q0 + (QB - 1) * K < nq; q0 += QB * K) {
+    double w[QB][4], xv[QB][4];
+    uint2 code[QB];
+#pragma unroll
+    for (int u = 0; u < QB; ++u) {
+      code[u] = op.codes(q0 + u * K);
+      ld_stream_d4(w64 + 128 * (size_t)(q0 + u * K), w[u]);
     }
-    write_partials<1>(v, item, part, sm);
-    if (item_done(&v.ticket[t.inst], v.tile_count[t.inst], &s_last)) {
+#pragma unroll
+    for (int u = 0; u < QB; ++u)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) xv[u][t] = __ldg(x + code_node(hb, quad_code(code[u], t)));
+#pragma unroll
+    for (int u = 0; u < QB; ++u)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) acc[t] = fma(w[u][t], xv[u][t], acc[t]);
+  }
+  for (; q0 < nq; q0 += K) {
+    double w[4];
+    const uint2 code = op.codes(q0);
+    ld_stream_d4(w64 + 128 * (size_t)q0, w);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[t] = fma(w[t], __ldg(x + code_node(hb, quad_code(code, t))), acc[t]);
+  }
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+}
+
+// FP64 operator on the CG slices (q = A z + beta q, p = z + beta p, p.q), one lane a row, K warps
+// a slice: bound by the stream (10 bytes a slot).  512k nodes: 0.1146 ms, against 0.2085
+// for FP64 weights per bond with halo tiles in shared memory (the tile form it replaces).
+template <int K>
+__global__ void __launch_bounds__(kBlock, 4) k_cg_spmv64(EngineView v) {
+  __shared__ double s_acc[K > 1 ? kBlock : 1];
+  __shared__ double sm[kBlock / 32];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.ncslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.cslices[have ? ss.sg : 0];
+    const int inst = __ldg(&d.inst);
+    const KParams& k = v.inst[inst];
+    const int first = __ldg(&v.cslice_first[inst]);
+    double sum[1] = {0.0};
+    int a = -1;
+    bool live = false;
+    if (have && __ldg(&k.ds->inner_active) != 0) {
+      a = k.cg_rows[__ldg(&d.row0) + lane];
+      live = a >= 0 && k.freem[a];
+      if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+      __syncwarp();
+      if (live) sum[0] = cg_row64<K>(k, d, k.cg_width[ss.sg - first], lane, ss.part, s_hb[warp], k.z64);
+    }
+    if (K > 1) split_sum<K, 1>(sum, s_acc);
+    if (have && ss.part == 0) {
+      double part[1] = {0.0};
+      if (live) {
+        const double za = k.z64[a];
+        const double beta = k.ds->beta;
+        const double qn = fma(beta, k.q64[a], fma(k.dsum64[a], za, -sum[0]));
+        const double pn = fma(beta, k.p64[a], za);
+        k.q64[a] = qn;
+        k.p64[a] = pn;
+        part[0] = pn * qn;
+      }
+      part[0] = warp_sum_d(part[0]);
+      slice_partials64<1>(v, inst, first, __ldg(&v.cslice_count[inst]), ss.sg, part);
+    }
+    if (K > 1) __syncthreads();
+    else __syncwarp();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
       double tot[1];
-      reduce_items<1>(v.partials, v.stride, v.tile_first[t.inst], v.tile_count[t.inst], tot, sm);
+      reduce_slices64<1>(v, i, v.cslice_first[i], v.cslice_count[i], tot, sm);
       if (threadIdx.x == 0) {
-        DevState* ds = k.ds;
+        DevState* ds = v.inst[i].ds;
         if (ds->inner_active) {
           ds->alpha = (tot[0] > 0.0 && isfinite(tot[0])) ? ds->rz / tot[0] : 0.0;
           ds->pq = tot[0];
         }
-        v.ticket[t.inst] = 0;
       }
     }
-    __syncthreads();
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
   }
 }
 
@@ -2284,90 +2377,6 @@ __global__ void __launch_bounds__(kBlock) k_warm_apply(EngineView v) {
   }
 }
 
-// phi += e on the unknowns; FP64 residual r -= A e (FP64 weights); outer stop test.
-template <typename P, int W>
-__global__ void __launch_bounds__(kBlock) k_ir_update(EngineView v, cudaGraphConditionalHandle hc) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ TileSmem ts;
-  __shared__ double sm[kBlock / 32];
-  __shared__ int s_last;
-  const int sub = threadIdx.x % W, seg = threadIdx.x / W, nseg = kBlock / W;
-  const bool mixed = sizeof(P) == 4;
-  for (int item = blockIdx.x; item < v.ntiles; item += gridDim.x) {
-    const TileDesc t = v.tiles[item];
-    const KParams& k = v.inst[t.inst];
-    const bool active = *((volatile int*)&k.ds->outer_active) != 0;
-    double part[1] = {0.0};
-    if (active) {
-      load_tile(t, ts);
-      double* hs = reinterpret_cast<double*>(dsm);
-      const unsigned short* sslot = stage_slots(k.slot16, t, dsm + align16(sizeof(double) * (size_t)t.halo));
-      const P* e = VecSel<P>::e(k);
-      for (int s = threadIdx.x; s < t.halo; s += kBlock) hs[s] = (double)e[halo_node(ts, s)];
-      __syncthreads();
-      const int* row = k.row;
-      const double* w64 = k.w64;
-      const unsigned char* freem = k.freem;
-      const int own0 = ts.off[4] + (t.own_begin - t.hb[4]);
-      for (int a0 = t.own_begin; a0 < t.own_end; a0 += nseg) {
-        const int a = a0 + seg;
-        const bool act = a < t.own_end && freem[a];
-        double acc = 0.0;
-        if (mixed) {
-          // A e with the FP32 pair (w32, wlo32) and the FP32 correction e: exact products
-          // (TwoProd), TwoSum accumulation
-          float sh = 0.f, sl = 0.f;
-          if (act)
-            for (int j = row[a] + sub; j < row[a + 1]; j += W) {
-              const float ev = (float)hs[sslot[j - t.bond0]];
-              float ph, pl;
-              pair_mul(k.w32[j], k.wlo32[j], ev, 0.0f, ph, pl);
-              pair_add(sh, sl, ph, pl);
-            }
-          acc = seg_reduce_pair<W>(sh, sl);
-        } else {
-          if (act)
-            for (int j = row[a] + sub; j < row[a + 1]; j += W) acc = fma(w64[j], hs[sslot[j - t.bond0]], acc);
-          acc = seg_reduce_d<W>(acc);
-        }
-        if (act && sub == 0) {
-          const double ea = hs[own0 + (a - t.own_begin)];
-          const double r = k.r64[a] - (k.dsum64[a] * ea - acc);
-          k.r64[a] = r;
-          const double ph = k.phi64[a] + ea;
-          k.phi64[a] = ph;
-          set_phi_rec(k, a, ph, mixed);
-          part[0] += r * r;
-        }
-      }
-    }
-    write_partials<1>(v, item, part, sm);
-    if (item_done(&v.ticket[t.inst], v.tile_count[t.inst], &s_last)) {
-      double tot[1];
-      reduce_items<1>(v.partials, v.stride, v.tile_first[t.inst], v.tile_count[t.inst], tot, sm);
-      if (threadIdx.x == 0) {
-        DevState* ds = k.ds;
-        if (ds->outer_active) {
-          ds->rnorm2 = tot[0];
-          ds->outer_it += 1;
-          ds->outer_total += 1;
-          const bool conv = tot[0] <= ds->tol * ds->tol * ds->bnorm2;
-          const bool go = !conv && ds->outer_it < ds->max_outer && ds->solve_iters < ds->max_iter &&
-                          isfinite(tot[0]);
-          if (!go) {
-            ds->cg_solves += 1;
-            ds->last_relres = sqrt(tot[0] / ds->bnorm2);
-            if (!conv) ds->cg_nc += 1;
-          }
-          ds->outer_active = go ? 1 : 0;
-        }
-        instance_finished(v, t.inst, 0, hc);
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // ---------------------------------------------------- potential residuals on the slices ----
 // Mixed path: the prep and the refinement residual as slice kernels over the sliced operator
 // (one lane per row, bond columns streamed in batches of 8, neighbour values gathered through
@@ -2380,7 +2389,93 @@ __device__ __forceinline__ const float* sell_lo_col(const KParams& k, const Slic
   return k.sell_lo + (size_t)(d.off >> 5) * 32;
 }
 
-// per node {phi_hi, phi_lo} (zero on solid nodes), liquid flag, potential-Dirichlet flag
+// A lane's row of the CG operator as the preps write it: bonds are collected four at a time and
+// stored as a quad (one 16- or 32-byte and one 8-byte store instead of scattered words).  W: float
+// with low words, or double.
+template <typename W>
+struct CgRowWriter {
+  float* sell;            // the slice's interleaved array (weights unless W is double, codes)
+  float* lo;              // the weights' low words (W = float)
+  double* w64;            // the FP64 weights (W = double)
+  int lane, n;
+  W w[4];
+  float l[4];
+  unsigned int c[4];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      w[u] = W(0);
+      l[u] = 0.0f;
+      c[u] = 0u;
+    }
+  }
+  __device__ __forceinline__ void flush(int q) {
+    float* base = sell + (size_t)q * kQuadW;
+    reinterpret_cast<uint2*>(base + 128)[lane] = make_uint2(c[0] | c[1] << 16, c[2] | c[3] << 16);
+    if constexpr (sizeof(W) == 4) {
+      reinterpret_cast<float4*>(base)[lane] = make_float4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<float4*>(lo + (size_t)q * 128)[lane] = make_float4(l[0], l[1], l[2], l[3]);
+    } else {
+      double2* o = reinterpret_cast<double2*>(w64 + (size_t)q * 128 + 4 * lane);
+      o[0] = make_double2(w[0], w[1]);
+      o[1] = make_double2(w[2], w[3]);
+    }
+    clear();
+  }
+  __device__ __forceinline__ void add(W weight, float low, unsigned int code) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if ((n & 3) == u) {
+        w[u] = weight;
+        l[u] = low;
+        c[u] = code;
+      }
+    if ((++n & 3) == 0) flush((n >> 2) - 1);
+  }
+  // the last quad and zero quads up to the slice's capacity (columns, a multiple of 4)
+  __device__ __forceinline__ void finish(int capacity) {
+    for (int q = n >> 2; q < capacity >> 2; ++q) flush(q);
+  }
+};
+
+// an instance's decision after the prep from ||b||^2 and ||r||^2 (one thread)
+__device__ __forceinline__ void prep_decide(DevState* ds, double bb, double rr) {
+  ds->op_valid = 1;
+  const double bn = bb > 0.0 ? bb : 1.0;
+  ds->bnorm2 = bn;
+  ds->rnorm2 = rr;
+  ds->outer_it = 0;
+  ds->solve_iters = 0;
+  const bool go = rr > ds->tol * ds->tol * bn && ds->max_outer > 0;
+  if (!go) {
+    ds->cg_solves += 1;
+    ds->last_relres = sqrt(rr / bn);
+  }
+  ds->outer_active = go ? 1 : 0;
+  ds->inner_active = 0;
+}
+
+// bond columns c0 .. c0 + nc - 1 (whole quads) of the slice: weights as FP32 pairs, codes
+__device__ __forceinline__ void load_residual_quads(const QuadPtr& op, const float4* lo, int c0, int nc,
+                                                    float (&w)[kResB], float (&wl)[kResB],
+                                                    unsigned int (&code)[kResB]) {
+#pragma unroll
+  for (int q = 0; q < kResB / 4; ++q)
+    if (4 * q < nc) {
+      const float4 wq = op.weights((c0 >> 2) + q), lq = ld_stream(lo + 32 * ((c0 >> 2) + q));
+      const uint2 cq = op.codes((c0 >> 2) + q);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        w[4 * q + u] = quad_weight(wq, u);
+        wl[4 * q + u] = quad_weight(lq, u);
+        code[4 * q + u] = quad_code(cq, u);
+      }
+    }
+}
+
+// per node {phi_hi, phi_lo} (zero on solid nodes), liquid flag, potential-Dirichlet flag; the FP64
+// path's preps read the potential from z64 instead
+template <typename P>
 __global__ void __launch_bounds__(kBlock) k_phi4(EngineView v) {
   // a prep that forms the mask sums rewrites the CG operator's rows: their slices' longest
   // rows start from zero
@@ -2393,8 +2488,9 @@ __global__ void __launch_bounds__(kBlock) k_phi4(EngineView v) {
     const Chunk c = v.chunks[item];
     const KParams& k = v.inst[c.inst];
     for (int a = c.begin + threadIdx.x; a < c.end; a += kBlock) {
-      const bool liq = k.rec32_cur[a].phase == 0.0f;
+      const bool liq = phase_of<P>(k, a) == 0.0f;
       const double ph = k.phi64[a];
+      if (sizeof(P) == 8) k.z64[a] = liq ? ph : 0.0;
       const float hi = (float)ph;
       const float lo = (float)(ph - (double)hi);
       k.phi4[a] = make_float4(liq ? hi : 0.0f, liq ? lo : 0.0f, liq ? 1.0f : 0.0f,
@@ -2428,9 +2524,8 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
     }
     const bool scan = rowok && fa.z != 0.0f && fa.w == 0.0f;
     const int* hb = s_hb[warp];
-    const float* ws = sell_w(k, d) + lane;
-    const float* wls = sell_lo_col(k, d) + lane;
-    const unsigned short* cs = sell_code(k, d) + lane;
+    const QuadPtr op(sell_w(k, d), lane);
+    const float4* wls = reinterpret_cast<const float4*>(sell_lo_col(k, d)) + lane;
     // sum_j w phi_j over the liquid columns as an FP32 pair in bond order (the cached pass
     // adds the solid columns' exact zeros, so both passes give the same bits).  The mask
     // sums also write the row into the CG operator's slices: its bonds to possible unknowns
@@ -2438,35 +2533,28 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
     // padding, and the slice's longest row.
     const int cpos = scan && !cached ? k.cg_pos[a] : -1;
     const SliceDesc* cd = nullptr;
-    float* wcg = nullptr;
-    float* wlcg = nullptr;
-    unsigned short* ccg = nullptr;
+    CgRowWriter<float> out;
     int cby = 0, cbz = 0;
     if (cpos >= 0) {
       cd = v.cslices + v.cslice_first[d.inst] + (cpos >> 5);
       const size_t col0 = (size_t)(cd->off >> 5);
-      wcg = k.sell_cg + col0 * kSellW + (cpos & 31);
-      wlcg = k.sell_cg_lo + col0 * 32 + (cpos & 31);
-      ccg = reinterpret_cast<unsigned short*>(k.sell_cg + col0 * kSellW + 32) + (cpos & 31);
+      out.sell = k.sell_cg + col0 * kSellW;
+      out.lo = k.sell_cg_lo + col0 * 32;
+      out.lane = cpos & 31;
+      out.n = 0;
+      out.clear();
       cby = cd->tile & 0xffff;
       cbz = cd->tile >> 16;
     }
-    int ncg = 0;
     float dh = 0.f, dl = 0.f, sh = 0.f, sl = 0.f, ch = 0.f, cl = 0.f;
     int anyll = 0;
     if (__any_sync(0xffffffffu, scan)) {
       const int width = d.width;
       for (int c0 = 0; c0 < width; c0 += kResB) {
-        const int nc = min(kResB, width - c0);
+        const int nc = min(kResB, width - c0);  // a multiple of 4
         float w[kResB], wl[kResB];
         unsigned int code[kResB];
-#pragma unroll
-        for (int u = 0; u < kResB; ++u)
-          if (u < nc) {
-            w[u] = ld_stream(ws + kSellW * (c0 + u));
-            wl[u] = ld_stream(wls + 32 * (c0 + u));
-            code[u] = ld_stream(cs + kSellC * (c0 + u));
-          }
+        load_residual_quads(op, wls, c0, nc, w, wl, code);
         if (cached) {
           float2 f[kResB];
 #pragma unroll
@@ -2499,22 +2587,15 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
               const int m = code_node(hb, code[u]);
               const int xr = k.xrow[m];
               const int r = ((xr & 0xffff) - cby + 1) + 3 * ((xr >> 16) - cbz + 1);
-              wcg[(size_t)kSellW * ncg] = w[u];
-              wlcg[(size_t)32 * ncg] = wl[u];
-              ccg[(size_t)kSellC * ncg] = (unsigned short)((r << 12) | (m - cd->gbase[r]));
-              ++ncg;
+              out.add(w[u], wl[u], (unsigned int)((r << 12) | (m - cd->gbase[r])));
             }
           }
       }
     }
     if (cpos >= 0) {
       // zero padding up to the slice's capacity (its longest full row)
-      for (int c = ncg; c < cd->width; ++c) {
-        wcg[(size_t)kSellW * c] = 0.0f;
-        wlcg[(size_t)32 * c] = 0.0f;
-        ccg[(size_t)kSellC * c] = 0;
-      }
-      atomicMax(&k.cg_width[cpos >> 5], ncg);
+      out.finish(cd->width);
+      atomicMax(&k.cg_width[cpos >> 5], out.n);
     }
     float b2h = 0.0f, b2l = 0.0f, r2h = 0.0f, r2l = 0.0f;  // b.b and r.r as FP32 pairs
     if (rowok) {
@@ -2566,20 +2647,7 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
       double tot[2];
       reduce_pair_items<2>(v.partials, v.stride, v.slice_first[i], v.slice_count[i], tot, sm);
       if (threadIdx.x == 0) {
-        DevState* ds = v.inst[i].ds;
-        ds->op_valid = 1;
-        const double bn = tot[0] > 0.0 ? tot[0] : 1.0;
-        ds->bnorm2 = bn;
-        ds->rnorm2 = tot[1];
-        ds->outer_it = 0;
-        ds->solve_iters = 0;
-        const bool go = tot[1] > ds->tol * ds->tol * bn && ds->max_outer > 0;
-        if (!go) {
-          ds->cg_solves += 1;
-          ds->last_relres = sqrt(tot[1] / bn);
-        }
-        ds->outer_active = go ? 1 : 0;
-        ds->inner_active = 0;
+        prep_decide(v.inst[i].ds, tot[0], tot[1]);
         instance_finished(v, i, 0, hc);
       }
       __syncthreads();
@@ -2588,6 +2656,310 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
       v.ticket[v.M + 1] = 0;
       v.ticket[v.M + 2] = 0;
     }
+  }
+}
+
+// The FP64 path's prep on the transport's slices (k_prep_slices with FP64 weights and sums): b,
+// r = b - A phi and their norms, K warps a slice; phi of the liquid nodes (zero on solid ones)
+// is gathered from z64 (written by k_phi4, free until the CG starts).  While the mask sums
+// hold (op_valid) only sum_j w phi_j is formed; otherwise part 0 forms the row's sums alone and
+// writes its bonds to possible unknowns into the CG slices.
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_prep64(EngineView v, cudaGraphConditionalHandle hc) {
+  __shared__ double s_acc[K > 1 ? kBlock : 1];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ double sm[2 * kBlock / 32];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.nslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.slices[have ? ss.sg : 0];
+    const KParams& k = v.inst[d.inst];
+    const bool cached = k.ds->op_valid != 0;
+    if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+    __syncwarp();
+    const int* hb = s_hb[warp];
+    const int a = d.row0 + lane;
+    const bool rowok = have && lane < d.nrows;
+    float4 fa = make_float4(0.f, 0.f, 0.f, 0.f);
+    int len = 0;
+    if (rowok) {
+      fa = k.phi4[a];
+      len = k.row[a + 1] - k.row[a];
+    }
+    const bool scan = rowok && fa.z != 0.0f && fa.w == 0.0f;
+    const QuadPtr op(sell_w(k, d), lane);
+    const double* w64 = k.sell64 + (size_t)(d.off >> 5) * 32 + 4 * lane;
+    const double* phil = k.z64;
+    double dsum = 0.0, cpl = 0.0;
+    int anyll = 0;
+    // sum_j w phi_j over the liquid columns (zero elsewhere), the same order whether the rows are
+    // cached or not: a step that is repeated from a restored state gives the same bits
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (scan && (cached ? k.freem[a] != 0 : K > 1)) {
+      const int nq = (len + 3) >> 2;
+#pragma unroll 2
+      for (int q = ss.part; q < nq; q += K) {
+        double w[4];
+        const uint2 code = op.codes(q);
+        ld_stream_d4(w64 + 128 * (size_t)q, w);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc[t] = fma(w[t], __ldg(phil + code_node(hb, quad_code(code, t))), acc[t]);
+      }
+    }
+    if (!cached && ss.part == 0) {
+      const int cpos = scan ? k.cg_pos[a] : -1;
+      const SliceDesc* cd = nullptr;
+      CgRowWriter<double> out;
+      int cby = 0, cbz = 0;
+      if (cpos >= 0) {
+        cd = v.cslices + v.cslice_first[d.inst] + (cpos >> 5);
+        const size_t col0 = (size_t)(cd->off >> 5);
+        out.w64 = k.sell_cg64 + col0 * 32;
+        out.sell = k.sell_cg + col0 * kSellW;
+        out.lane = cpos & 31;
+        out.n = 0;
+        out.clear();
+        cby = cd->tile & 0xffff;
+        cbz = cd->tile >> 16;
+      }
+      if (scan)
+        for (int q = 0; 4 * q < len; ++q) {
+          double w[4];
+          const uint2 code = op.codes(q);
+          ld_stream_d4(w64 + 128 * (size_t)q, w);
+          float4 f[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) f[t] = __ldg(k.phi4 + code_node(hb, quad_code(code, t)));
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            if (4 * q + t >= len || f[t].z == 0.0f) continue;
+            const int m = code_node(hb, quad_code(code, t));
+            const double ph = phil[m];
+            dsum += w[t];
+            if (K == 1) acc[t] = fma(w[t], ph, acc[t]);
+            anyll = 1;
+            if (f[t].w != 0.0f) {
+              cpl += w[t] * ph;
+            } else if (cpos >= 0) {
+              const int xr = k.xrow[m];
+              const int r = ((xr & 0xffff) - cby + 1) + 3 * ((xr >> 16) - cbz + 1);
+              out.add(w[t], 0.0f, (unsigned int)((r << 12) | (m - cd->gbase[r])));
+            }
+          }
+        }
+      if (cpos >= 0) {
+        out.finish(cd->width);
+        atomicMax(&k.cg_width[cpos >> 5], out.n);
+      }
+    }
+    double swphi[1] = {(acc[0] + acc[1]) + (acc[2] + acc[3])};
+    if (K > 1) split_sum<K, 1>(swphi, s_acc);
+    if (have && ss.part == 0) {
+      double part[2] = {0.0, 0.0};
+      if (rowok) {
+        double b;
+        if (k.b_override) {
+          b = k.b_override[a];
+        } else {
+          double R11 = 0.0;
+          for (int s = 0; s < S; ++s) R11 += k.z[s] * conc_of<double>(k, a, s);
+          b = k.lam * R11;
+        }
+        bool fr;
+        if (cached) {
+          fr = k.freem[a] != 0;
+          dsum = k.dsum64[a];
+          cpl = k.cpl64[a];
+        } else {
+          fr = scan && anyll;
+          k.freem[a] = fr ? 1 : 0;
+          k.dsum64[a] = fr ? dsum : 1.0;
+          k.cpl64[a] = fr ? cpl : 0.0;
+          k.dinv64[a] = fr ? 1.0 / dsum : 0.0;
+          k.d32[a] = fr ? (float)dsum : 1.0f;
+          k.dinv32[a] = fr ? (float)(1.0 / dsum) : 0.0f;
+        }
+        const double bb = fr ? b : 0.0;
+        const double r = fr ? bb - (dsum * k.phi64[a] - swphi[0]) : 0.0;
+        k.b64[a] = bb;
+        k.r64[a] = r;
+        const double be = bb + (fr ? cpl : 0.0);
+        part[0] = be * be;
+        part[1] = r * r;
+      }
+      part[0] = warp_sum_d(part[0]);
+      part[1] = warp_sum_d(part[1]);
+      slice_partials64<2>(v, d.inst, v.slice_first[d.inst], v.slice_count[d.inst], ss.sg, part);
+    }
+    if (K > 1) __syncthreads();
+    else __syncwarp();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
+      double tot[2];
+      reduce_slices64<2>(v, i, v.slice_first[i], v.slice_count[i], tot, sm);
+      if (threadIdx.x == 0) {
+        prep_decide(v.inst[i].ds, tot[0], tot[1]);
+        instance_finished(v, i, 0, hc);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
+  }
+}
+
+// an instance's outer decision from ||r||^2 after a refinement (one thread)
+__device__ __forceinline__ void refine_decide(DevState* ds, double rr) {
+  if (!ds->outer_active) return;
+  ds->rnorm2 = rr;
+  ds->outer_it += 1;
+  ds->outer_total += 1;
+  const bool conv = rr <= ds->tol * ds->tol * ds->bnorm2;
+  const bool go = !conv && ds->outer_it < ds->max_outer && ds->solve_iters < ds->max_iter && isfinite(rr);
+  if (!go) {
+    ds->cg_solves += 1;
+    ds->last_relres = sqrt(rr / ds->bnorm2);
+    if (!conv) ds->cg_nc += 1;
+  }
+  ds->outer_active = go ? 1 : 0;
+}
+
+// the refinement with K warps a slice (small cases): k_ir_slices below, the pairs of the parts'
+// sums added in part order
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_ir_split(EngineView v, cudaGraphConditionalHandle hc) {
+  __shared__ float2 s_sum[kBlock];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ double sm[kBlock / 32];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.ncslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.cslices[have ? ss.sg : 0];
+    const int inst = __ldg(&d.inst);
+    const KParams& k = v.inst[inst];
+    float sh = 0.f, sl = 0.f;
+    int a = -1;
+    bool live = false;
+    if (have && *((volatile int*)&k.ds->outer_active) != 0) {
+      if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+      __syncwarp();
+      a = k.cg_rows[__ldg(&d.row0) + lane];
+      live = a >= 0 && k.freem[a];
+      const int len = __any_sync(0xffffffffu, live) ? (k.cg_width[ss.sg - __ldg(&v.cslice_first[inst])] + 3) & ~3 : 0;
+      const QuadPtr op(sell_cg_w(k, d), lane);
+      const float4* wls = reinterpret_cast<const float4*>(k.sell_cg_lo + (size_t)(__ldg(&d.off) >> 5) * 32) + lane;
+      for (int c0 = kResB * ss.part; c0 < len; c0 += kResB * K) {
+        const int nc = min(kResB, len - c0);
+        float w[kResB], wl[kResB], ev[kResB];
+        unsigned int code[kResB];
+        load_residual_quads(op, wls, c0, nc, w, wl, code);
+#pragma unroll
+        for (int u = 0; u < kResB; ++u)
+          if (u < nc) ev[u] = __ldg(k.e32 + code_node(s_hb[warp], code[u]));
+#pragma unroll
+        for (int u = 0; u < kResB; ++u)
+          if (u < nc) {
+            float ph, pl;
+            pair_mul(w[u], wl[u], ev[u], 0.0f, ph, pl);
+            pair_add(sh, sl, ph, pl);
+          }
+      }
+    }
+    if (ss.part) s_sum[threadIdx.x] = make_float2(sh, sl);
+    __syncthreads();
+    if (have && ss.part == 0) {
+#pragma unroll
+      for (int h = 1; h < K; ++h) pair_add(sh, sl, s_sum[threadIdx.x + 32 * h].x, s_sum[threadIdx.x + 32 * h].y);
+      float rh = 0.0f, rl = 0.0f;
+      if (live) {
+        const double ea = (double)k.e32[a];
+        const double r = k.r64[a] - (k.dsum64[a] * ea - ((double)sh + (double)sl));
+        k.r64[a] = r;
+        const double ph = k.phi64[a] + ea;
+        k.phi64[a] = ph;
+        set_phi_rec(k, a, ph, true);
+        pair_square(r, rh, rl);
+      }
+      pair_warp_sum(rh, rl);
+      if (lane == 0) store_pair(v.partials, ss.sg, rh, rl);
+    }
+    __syncthreads();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
+      double tot[1];
+      reduce_pair_items<1>(v.partials, v.stride, v.cslice_first[i], v.cslice_count[i], tot, sm);
+      if (threadIdx.x == 0) {
+        refine_decide(v.inst[i].ds, tot[0]);
+        instance_finished(v, i, 0, hc);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
+  }
+}
+
+// FP64 path: phi += e on the unknowns, r -= A e, outer stop test
+template <int K>
+__global__ void __launch_bounds__(kBlock, 4) k_ir64(EngineView v, cudaGraphConditionalHandle hc) {
+  __shared__ double s_acc[K > 1 ? kBlock : 1];
+  __shared__ double sm[kBlock / 32];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.ncslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.cslices[have ? ss.sg : 0];
+    const int inst = __ldg(&d.inst);
+    const KParams& k = v.inst[inst];
+    const int first = __ldg(&v.cslice_first[inst]);
+    double sum[1] = {0.0};
+    int a = -1;
+    bool live = false;
+    if (have && *((volatile int*)&k.ds->outer_active) != 0) {
+      a = k.cg_rows[__ldg(&d.row0) + lane];
+      live = a >= 0 && k.freem[a];
+      if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+      __syncwarp();
+      if (live) sum[0] = cg_row64<K>(k, d, k.cg_width[ss.sg - first], lane, ss.part, s_hb[warp], k.e64);
+    }
+    if (K > 1) split_sum<K, 1>(sum, s_acc);
+    if (have && ss.part == 0) {
+      double part[1] = {0.0};
+      if (live) {
+        const double ea = k.e64[a];
+        const double r = k.r64[a] - (k.dsum64[a] * ea - sum[0]);
+        k.r64[a] = r;
+        const double ph = k.phi64[a] + ea;
+        k.phi64[a] = ph;
+        set_phi_rec(k, a, ph, false);
+        part[0] = r * r;
+      }
+      part[0] = warp_sum_d(part[0]);
+      slice_partials64<1>(v, inst, first, __ldg(&v.cslice_count[inst]), ss.sg, part);
+    }
+    if (K > 1) __syncthreads();
+    else __syncwarp();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
+      double tot[1];
+      reduce_slices64<1>(v, i, v.cslice_first[i], v.cslice_count[i], tot, sm);
+      if (threadIdx.x == 0) {
+        refine_decide(v.inst[i].ds, tot[0]);
+        instance_finished(v, i, 0, hc);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
   }
 }
 
@@ -2611,24 +2983,17 @@ __global__ void __launch_bounds__(kBlock) k_ir_slices(EngineView v, cudaGraphCon
       // the CG operator's slices: the correction e is zero off the unknowns
       const int a = k.cg_rows[__ldg(&d.row0) + lane];
       const bool live = a >= 0 && k.freem[a];
-      const int len = __any_sync(0xffffffffu, live) ? k.cg_width[sg - __ldg(&v.cslice_first[inst])] : 0;
+      const int len = __any_sync(0xffffffffu, live) ? (k.cg_width[sg - __ldg(&v.cslice_first[inst])] + 3) & ~3 : 0;
       const int* hb = s_hb[warp];
-      const float* ws = sell_cg_w(k, d) + lane;
-      const float* wls = k.sell_cg_lo + (size_t)(__ldg(&d.off) >> 5) * 32 + lane;
-      const unsigned short* cs = sell_cg_code(k, d) + lane;
+      const QuadPtr op(sell_cg_w(k, d), lane);
+      const float4* wls = reinterpret_cast<const float4*>(k.sell_cg_lo + (size_t)(__ldg(&d.off) >> 5) * 32) + lane;
       const float* e = k.e32;
       float sh = 0.f, sl = 0.f;
       for (int c0 = 0; c0 < len; c0 += kResB) {
         const int nc = min(kResB, len - c0);
         float w[kResB], wl[kResB], ev[kResB];
         unsigned int code[kResB];
-#pragma unroll
-        for (int u = 0; u < kResB; ++u)
-          if (u < nc) {
-            w[u] = ld_stream(ws + kSellW * (c0 + u));
-            wl[u] = ld_stream(wls + 32 * (c0 + u));
-            code[u] = ld_stream(cs + kSellC * (c0 + u));
-          }
+        load_residual_quads(op, wls, c0, nc, w, wl, code);
 #pragma unroll
         for (int u = 0; u < kResB; ++u)
           if (u < nc) ev[u] = __ldg(e + code_node(hb, code[u]));
@@ -2659,21 +3024,7 @@ __global__ void __launch_bounds__(kBlock) k_ir_slices(EngineView v, cudaGraphCon
       double tot[1];
       reduce_pair_items<1>(v.partials, v.stride, v.cslice_first[i], v.cslice_count[i], tot, sm);
       if (threadIdx.x == 0) {
-        DevState* ds = v.inst[i].ds;
-        if (ds->outer_active) {
-          ds->rnorm2 = tot[0];
-          ds->outer_it += 1;
-          ds->outer_total += 1;
-          const bool conv = tot[0] <= ds->tol * ds->tol * ds->bnorm2;
-          const bool go = !conv && ds->outer_it < ds->max_outer && ds->solve_iters < ds->max_iter &&
-                          isfinite(tot[0]);
-          if (!go) {
-            ds->cg_solves += 1;
-            ds->last_relres = sqrt(tot[0] / ds->bnorm2);
-            if (!conv) ds->cg_nc += 1;
-          }
-          ds->outer_active = go ? 1 : 0;
-        }
+        refine_decide(v.inst[i].ds, tot[0]);
         instance_finished(v, i, 0, hc);
       }
       __syncthreads();
@@ -2712,20 +3063,6 @@ __device__ __forceinline__ void finish_instance(const KParams& k, const double (
   }
 }
 
-__device__ __forceinline__ void transport_finish(const EngineView& v, const TileDesc& t,
-                                                 const KParams& k, int item,
-                                                 double (&part)[kDiagSlots], double* sm,
-                                                 int* s_last) {
-  write_partials<kDiagSlots>(v, item, part, sm);
-  if (!item_done(&v.ticket[t.inst], v.tile_count[t.inst], s_last)) return;
-  double tot[kDiagSlots];
-  reduce_items<kDiagSlots>(v.partials, v.stride, v.tile_first[t.inst], v.tile_count[t.inst], tot, sm);
-  if (threadIdx.x == 0) {
-    v.ticket[t.inst] = 0;
-    finish_instance(k, tot);
-  }
-}
-
 // The solution of this step's solve and its image A x = b - r into the warm-start ring.
 __device__ __forceinline__ void record_history(const KParams& k, int a, int hslot) {
   if (k.hist_m < 3) return;
@@ -2759,6 +3096,13 @@ __device__ __forceinline__ void ld_rec32(const float4* p, float4& c, float4& t) 
       : "l"(p));
 }
 
+// an FP64 record's concentrations and {phi, phase} in a 256-bit and a 128-bit read-only load
+__device__ __forceinline__ void ld_rec64(const Rec64* p, double (&c)[S], double (&t)[2]) {
+  const double* q = reinterpret_cast<const double*>(p);
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(c[0]), "=d"(c[1]), "=d"(c[2]), "=d"(c[3]) : "l"(q));
+  asm("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(t[0]), "=d"(t[1]) : "l"(q + 4));
+}
+
 // Mixed transport of one 32-row slice sg.  RESID: write F_k = sum_KRk1 + sum_KRk2 - R_k
 // (utils.h:177) to F_out (single instance) and change nothing; otherwise advance the state
 // into rec32_nxt / clo and store the slice's diagnostics partials.  One lane per node streams
@@ -2766,10 +3110,10 @@ __device__ __forceinline__ void ld_rec32(const float4* p, float4& c, float4& t) 
 // gathers each neighbour's 32-byte record through rec(i), where i = hb[code >> 12] +
 // (code & 4095) and hb[r] = gbase[r] - radj[r] (radj == nullptr: i is the node).  hb is the
 // warp's 9-int table in shared memory.
-// bond columns per batch of the FP32 transport: with 256-bit record loads 7 (128 registers,
-// 2 CTAs an SM) measured 0.358 ms at 512k against 0.366 for 6 (8 spills); with two 16-byte
-// loads a record 6 took 0.378 ms, 5 0.389, 4 0.405, 2 0.467
-constexpr int kTrB = 7;
+// bond columns per batch of the FP32 transport, two quads: 128 registers, 2 CTAs an SM.  Weights
+// and codes by the quad (16 and 8 bytes a lane) take 0.318 ms at 512k; by the column (4 and 2
+// bytes, batches of 7) 0.358
+constexpr int kTrB = 8;
 template <bool RESID, int B, bool EARLY, bool PIPE, typename Rec>
 __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int lane, int* hbw,
                                                 const int* radj, Rec rec, double* F_out) {
@@ -2782,21 +3126,26 @@ __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int
   for (int q = 0; q < 6; ++q) ph_hi[q] = ph_lo[q] = 0.0f;
   int n_solid = 0, n_bad = 0;
   const int a = __ldg(&d.row0) + lane;
-  if (lane < __ldg(&d.nrows)) {
+  const bool rowok = lane < __ldg(&d.nrows);
+  float a1[S], a2[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) a1[s] = a2[s] = 0.0f;
+  int iface = 0;
+  float4 ca = make_float4(0.0f, 0.0f, 0.0f, 0.0f), cb = ca;  // the node's record: c | phi_hi, phi_lo, phase, pad
+  float pa = 0.0f;
+  if (rowok) {
     const float4* rc = reinterpret_cast<const float4*>(k.rec32_cur);
     const double BV = *k.bv_ptr;
-    float cLL[S], cX[S], cSS[S], K1f[S], K2f[S];
+    float cLL[S], cX[S], cSS[S];
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      cLL[s] = (float)k.DL[s];
-      cX[s] = (float)(s == 0 ? k.DSo[0] * BV : k.DSo[s]);
-      cSS[s] = s == 0 ? (float)k.DSo[0] : 0.0f;
-      K1f[s] = (float)k.K1[s];
-      K2f[s] = (float)k.K2zF[s];
+      cLL[s] = k.DLf[s];
+      cX[s] = s == 0 ? (float)(k.DSo[0] * BV) : k.DSof[s];
+      cSS[s] = s == 0 ? k.DSof[0] : 0.0f;
     }
-    const float4 ca = rc[2 * a];
-    const float4 cb = rc[2 * a + 1];  // phi_hi, phi_lo, phase, pad
-    const float pa = cb.z;
+    ca = rc[2 * a];
+    cb = rc[2 * a + 1];
+    pa = cb.z;
     // bond coefficient by the neighbour's phase (utils.h:100-153): liquid-liquid D_liquid,
     // mixed D_solid (BV for Mg), solid-solid D_solid for Mg only
     float cfL[S], cfS[S];
@@ -2805,45 +3154,48 @@ __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int
       cfL[s] = pa == 0.0f ? cLL[s] : cX[s];
       cfS[s] = pa == 0.0f ? cX[s] : cSS[s];
     }
-    float a1[S], a2[S];
-#pragma unroll
-    for (int s = 0; s < S; ++s) a1[s] = a2[s] = 0.0f;
-    int iface = 0;
-    const float* ws = sell_w(k, d) + lane;
-    const unsigned short* cs = sell_code(k, d) + lane;
+    const QuadPtr op(sell_w(k, d), lane);
     const int len = k.row[a + 1] - k.row[a];
     // bonds in batches of B columns: the batch's streamed codes and weights, then its
     // neighbour records, all in flight before the arithmetic (column order is kept, so the
     // sums do not depend on the batch size)
     // PIPE: the next batch's codes and weights are loaded before the current batch's terms
-    float wn[PIPE ? B : 1];
-    unsigned int coden[PIPE ? B : 1];
+    constexpr int QB = B / 4;
+    float4 wn[PIPE ? QB : 1];
+    uint2 coden[PIPE ? QB : 1];
     if (PIPE)
 #pragma unroll
-      for (int u = 0; u < B; ++u)
-        if (u < len) {
-          wn[PIPE ? u : 0] = ld_stream(ws + kSellW * u);
-          coden[PIPE ? u : 0] = ld_stream(cs + kSellC * u);
+      for (int u = 0; u < QB; ++u)
+        if (4 * u < len) {
+          wn[PIPE ? u : 0] = op.weights(u);
+          coden[PIPE ? u : 0] = op.codes(u);
         }
     for (int c0 = 0; c0 < len; c0 += B) {
-      float w[B];
-      unsigned int code[B];
+      float4 wq[QB];
+      uint2 cq[QB];
 #pragma unroll
-      for (int u = 0; u < B; ++u)
+      for (int u = 0; u < QB; ++u)
         if (PIPE) {
-          w[u] = wn[PIPE ? u : 0];
-          code[u] = coden[PIPE ? u : 0];
-        } else if (c0 + u < len) {
-          w[u] = ld_stream(ws + kSellW * (c0 + u));
-          code[u] = ld_stream(cs + kSellC * (c0 + u));
+          wq[u] = wn[PIPE ? u : 0];
+          cq[u] = coden[PIPE ? u : 0];
+        } else if (c0 + 4 * u < len) {
+          wq[u] = op.weights((c0 >> 2) + u);
+          cq[u] = op.codes((c0 >> 2) + u);
         }
       if (PIPE)
 #pragma unroll
-        for (int u = 0; u < B; ++u)
-          if (c0 + B + u < len) {
-            wn[PIPE ? u : 0] = ld_stream(ws + kSellW * (c0 + B + u));
-            coden[PIPE ? u : 0] = ld_stream(cs + kSellC * (c0 + B + u));
+        for (int u = 0; u < QB; ++u)
+          if (c0 + B + 4 * u < len) {
+            wn[PIPE ? u : 0] = op.weights(((c0 + B) >> 2) + u);
+            coden[PIPE ? u : 0] = op.codes(((c0 + B) >> 2) + u);
           }
+      float w[B];
+      unsigned int code[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        w[u] = quad_weight(wq[u >> 2], u & 3);
+        code[u] = quad_code(cq[u >> 2], u & 3);
+      }
       // EARLY: the batch's records all in flight before the arithmetic (L1/L2 latency);
       // otherwise each one just before its bond's terms (shared memory)
       float4 cn[EARLY ? B : 1], nb[EARLY ? B : 1];
@@ -2873,6 +3225,8 @@ __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int
     const bool src_on = iface && !(dm & 1);
     const double swv = src_on ? dissolve_switch((double)ca.x + (double)lo4.x, k.csat, k.sw) : 0.0;
     const float Rmg = src_on ? (float)(-k.k_diss * swv) : 0.0f;
+    const float* K1f = k.K1f;
+    const float* K2f = k.K2zFf;
     if (RESID) {
 #pragma unroll
       for (int s = 0; s < S; ++s)
@@ -2881,7 +3235,7 @@ __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int
     } else {
       // c + dt (K1 a1 + K2 a2 + R) on the compensated pair (hi, lo), renormalised: hi is
       // the FP32 rounding of the exact pair sum and lo its exact remainder
-      const float dtf = (float)k.dt;
+      const float dtf = k.dtf;
       float hi[S], lo[S];
       bool bad = false;
 #pragma unroll
@@ -2983,7 +3337,7 @@ __device__ __forceinline__ void transport_last_cta(const EngineView& v, double* 
 // Mixed transport, neighbour records gathered from L1/L2.  Warps claim slices one at a time
 // (slices of solid nodes, narrow and partial slices cost less than full ones); the residual
 // form, which has no last CTA to reset the counter, keeps the static split.
-template <int W, bool RESID>
+template <bool RESID>
 __global__ void __launch_bounds__(kBlock, 2) k_transport32(EngineView v, double* F_out) {
   __shared__ int s_hb[kBlock / 32][12];
   __shared__ double sm[kDiagSlots * kBlock / 32];
@@ -3128,13 +3482,12 @@ __global__ void __launch_bounds__(kBlock) k_flip_guess(EngineView v) {
   }
 }
 
-// FP64 transport (the plain FP64 path)
-template <int W, bool RESID>
-__global__ void __launch_bounds__(kBlock) k_transport64(EngineView v, double* F_out) {
+// FP64 bond sums of the residual entry point (F_k = sum_KRk1 + sum_KRk2 - R_k, utils.h:177): CTA per
+// tile, its halo staged in shared memory, W lanes a node
+template <int W>
+__global__ void __launch_bounds__(kBlock) k_residual64(EngineView v, double* F_out) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ TileSmem ts;
-  __shared__ double sm[kDiagSlots * kBlock / 32];
-  __shared__ int s_last;
   const int sub = threadIdx.x % W, seg = threadIdx.x / W, nseg = kBlock / W;
   for (int item = blockIdx.x; item < v.ntiles; item += gridDim.x) {
     const TileDesc t = v.tiles[item];
@@ -3160,14 +3513,9 @@ __global__ void __launch_bounds__(kBlock) k_transport64(EngineView v, double* F_
       cX[s] = s == 0 ? k.DSo[0] * BV : k.DSo[s];
       cSS[s] = s == 0 ? k.DSo[0] : 0.0;
     }
-    const long long step_no = k.ds->steps + 1;
-    const int hslot = k.hist_m >= 3 ? (k.ds->hist_head + 1) % k.hist_m : 0;
     const int* row = k.row;
     const double* w64 = k.w64;
     const int own0 = ts.off[4] + (t.own_begin - t.hb[4]);
-    double part[kDiagSlots];
-#pragma unroll
-    for (int q = 0; q < kDiagSlots; ++q) part[q] = 0.0;
     for (int a0 = t.own_begin; a0 < t.own_end; a0 += nseg) {
       const int a = a0 + seg;
       const bool act = a < t.own_end;
@@ -3213,51 +3561,159 @@ __global__ void __launch_bounds__(kBlock) k_transport64(EngineView v, double* F_
       const bool src_on = iface && !(dm & 1);
       const double swv = src_on ? dissolve_switch(ca[0], k.csat, k.sw) : 0.0;
       const double Rmg = src_on ? -k.k_diss * swv : 0.0;
-      if (RESID) {
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-          F_out[(size_t)s * k.N + a] = -k.K1[s] * a1[s] - k.K2zF[s] * a2[s] - (s == 0 ? Rmg : 0.0);
-        continue;
-      }
-      double val[S];
-      bool bad = false;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const double F = -k.K1[s] * a1[s] - k.K2zF[s] * a2[s] - (s == 0 ? Rmg : 0.0);
-        double x = ca[s] - k.dt * F;
-        if ((dm >> s) & 1) x = k.bcval[(size_t)s * k.N + a];
-        if (x < k.c_floor) x = k.c_floor;
-        if (!isfinite(x)) bad = true;
-        val[s] = x;
-      }
-      double pnew = pa;
-      if (pa != 0.0 && val[0] <= k.csat) {
-        pnew = 0.0;
-        k.flip_step[a] = (int)step_no;
-        k.flip_list[atomicAdd(&k.ds->nflip, 1)] = a;
-        k.ds->op_valid = 0;
-        k.ds->defl = 0;
-      }
-      record_history(k, a, hslot);
-      const double g = next_phi_guess(k, a);
-      Rec64 out;
-#pragma unroll
-      for (int s = 0; s < S; ++s) out.c[s] = val[s];
-      out.phi = g;
-      out.phase = pnew;
-      out.pad[0] = out.pad[1] = 0.0;
-      k.rec64_nxt[a] = out;
-#pragma unroll
-      for (int s = 0; s < S; ++s) part[s] += val[s];
-      if (pnew != 0.0) {
-        part[4] += 1.0;
-        part[5] += val[0] - k.csat;
-      }
-      part[6] += k.k_diss * swv;
-      part[7] += bad ? 1.0 : 0.0;
+      for (int s = 0; s < S; ++s)
+        F_out[(size_t)s * k.N + a] = -k.K1[s] * a1[s] - k.K2zF[s] * a2[s] - (s == 0 ? Rmg : 0.0);
     }
-    if (!RESID) transport_finish(v, t, k, item, part, sm, &s_last);
     __syncthreads();
+  }
+}
+
+// FP64 transport (the plain FP64 path), one lane a row of the transport's slices, K warps a slice.
+// A bond adds w (c_n - c_a) and w dphi c_n to the sums of its neighbour's phase (the bond
+// coefficients follow from the two phases, utils.h:100-153, and multiply the sums at the end): 14
+// FP64 instructions for the four species.  Bound by the FP64 pipe, which a warp-wide instruction
+// holds for 64 cycles.  512k nodes 2.14 ms, against 3.78 with the
+// coefficients multiplied into every bond (26 FP64 instructions).
+template <int K>
+__global__ void __launch_bounds__(kBlock, 1) k_transport64(EngineView v) {
+  constexpr int NV = 4 * S;  // liquid: w d, w dphi c; solid: the same
+  extern __shared__ __align__(16) unsigned char dsm[];
+  double* s_sum = reinterpret_cast<double*>(dsm);  // kBlock * NV (K > 1)
+  __shared__ int s_iface[kBlock];
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ double sm[kDiagSlots * kBlock / 32];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ns = v.nslices;
+  for (int base = blockIdx.x * SplitSlice<K>::kSlices; base < ns; base += gridDim.x * SplitSlice<K>::kSlices) {
+    const SplitSlice<K> ss(base);
+    const bool have = ss.sg < ns;
+    const SliceDesc& d = v.slices[have ? ss.sg : 0];
+    const int inst = __ldg(&d.inst);
+    const KParams& k = v.inst[inst];
+    if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+    __syncwarp();
+    const int* hb = s_hb[warp];
+    const int a = d.row0 + lane;
+    const bool rowok = have && lane < d.nrows;
+    double sum[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sum[q] = 0.0;
+    double ca[S], pha = 0.0;
+    int solid = 0, liquids = 0;
+    if (rowok) {
+      const Rec64* rc = k.rec64_cur;
+      double pp[2];
+      ld_rec64(rc + a, ca, pp);
+      pha = pp[0];
+      solid = __double2hiint(pp[1]) != 0;
+      const int len = k.row[a + 1] - k.row[a];
+      const QuadPtr op(sell_w(k, d), lane);
+      const double* w64 = k.sell64 + (size_t)(d.off >> 5) * 32 + 4 * lane;
+      for (int q = ss.part; 4 * q < len; q += K) {
+        double w[4];
+        const uint2 code = op.codes(q);
+        ld_stream_d4(w64 + 128 * (size_t)q, w);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          double cn[2][S], pn[2][2];
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            if (4 * q + 2 * h + t < len) ld_rec64(rc + code_node(hb, quad_code(code, 2 * h + t)), cn[t], pn[t]);
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (4 * q + 2 * h + t >= len) continue;
+            const double wt = w[2 * h + t];
+            const double wd = wt * (pn[t][0] - pha);
+            if (__double2hiint(pn[t][1]) == 0) {
+              ++liquids;
+#pragma unroll
+              for (int s = 0; s < S; ++s) {
+                sum[s] = fma(wt, cn[t][s] - ca[s], sum[s]);
+                sum[S + s] = fma(wd, cn[t][s], sum[S + s]);
+              }
+            } else {
+#pragma unroll
+              for (int s = 0; s < S; ++s) {
+                sum[2 * S + s] = fma(wt, cn[t][s] - ca[s], sum[2 * S + s]);
+                sum[3 * S + s] = fma(wd, cn[t][s], sum[3 * S + s]);
+              }
+            }
+          }
+        }
+      }
+    }
+    if (K > 1) {
+      s_iface[threadIdx.x] = liquids;
+      split_sum<K, NV>(sum, s_sum);
+    }
+    if (have && ss.part == 0) {
+      if (K > 1)
+        for (int h = 1; h < K; ++h) liquids += s_iface[threadIdx.x + 32 * h];
+      double part[kDiagSlots];
+#pragma unroll
+      for (int q = 0; q < kDiagSlots; ++q) part[q] = 0.0;
+      if (rowok) {
+        const unsigned char dm = k.dirmask[a];
+        const bool src_on = solid && liquids > 0 && !(dm & 1);
+        const double swv = src_on ? dissolve_switch(ca[0], k.csat, k.sw) : 0.0;
+        const double Rmg = src_on ? -k.k_diss * swv : 0.0;
+        double val[S];
+        bool bad = false;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const double cX = s == 0 ? k.DSo[0] * *k.bv_ptr : k.DSo[s];
+          const double cL = solid ? cX : k.DL[s], cS = solid ? (s == 0 ? k.DSo[0] : 0.0) : cX;
+          const double a1 = cL * sum[s] + cS * sum[2 * S + s], a2 = cL * sum[S + s] + cS * sum[3 * S + s];
+          const double F = -k.K1[s] * a1 - k.K2zF[s] * a2 - (s == 0 ? Rmg : 0.0);
+          double x = ca[s] - k.dt * F;
+          if ((dm >> s) & 1) x = k.bcval[(size_t)s * k.N + a];
+          if (x < k.c_floor) x = k.c_floor;
+          if (!isfinite(x)) bad = true;
+          val[s] = x;
+        }
+        double pnew = solid ? 1.0 : 0.0;
+        if (solid && val[0] <= k.csat) {
+          pnew = 0.0;
+          k.flip_step[a] = (int)(k.ds->steps + 1);
+          k.flip_list[atomicAdd(&k.ds->nflip, 1)] = a;
+          k.ds->op_valid = 0;
+          k.ds->defl = 0;
+        }
+        record_history(k, a, k.hist_m >= 3 ? (k.ds->hist_head + 1) % k.hist_m : 0);
+        const double g = next_phi_guess(k, a);
+        Rec64 out;
+#pragma unroll
+        for (int s = 0; s < S; ++s) out.c[s] = val[s];
+        out.phi = g;
+        out.phase = pnew;
+        out.pad[0] = out.pad[1] = 0.0;
+        k.rec64_nxt[a] = out;
+#pragma unroll
+        for (int s = 0; s < S; ++s) part[s] = val[s];
+        if (pnew != 0.0) {
+          part[4] = 1.0;
+          part[5] = val[0] - k.csat;
+        }
+        part[6] = k.k_diss * swv;
+        part[7] = bad ? 1.0 : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) part[q] = warp_sum_d(part[q]);
+      slice_partials64<kDiagSlots>(v, inst, __ldg(&v.slice_first[inst]), __ldg(&v.slice_count[inst]), ss.sg, part);
+    }
+    if (K > 1) __syncthreads();
+    else __syncwarp();
+  }
+  if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
+    for (int i = 0; i < v.M; ++i) {
+      double tot[kDiagSlots];
+      reduce_slices64<kDiagSlots>(v, i, v.slice_first[i], v.slice_count[i], tot, sm);
+      if (threadIdx.x == 0) finish_instance(v.inst[i], tot);
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) v.ticket[v.M + 1] = 0;
   }
 }
 
@@ -3463,7 +3919,7 @@ int claim_grid(K kern, size_t smem, int sms, int nslices) {
 
 size_t smem_slots(int B) { return (size_t)(B + 16) * sizeof(unsigned short); }
 size_t smem_prep(int H, int B) { return align16((size_t)H * (sizeof(double) + 1)) + smem_slots(B); }
-size_t smem_vec64(int H, int B) { return align16((size_t)H * sizeof(double)) + smem_slots(B); }
+size_t smem_transport64() { return (size_t)kBlock * 4 * S * sizeof(double); }
 size_t smem_spmv_staged() { return kTmaRingBytes + kTmaWinBytes + kTmaBarBytes; }
 // streamed operator: the deepest ring (2..4 stages) that fits beside windows of win_cap nodes
 constexpr size_t kSmemCta = 225 * 1024;
@@ -3684,7 +4140,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_transport32(EngineView v, con
       float cfL[S], cfS[S];  // pair coefficient for a liquid / solid neighbour (BV = 1)
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        const float dl = (float)k.DL[q], ds = (float)k.DSo[q];
+        const float dl = k.DLf[q], ds = k.DSof[q];
         cfL[q] = pm ? ds : dl;
         cfS[q] = pm ? (q == 0 ? ds : 0.0f) : ds;
       }
@@ -3692,20 +4148,21 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_transport32(EngineView v, con
 #pragma unroll
       for (int q = 0; q < S; ++q) A1[q] = A2[q] = a1[q] = a2[q] = sl[q] = sc[q] = 0.0f;
       int iface = 0;
-      const float* ws = sell_w(k, d) + lane;
-      const unsigned short* cs = sell_code(k, d) + lane;
+      const QuadPtr op(sell_w(k, d), lane);
       const int len = k.row[a + 1] - k.row[a];
       // bonds in batches of kAdjB columns (codes, weights and records in flight together;
       // the column order of the sums is kept)
       for (int c0 = 0; c0 < len; c0 += kAdjB) {
+        static_assert(kAdjB == 4, "the adjoint's batch is a quad");
+        const float4 wq = op.weights(c0 >> 2);
+        const uint2 cq = op.codes(c0 >> 2);
         float wv[kAdjB];
         unsigned int code[kAdjB];
 #pragma unroll
-        for (int u = 0; u < kAdjB; ++u)
-          if (c0 + u < len) {
-            wv[u] = ld_stream(ws + kSellW * (c0 + u));
-            code[u] = ld_stream(cs + kSellC * (c0 + u));
-          }
+        for (int u = 0; u < kAdjB; ++u) {
+          wv[u] = quad_weight(wq, u);
+          code[u] = quad_code(cq, u);
+        }
         float4 cnv[kAdjB], lnv[kAdjB], pnv[kAdjB];
 #pragma unroll
         for (int u = 0; u < kAdjB; ++u)
@@ -3739,11 +4196,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_transport32(EngineView v, con
       }
       const unsigned char dm = k.dirmask[a];
       const bool src = iface && !(dm & 1);
-      const float dt = (float)k.dt;
+      const float dt = k.dtf;
       float nu_a = 0.0f;
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        const float K1 = (float)k.K1[q], K2 = (float)k.K2zF[q];
+        const float K1 = k.K1f[q], K2 = k.K2zFf[q];
         const float lmq = sel4(lm4, q), cmq = sel4(cm4, q);
         float m = lmq + dt * (K1 * A1[q] + K2 * A2[q]);
         if (q == 0 && src) {
@@ -3757,7 +4214,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_adj_transport32(EngineView v, con
         }
         mu[(size_t)q * k.N + a] = (double)m;
         nu_a = fmaf(dt * K2, cmq * sl[q] - lmq * sc[q], nu_a);
-        const float gq = lmq * dt * (K1 * a1[q] + K2 * a2[q]) / (float)k.DL[q];
+        const float gq = lmq * dt * (K1 * a1[q] + K2 * a2[q]) / k.DLf[q];
         float e;
         two_sum(gh[q], gq, gh[q], e);
         gl[q] += e;
@@ -3956,19 +4413,17 @@ nnpp_status prepare_kernels(int H, int B, int lanes) {
   NNPP_TRY(allow_smem(k_transport32h<8, true, 4>, kTrHaloSmemMax));
   return dispatch_lanes(lanes, [&](auto wc) -> nnpp_status {
     constexpr int W = decltype(wc)::value;
-    NNPP_TRY(allow_smem(k_prep<float, W>, smem_prep(H, B)));
-    NNPP_TRY(allow_smem(k_prep<double, W>, smem_prep(H, B)));
-    NNPP_TRY(allow_smem(k_cg_spmv64<W>, smem_vec64(H, B)));
+    NNPP_TRY(allow_smem(k_f11<float, W>, smem_prep(H, B)));
+    NNPP_TRY(allow_smem(k_f11<double, W>, smem_prep(H, B)));
     NNPP_TRY(allow_smem(k_cg_spmv32t<W>, smem_spmv_staged()));
     NNPP_TRY(allow_smem(k_cg_spmv32s<W, kStreamCol>, kSmemCta));
     NNPP_TRY(allow_smem(k_cg_spmv32<W, true, 8, true, 3>, smem_spmv_win()));
     NNPP_TRY(allow_smem(k_cg_spmv32<W, true, 16, false, 3>, smem_spmv_win()));
     NNPP_TRY(allow_smem(k_cg_spmv32<W, true, 16, false, 3, 3>, smem_spmv_win()));
     NNPP_TRY(allow_smem(k_cg_spmv32<W, true, 8, true, 3, 4>, smem_spmv_win()));
-    NNPP_TRY(allow_smem(k_ir_update<float, W>, smem_vec64(H, B)));
-    NNPP_TRY(allow_smem(k_ir_update<double, W>, smem_vec64(H, B)));
-    NNPP_TRY(allow_smem(k_transport64<W, false>, smem_tr64(H, B)));
-    NNPP_TRY(allow_smem(k_transport64<W, true>, smem_tr64(H, B)));
+    NNPP_TRY(allow_smem(k_residual64<W>, smem_tr64(H, B)));
+    NNPP_TRY(allow_smem(k_transport64<2>, smem_transport64()));
+    NNPP_TRY(allow_smem(k_transport64<4>, smem_transport64()));
     return NNPP_OK;
   });
 }
@@ -3987,9 +4442,7 @@ void launch_spmv_gather(int variant, const EngineView& v, int sms, cudaStream_t 
       break;
     }
     case 3:
-      // 40 registers: six CTAs an SM (measured 0.087 ms at 512k; five CTAs 0.088, eight with
-      // 32 registers 0.120, batches of 32 columns at four 0.089)
-      k_cg_spmv32<W, false, 16, false, 6><<<claim_grid(k_cg_spmv32<W, false, 16, false, 6>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
+      k_cg_spmv32<W, false, 8, true, 5><<<claim_grid(k_cg_spmv32<W, false, 8, true, 5>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
       break;
     case 4: {
       const size_t sh = smem_spmv_win();
@@ -4002,7 +4455,7 @@ void launch_spmv_gather(int variant, const EngineView& v, int sms, cudaStream_t 
       break;
     }
     case 6:
-      k_cg_spmv32<W, false, 16, false, 5, 3><<<slice_grid(k_cg_spmv32<W, false, 16, false, 5, 3>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
+      k_cg_spmv32<W, false, 16, false, 4, 3><<<slice_grid(k_cg_spmv32<W, false, 16, false, 4, 3>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
       break;
     case 7: {
       const size_t sh = smem_spmv_win();
@@ -4010,9 +4463,9 @@ void launch_spmv_gather(int variant, const EngineView& v, int sms, cudaStream_t 
       break;
     }
     default:
-      // measured 0.071 ms at 512k against 0.076 for 3; batches of 8 at 64 warps an SM took
-      // 0.105, pipelined 16 at 3 CTAs 0.072, pipelined 24 at 3 CTAs (spilling) slower
-      k_cg_spmv32<W, false, 16, true, 4><<<claim_grid(k_cg_spmv32<W, false, 16, true, 4>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
+      // measured at 512k (ms): 0.0575; pipelined batches of 8 at five CTAs 0.0588 (variant 3), of 12
+      // at four 0.0592, of 16 at four (64 registers, spilling) 0.0687; unpipelined 16 at five 0.0615
+      k_cg_spmv32<W, false, 16, true, 3><<<claim_grid(k_cg_spmv32<W, false, 16, true, 3>, 0, sms, v.ncslices), kBlock, 0, st>>>(v);
   }
 }
 
@@ -4035,6 +4488,35 @@ bool spmv_halo_fits(const Engine& e) {
   return e.halo_op && e.T <= 8 && smem_spmv_halo(e.halo_max, e.hcode_max16, e.hquad_max) <= 200 * 1024;
 }
 
+// Warps that share a slice: the most of 1, 2, 4, 8 with which the slices' warps still fit about half
+// of the SMs' 48-64 resident ones.  Measured, split against one warp a slice, us: 8k nodes FP32
+// operator 9.0 against 12.3, its refinement 12.8 against 22.9, FP64 operator 12.4 against 19.6,
+// refinement 16.4 against 22.0, transport 96 against 239; 64k nodes FP32 operator 16.5 against 18.3,
+// refinement 25 against 37; from 262k nodes on one warp a slice fills the SMs.
+constexpr int kSplitWarpsPerSm = 32;
+int split_warps(int sms, int slices, int most) {
+  int k = 1;
+  while (k < most && (long long)slices * 2 * k <= (long long)sms * kSplitWarpsPerSm) k *= 2;
+  return k;
+}
+// calls f with the split as a constant
+template <typename F>
+void dispatch_split(int k, F&& f) {
+  if (k >= 8)
+    f(std::integral_constant<int, 8>());
+  else if (k == 4)
+    f(std::integral_constant<int, 4>());
+  else if (k == 2)
+    f(std::integral_constant<int, 2>());
+  else
+    f(std::integral_constant<int, 1>());
+}
+// CTAs of a split slice kernel: every one that fits at once, at most one per group of slices
+template <int K, typename Kern>
+int split_grid(Kern kern, size_t smem, int sms, int slices) {
+  return occ_grid(kern, smem, sms, (slices + SplitSlice<K>::kSlices - 1) / SplitSlice<K>::kSlices);
+}
+
 nnpp_status launch_warm_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {
   if (prec == NNPP_MIXED) {
     k_warm_dots<float><<<occ_grid(k_warm_dots<float>, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v);
@@ -4050,8 +4532,17 @@ nnpp_status launch_warm_b(const Engine& e, const EngineView& v, int prec, cudaSt
 nnpp_status launch_prep_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st,
                           cudaGraphConditionalHandle hc, double* F11_out) {
   if (prec == NNPP_MIXED && !F11_out) {
-    k_phi4<<<occ_grid(k_phi4, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v);
+    k_phi4<float><<<occ_grid(k_phi4<float>, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v);
     k_prep_slices<<<claim_grid(k_prep_slices, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, hc);
+    NNPP_CUDA(cudaGetLastError());
+    return NNPP_OK;
+  }
+  if (!F11_out) {
+    k_phi4<double><<<occ_grid(k_phi4<double>, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v);
+    dispatch_split(split_warps(e.sms, v.nslices, 8), [&](auto kc) {
+      constexpr int K = decltype(kc)::value;
+      k_prep64<K><<<split_grid<K>(k_prep64<K>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, hc);
+    });
     NNPP_CUDA(cudaGetLastError());
     return NNPP_OK;
   }
@@ -4059,9 +4550,9 @@ nnpp_status launch_prep_b(const Engine& e, const EngineView& v, int prec, cudaSt
     constexpr int W = decltype(wc)::value;
     const size_t sh = smem_prep(v.halo_max, v.bond_max);
     if (prec == NNPP_MIXED)
-      k_prep<float, W><<<occ_grid(k_prep<float, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, hc, F11_out);
+      k_f11<float, W><<<occ_grid(k_f11<float, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, F11_out);
     else
-      k_prep<double, W><<<occ_grid(k_prep<double, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, hc, F11_out);
+      k_f11<double, W><<<occ_grid(k_f11<double, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, F11_out);
     NNPP_CUDA(cudaGetLastError());
     return NNPP_OK;
   });
@@ -4129,11 +4620,19 @@ nnpp_status launch_cg_spmv_b(const Engine& e, const EngineView& v, int prec, cud
       } else if (e.spmv_variant == 1) {
         const size_t sh = smem_spmv_staged();
         k_cg_spmv32t<W><<<occ_grid(k_cg_spmv32t<W>, sh, e.sms, (v.nslices + 7) / 8), kBlock, sh, st>>>(v);
+      } else if (const int split = split_warps(e.sms, v.ncslices, 8); split > 1 && e.spmv_variant == 0) {
+        dispatch_split(split, [&](auto kc) {
+          constexpr int K = decltype(kc)::value;
+          k_cg_spmv32k<K><<<split_grid<K>(k_cg_spmv32k<K>, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v);
+        });
       } else {
         launch_spmv_gather<W>(e.spmv_variant, v, e.sms, st);
       }
     else
-      { const size_t sh = smem_vec64(v.halo_max, v.bond_max); k_cg_spmv64<W><<<occ_grid(k_cg_spmv64<W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v); }
+      dispatch_split(split_warps(e.sms, v.ncslices, 8), [&](auto kc) {
+        constexpr int K = decltype(kc)::value;
+        k_cg_spmv64<K><<<split_grid<K>(k_cg_spmv64<K>, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v);
+      });
     NNPP_CUDA(cudaGetLastError());
     return NNPP_OK;
   });
@@ -4209,21 +4708,23 @@ nnpp_status launch_cg_update_b(const Engine& e, const EngineView& v, int prec, c
 
 nnpp_status launch_ir_update_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st,
                                cudaGraphConditionalHandle hc) {
+  const int split = split_warps(e.sms, v.ncslices, 8);
   if (prec == NNPP_MIXED) {
-    k_ir_slices<<<claim_grid(k_ir_slices, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v, hc);
-    NNPP_CUDA(cudaGetLastError());
-    return NNPP_OK;
-  }
-  return dispatch_lanes(e.W, [&](auto wc) -> nnpp_status {
-    constexpr int W = decltype(wc)::value;
-    const size_t sh = smem_vec64(v.halo_max, v.bond_max);
-    if (prec == NNPP_MIXED)
-      k_ir_update<float, W><<<occ_grid(k_ir_update<float, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, hc);
+    if (split > 1)
+      dispatch_split(split, [&](auto kc) {
+        constexpr int K = decltype(kc)::value;
+        k_ir_split<K><<<split_grid<K>(k_ir_split<K>, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v, hc);
+      });
     else
-      k_ir_update<double, W><<<occ_grid(k_ir_update<double, W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, hc);
-    NNPP_CUDA(cudaGetLastError());
-    return NNPP_OK;
-  });
+      k_ir_slices<<<claim_grid(k_ir_slices, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v, hc);
+  } else {
+    dispatch_split(split, [&](auto kc) {
+      constexpr int K = decltype(kc)::value;
+      k_ir64<K><<<split_grid<K>(k_ir64<K>, 0, e.sms, v.ncslices), kBlock, 0, st>>>(v, hc);
+    });
+  }
+  NNPP_CUDA(cudaGetLastError());
+  return NNPP_OK;
 }
 
 // The halo-staged FP32 transport (form 1): batches of 8 bond columns, the next batch's codes
@@ -4245,21 +4746,25 @@ nnpp_status launch_transport_b(const Engine& e, const EngineView& v, int prec, c
     constexpr int W = decltype(wc)::value;
     if (prec == NNPP_MIXED) {
       if (F_out)
-        k_transport32<W, true><<<slice_grid(k_transport32<W, true>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, F_out);
+        k_transport32<true><<<slice_grid(k_transport32<true>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, F_out);
       else {
         if (e.tr_variant > 0 && transport_halo_fits(e)) {
           launch_transport_staged(v, e.sms, st);
         } else {
-          k_transport32<W, false><<<claim_grid(k_transport32<W, false>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, nullptr);
+          k_transport32<false><<<claim_grid(k_transport32<false>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, nullptr);
         }
         k_flip_guess<float><<<kFlipGuessCtas, kBlock, 0, st>>>(v);
       }
     } else {
       const size_t sh = smem_tr64(v.halo_max, v.bond_max);
       if (F_out)
-        k_transport64<W, true><<<occ_grid(k_transport64<W, true>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, F_out);
+        k_residual64<W><<<occ_grid(k_residual64<W>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, F_out);
       else {
-        k_transport64<W, false><<<occ_grid(k_transport64<W, false>, sh, e.sms, v.ntiles), kBlock, sh, st>>>(v, nullptr);
+        dispatch_split(split_warps(e.sms, v.nslices, 4), [&](auto kc) {
+          constexpr int K = decltype(kc)::value < 4 ? decltype(kc)::value : 4;
+          const size_t sh = K > 1 ? smem_transport64() : 0;
+          k_transport64<K><<<split_grid<K>(k_transport64<K>, sh, e.sms, v.nslices), kBlock, sh, st>>>(v);
+        });
         k_flip_guess<double><<<kFlipGuessCtas, kBlock, 0, st>>>(v);
       }
     }
@@ -4315,6 +4820,8 @@ KParams make_kparams(Handle& h, int cur) {
   k.sell_lo = h.sell_lo.get();
   k.sell_cg = h.sell_cg.get();
   k.sell_cg_lo = h.sell_cg_lo.get();
+  k.sell64 = h.sell64.get();
+  k.sell_cg64 = h.sell_cg64.get();
   k.cg_width = h.cg_width.get();
   k.cg_rows = h.cg_rows.get();
   k.cg_pos = h.cg_pos.get();
@@ -4386,7 +4893,12 @@ KParams make_kparams(Handle& h, int cur) {
     k.DL[s] = p.D_liquid[s];
     k.DSo[s] = p.D_solid[s];
     k.z[s] = p.z[s];
+    k.K1f[s] = (float)k.K1[s];
+    k.K2zFf[s] = (float)k.K2zF[s];
+    k.DLf[s] = (float)k.DL[s];
+    k.DSof[s] = (float)k.DSo[s];
   }
+  k.dtf = (float)k.dt;
   k.sub_step_no = p.sub_step_no;
   k.dissolve_count = 1;
   k.extrapolate = h.extrapolate;

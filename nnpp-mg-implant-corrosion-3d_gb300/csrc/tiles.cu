@@ -1,6 +1,6 @@
 // tiles.cu -- tile work items of one instance, 16-bit halo slots of every bond, FP32
-// position records and the sliced operator (32 rows per slice, column-major, each bond
-// column 32 FP32 weights + 32 16-bit codes) that the FP32 kernels stream.
+// position records and the sliced operator (32 rows per slice, quads of bond columns, each
+// 32 lanes' four FP32 weights + 32 lanes' four 16-bit codes) that the FP32 kernels stream.
 //
 // A tile is T consecutive bins along x (bins of side >= the horizon radius, x-fastest
 // order, so the tile's own nodes and each of its 3x3 halo rows are contiguous node
@@ -143,9 +143,10 @@ __global__ void k_slice_windows(int nslices, const SliceDesc* sl, const int* pre
   }
 }
 
-// warp per slice: bond c of lane l (row row0 + l): its FP32 weight at float 48 (off/32 + c)
-// + l of the interleaved array, its code (window row << 12 | node - gbase[row]) at 16-bit
-// element 96 (off/32 + c) + 64 + l; padding: code 0, weight 0
+// warp per slice: the interleaved quads of bond columns (see quad_w in step.cu: per quad 32 lanes'
+// four FP32 weights, then their four 16-bit codes, window row << 12 | node - gbase[row]) and the
+// weights' low words in the same order; padding: code 0, weight 0.  One 16-byte and one 8-byte
+// store a lane and quad.
 __global__ void k_sell_fill(int nslices, const SliceDesc* sl, const int* pre_hb, const int* row,
                             const unsigned short* slot, const float* w32, const float* wlo32, float* sell,
                             float* sell_lo) {
@@ -158,20 +159,41 @@ __global__ void k_sell_fill(int nslices, const SliceDesc* sl, const int* pre_hb,
     const bool live = lane < d.nrows;
     const int j0 = live ? row[d.row0 + lane] : 0;
     const int len = live ? row[d.row0 + lane + 1] - j0 : 0;
-    for (int c = 0; c < d.width; ++c) {
-      float* col = sell + ((size_t)(d.off >> 5) + c) * 48;
-      unsigned short code = 0;
-      float w = 0.0f, wl = 0.0f;
-      if (c < len) {
+    for (int q = 0; q < d.width / 4; ++q) {
+      float* quad = sell + (size_t)(d.off >> 5) * 48 + (size_t)192 * q;
+      unsigned int code[4] = {0u, 0u, 0u, 0u};
+      float w[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wl[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = 4 * q + u;
+        if (c >= len) continue;
         int r, node;
         slot_node(slot[j0 + c], pre, hb, &r, &node);
-        code = (unsigned short)((r << 12) | (node - d.gbase[r]));
-        w = w32[j0 + c];
-        wl = wlo32[j0 + c];
+        code[u] = (unsigned int)((r << 12) | (node - d.gbase[r]));
+        w[u] = w32[j0 + c];
+        wl[u] = wlo32[j0 + c];
       }
-      col[lane] = w;
-      reinterpret_cast<unsigned short*>(col + 32)[lane] = code;
-      sell_lo[((size_t)(d.off >> 5) + c) * 32 + lane] = wl;
+      reinterpret_cast<float4*>(quad)[lane] = make_float4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint2*>(quad + 128)[lane] = make_uint2(code[0] | code[1] << 16, code[2] | code[3] << 16);
+      reinterpret_cast<float4*>(sell_lo + (size_t)(d.off >> 5) * 32 + (size_t)128 * q)[lane] =
+          make_float4(wl[0], wl[1], wl[2], wl[3]);
+    }
+  }
+}
+
+// warp per slice: the FP64 weights in sell_lo's order (per quad 32 lanes' four values)
+__global__ void k_sell64_fill(int nslices, const SliceDesc* sl, const int* row, const double* w64, double* sell64) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslices; s += warps) {
+    const SliceDesc& d = sl[s];
+    const bool live = lane < d.nrows;
+    const int j0 = live ? row[d.row0 + lane] : 0;
+    const int len = live ? row[d.row0 + lane + 1] - j0 : 0;
+    for (int q = 0; q < d.width / 4; ++q) {
+      double* o = sell64 + (size_t)(d.off >> 5) * 32 + (size_t)128 * q + 4 * lane;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) o[u] = 4 * q + u < len ? w64[j0 + 4 * q + u] : 0.0;
     }
   }
 }
@@ -333,6 +355,7 @@ nnpp_status build_tiles(Handle& h, int T, std::vector<TileDesc>& tiles, std::vec
           for (int q = 0; q < 4; ++q) d.pad2[q] = 0;
           for (int r = 0; r < 9; ++r) d.lo[r] = d.woff[r] = d.wlen[r] = d.gbase[r] = 0;
           for (int l = 0; l < d.nrows; ++l) d.width = std::max(d.width, rows[r0 + l + 1] - rows[r0 + l]);
+          d.width = (d.width + 3) & ~3;  // whole quads of columns
           slices.push_back(d);
           int acc = 0;
           for (int r = 0; r < 9; ++r) {
@@ -349,6 +372,7 @@ nnpp_status build_tiles(Handle& h, int T, std::vector<TileDesc>& tiles, std::vec
         bm = std::max(bm, t.bond1 - t.bond0);
         tiles.push_back(t);
       }
+  h.sell64_ok = false;
   // sliced copy of the slot codes and FP32 weights for the CG operator and the transport
   const size_t ns = slices.size();
   if (!h.sell.alloc((size_t)(soff / 32) * 48 + 48) || !h.sell_lo.alloc((size_t)(soff / 32) * 32 + 32))
@@ -477,6 +501,7 @@ nnpp_status build_cg_slices(Handle& h, std::vector<SliceDesc>& gcs, int inst, bo
             d.width = std::max(d.width, rows[a + 1] - rows[a]);
           }
         }
+        d.width = (d.width + 3) & ~3;  // whole quads of columns
         coff += 32LL * d.width;
         if (coff > 0x7fffffffLL) return set_error(NNPP_ERR_UNSUPPORTED, "CG operator above 2^31 entries");
         cs.push_back(d);
@@ -515,6 +540,21 @@ nnpp_status build_cg_slices(Handle& h, std::vector<SliceDesc>& gcs, int inst, bo
   }
   *windows_fit = fit;
   gcs.insert(gcs.end(), cs.begin(), cs.end());
+  return NNPP_OK;
+}
+
+nnpp_status build_sell64(Handle& h, const SliceDesc* slices, int count) {
+  if (h.sell64_ok) return NNPP_OK;
+  if (!h.sell64.alloc(h.sell_lo.size()) || !h.sell_cg64.alloc(h.sell_cg_lo.size()))
+    return set_error(NNPP_ERR_NOMEM, "FP64 sliced operator");
+  NNPP_CUDA(cudaMemsetAsync(h.sell_cg64.get(), 0, h.sell_cg64.bytes(), h.st));
+  if (count > 0)
+    k_sell64_fill<<<std::max(1, std::min((count * 32 + 255) / 256, 152 * 32)), 256, 0, h.st>>>(
+        count, slices, h.lay.row.get(), h.lay.w64.get(), h.sell64.get());
+  NNPP_CUDA(cudaGetLastError());
+  NNPP_CUDA(cudaMemsetAsync(&h.dstate.get()->op_valid, 0, sizeof(int), h.st));
+  NNPP_CUDA(cudaStreamSynchronize(h.st));  // the engine's stream may be another one
+  h.sell64_ok = true;
   return NNPP_OK;
 }
 

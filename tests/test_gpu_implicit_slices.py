@@ -1,7 +1,6 @@
 """The implicit step's sliced operator and device-side GMRES where they can go wrong: node counts off
-the slices of 32 rows, a size above the line below which four warps share a slice, and a time step
-long enough that the systems pass a GMRES restart -- against the oracle's step: the same Newton
-iterations, the states to 1e-9 (the bound of the other implicit tests: the GMRES tolerance's rounding),
+the slices of 32 rows, a size above the line below which four warps share a slice, whose potential
+system passes a GMRES restart -- against the oracle's step: the same Newton iterations, the states to 1e-9 (the bound of the other implicit tests: the GMRES tolerance's rounding),
 identical masks."""
 import numpy as np
 import pytest
