@@ -71,6 +71,9 @@ nnpp_status build_lists(Engine& e, int T) {
   std::vector<HTile> htiles;
   std::vector<SliceDesc> cslices;
   std::vector<int> meta(8 * M);
+  long long nodes = 0;
+  for (Handle* h : e.members) nodes += h->N;
+  const int chunk = nodes <= kSmallNodes ? kSmallChunk : kChunk;
   bool fit = true, hop = true;
   int hm = 0, bmax = 0, cmax = 0, qmax = 0;
   for (int i = 0; i < M; ++i) {
@@ -98,11 +101,11 @@ nnpp_status build_lists(Engine& e, int T) {
     hm = std::max(hm, hmi);
     bmax = std::max(bmax, bmi);
     meta[2 * M + i] = (int)chunks.size();
-    for (int b = 0; b < h.N; b += kChunk) {
+    for (int b = 0; b < h.N; b += chunk) {
       Chunk c;
       c.inst = i;
       c.begin = b;
-      c.end = std::min(h.N, b + kChunk);
+      c.end = std::min(h.N, b + chunk);
       c.pad = 0;
       chunks.push_back(c);
     }

@@ -103,7 +103,11 @@ struct EngineView {
   int hcode_max16;          // largest code block of a tile (16-byte units, variant 8)
 };
 
-constexpr int kChunk = 1024;  // nodes per elementwise work item
+// nodes per elementwise work item: four a thread, or one while four would leave some of the 152 SMs
+// without a block (8,000 nodes are eight blocks of 1024).  A mixed step, 256 against 1024 (ms): 8k nodes
+// 0.358 against 0.441, 64k 0.628 against 0.776, 262k 1.626 against 1.588
+constexpr int kChunk = 1024, kSmallChunk = 256;
+constexpr long long kSmallNodes = 152 * 1024;
 constexpr int kSpmvVariants = 9;  // FP32 CG operator variants the autotuner times
 constexpr int kSpmvHalo = 8;      // the halo-staged variant with recomputed weights
 constexpr int kTrVariants = 2;    // FP32 transport forms (0 L1/L2 gathers, 1 halo staged)
