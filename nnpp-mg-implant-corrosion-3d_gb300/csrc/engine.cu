@@ -51,7 +51,8 @@ nnpp_status sync_members(Engine& e) {
 
 // slots a value of the partials takes: the items, or the groups of slices (slice_group0)
 int partial_stride(const Engine& e) {
-  return std::max(std::max(e.ntiles, e.nchunks), std::max(e.nslices, e.ncslices)) + (int)e.members.size() + 1;
+  return std::max(std::max(std::max(e.ntiles, e.nchunks), std::max(e.nslices, e.ncslices)), e.sms) +
+         (int)e.members.size() + 1;
 }
 
 // the members' FP64 weights for the current lists (FP64 runs)
@@ -131,7 +132,7 @@ nnpp_status build_lists(Engine& e, int T) {
   if (!e.d_tiles.alloc(tiles.size()) || !e.d_chunks.alloc(chunks.size()) || !e.d_meta.alloc(meta.size()) ||
       !e.d_slices.alloc(std::max<size_t>(slices.size(), 1)) || !e.d_htiles.alloc(std::max<size_t>(htiles.size(), 1)) ||
       !e.d_cslices.alloc(std::max<size_t>(cslices.size(), 1)) ||
-      !e.d_ticket.alloc(M + 4) || !e.d_gcount.alloc((size_t)stride) ||
+      !e.d_ticket.alloc(M + 6) || !e.d_gcount.alloc((size_t)stride) ||
       !e.d_partials.alloc((size_t)kReduceSlots * stride) ||
       !e.d_inst[0].alloc(M) || !e.d_inst[1].alloc(M))
     return set_error(NNPP_ERR_NOMEM, "engine work lists");
@@ -217,7 +218,10 @@ nnpp_status tune(Engine& e, int prec) {
     // the warm-up launch forms the mask sums, the timed ones are a step's
     NNPP_TRY(timed(4, &t_prep, [&] { return launch_prep_b(e, v, prec, e.st, 0, nullptr); }));
     const bool win = prec == NNPP_MIXED && spmv_staged_fits(e);
-    const int nvar = prec == NNPP_MIXED ? kSpmvVariants : 1;
+    // a single instance with the two-level preconditioner runs its inner solve in one launch, which
+    // has variant 0's operator
+    const bool sweep = e.members.size() == 1 && e.members[0]->coarse_enabled && e.members[0]->coarse.n > 0;
+    const int nvar = prec == NNPP_MIXED && !sweep ? kSpmvVariants : 1;
     for (int var = 0; var < nvar; ++var) {
       if (!win && spmv_needs_windows(var)) continue;
       if (var == kSpmvHalo && !spmv_halo_fits(e)) continue;
@@ -277,6 +281,13 @@ nnpp_status capture_solve(Engine& e, const EngineView& v, int prec) {
   cudaGraph_t body_out;
   NNPP_TRY(add_while(e.st, hout, &body_out));
   NNPP_CUDA(cudaStreamBeginCaptureToGraph(e.st_b1, body_out, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+  if (cg_sweep_applies(e, prec)) {
+    NNPP_TRY(launch_cg_sweep_b(e, v, prec, e.st_b1));
+    NNPP_TRY(launch_ir_update_b(e, v, prec, e.st_b1, hout));
+    cudaGraph_t done;
+    NNPP_CUDA(cudaStreamEndCapture(e.st_b1, &done));
+    return NNPP_OK;
+  }
   cudaGraphConditionalHandle hin;
   NNPP_CUDA(cudaGraphConditionalHandleCreate(&hin, body_out, 0, 0));
   NNPP_TRY(launch_cg_init_b(e, v, prec, e.st_b1, hin));
@@ -314,6 +325,11 @@ nnpp_status eager_solve(Engine& e, const EngineView& v, int prec) {
   for (int outer = 0; outer < (1 << 20); ++outer) {
     NNPP_TRY(any_active(e, 0, &go));
     if (!go) break;
+    if (cg_sweep_applies(e, prec)) {
+      NNPP_TRY(launch_cg_sweep_b(e, v, prec, e.st));
+      NNPP_TRY(launch_ir_update_b(e, v, prec, e.st, 0));
+      continue;
+    }
     NNPP_TRY(launch_cg_init_b(e, v, prec, e.st, 0));
     for (int inner = 0; inner < (1 << 24); ++inner) {
       NNPP_TRY(any_active(e, 1, &go));

@@ -91,7 +91,8 @@ struct EngineView {
   const int* cslice_first;
   const int* cslice_count;
   unsigned int* ticket;     // per instance completion counters, + [M] global, + [M+1] grid,
-                            // + [M+2] slice claims, + [M+3] the next-guess pass
+                            // + [M+2] slice claims, + [M+3] the next-guess pass, + [M+4], [M+5]
+                            // k_cg_sweep's meetings and exits
   unsigned int* gcount;     // FP64 slice groups: slices done (zero between kernels)
   double* partials;         // kReduceSlots * stride
   int ntiles, nchunks, M, in_graph;
@@ -201,6 +202,9 @@ nnpp_status launch_coarse_part_b(const Engine& e, const EngineView& v, int prec,
 nnpp_status launch_cg_update_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st,
                                cudaGraphConditionalHandle hc);
 bool engine_coarse(const Engine& e);  // the two-level preconditioner applies (every member has one)
+// the inner solve of a refinement sweep in one launch, in place of the CG launches above and below
+bool cg_sweep_applies(const Engine& e, int prec);
+nnpp_status launch_cg_sweep_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st);
 nnpp_status launch_cg_final_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st);
 nnpp_status launch_ir_update_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st,
                                cudaGraphConditionalHandle hc);

@@ -311,6 +311,7 @@ struct VecSel<float> {
   __device__ static float* q(const KParams& k) { return k.q32; }
   __device__ static float* e(const KParams& k) { return k.e32; }
   __device__ static const float* dinv(const KParams& k) { return k.dinv32; }
+  __device__ static const float* d(const KParams& k) { return k.d32; }
 };
 template <>
 struct VecSel<double> {
@@ -320,6 +321,7 @@ struct VecSel<double> {
   __device__ static double* q(const KParams& k) { return k.q64; }
   __device__ static double* e(const KParams& k) { return k.e64; }
   __device__ static const double* dinv(const KParams& k) { return k.dinv64; }
+  __device__ static const double* d(const KParams& k) { return k.dsum64; }
 };
 
 template <typename P>
@@ -1502,13 +1504,13 @@ __global__ void __launch_bounds__(kBlock, 1) k_cg_spmv32s(EngineView v, int stag
 
 // The FP64 operator's row sums on the CG slices: sum over this part's quads of w x[node] (FP64
 // weights, 32 bytes a lane and quad, next to the codes of the FP32 operator), two quads in flight.
-template <int K>
-__device__ __forceinline__ double cg_row64(const KParams& k, const SliceDesc& d, int width, int lane, int part,
-                                           const int* hb, const double* x) {
+// CONST: x does not change while the kernel runs.
+template <int K, bool CONST = true>
+__device__ __forceinline__ double cg_row64(const KParams& k, int off, int nq, int lane, int part, const int* hb,
+                                           const double* x) {
   constexpr int QB = 2;
-  const double* w64 = k.sell_cg64 + (size_t)(d.off >> 5) * 32 + 4 * lane;
-  const QuadPtr op(sell_cg_w(k, d), lane);
-  const int nq = (width + 3) >> 2;
+  const double* w64 = k.sell_cg64 + (size_t)(off >> 5) * 32 + 4 * lane;
+  const QuadPtr op(k.sell_cg + (size_t)(off >> 5) * kSellW, lane);
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   int q0 = part;
   for (; q0 + (QB - 1) * K < nq; q0 += QB * K) {
@@ -1522,7 +1524,10 @@ __device__ __forceinline__ double cg_row64(const KParams& k, const SliceDesc& d,
 #pragma unroll
     for (int u = 0; u < QB; ++u)
 #pragma unroll
-      for (int t = 0; t < 4; ++t) xv[u][t] = __ldg(x + code_node(hb, quad_code(code[u], t)));
+      for (int t = 0; t < 4; ++t) {
+        const double* xp = x + code_node(hb, quad_code(code[u], t));
+        xv[u][t] = CONST ? __ldg(xp) : *xp;
+      }
 #pragma unroll
     for (int u = 0; u < QB; ++u)
 #pragma unroll
@@ -1533,7 +1538,10 @@ __device__ __forceinline__ double cg_row64(const KParams& k, const SliceDesc& d,
     const uint2 code = op.codes(q0);
     ld_stream_d4(w64 + 128 * (size_t)q0, w);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) acc[t] = fma(w[t], __ldg(x + code_node(hb, quad_code(code, t))), acc[t]);
+    for (int t = 0; t < 4; ++t) {
+      const double* xp = x + code_node(hb, quad_code(code, t));
+      acc[t] = fma(w[t], CONST ? __ldg(xp) : *xp, acc[t]);
+    }
   }
   return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
@@ -1564,7 +1572,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_cg_spmv64(EngineView v) {
       live = a >= 0 && k.freem[a];
       if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
       __syncwarp();
-      if (live) sum[0] = cg_row64<K>(k, d, k.cg_width[ss.sg - first], lane, ss.part, s_hb[warp], k.z64);
+      if (live) sum[0] = cg_row64<K>(k, d.off, (k.cg_width[ss.sg - first] + 3) >> 2, lane, ss.part, s_hb[warp], k.z64);
     }
     if (K > 1) split_sum<K, 1>(sum, s_acc);
     if (have && ss.part == 0) {
@@ -1678,9 +1686,9 @@ __device__ __forceinline__ bool deflating(const KParams& k) {
 // from the stored rows.  Eight slots at a time (with aggregates two or more bins wide, a
 // node's bonds reach at most 8 aggregates): their loads and gathers are in flight together,
 // the sum runs in slot order.
-__device__ __forceinline__ float ap_apply(const KParams& k, int i) {
-  const float* xc = k.xc;
-  float s = __ldg(k.d32 + i) * __ldg(xc + __ldg(k.agg + i));
+// xc: x_c, in global or shared memory.
+__device__ __forceinline__ float ap_apply(const KParams& k, int i, const float* xc) {
+  float s = __ldg(k.d32 + i) * xc[__ldg(k.agg + i)];
   const size_t N = (size_t)k.N;
   int q = 0;
   for (; q + 8 <= k.ap_k; q += 8) {
@@ -1692,13 +1700,13 @@ __device__ __forceinline__ float ap_apply(const KParams& k, int i) {
       val[u] = __ldg(k.ap_val + (size_t)(q + u) * N + i);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) xv[u] = __ldg(xc + col[u]);
+    for (int u = 0; u < 8; ++u) xv[u] = xc[col[u]];
 #pragma unroll
     for (int u = 0; u < 8; ++u) s = fmaf(val[u], xv[u], s);
   }
   for (; q < k.ap_k; ++q) {
     const size_t o = (size_t)q * N + i;
-    s = fmaf(__ldg(k.ap_val + o), __ldg(xc + __ldg(k.ap_col + o)), s);
+    s = fmaf(__ldg(k.ap_val + o), xc[__ldg(k.ap_col + o)], s);
   }
   return s;
 }
@@ -2023,7 +2031,7 @@ __global__ void __launch_bounds__(kBlock) k_z_form(EngineView v, cudaGraphCondit
           const float ea = e[a];
           const float ra = rin[a];
           const float ta = t[a];
-          const float w = qa - ap_apply(k, a);
+          const float w = qa - ap_apply(k, a, k.xc);
           e[a] = ea + alpha * pa;
           const float r = ra - alpha * w;
           rin[a] = r;
@@ -2100,7 +2108,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_zdots(EngineView v, cudaGraphCond
         P zz;
         if (def) {
           if (di != P(0)) {
-            r = r - (P)ap_apply(k, a);
+            r = r - (P)ap_apply(k, a, k.xc);
             rin[a] = r;
           }
           zz = r * di;
@@ -2153,6 +2161,828 @@ __global__ void __launch_bounds__(kBlock) k_cg_zdots(EngineView v, cudaGraphCond
     __syncthreads();
   }
 }
+
+// ------------------------------------------------------- the inner solve in one launch ---
+// One refinement sweep's correction solve of a single instance with the two-level preconditioner,
+// start to end, in one cooperative launch: the CG's right-hand side and first z, every iteration, and
+// the deflated form's final correction (the same steps as the kernels above, which ensembles, the
+// Jacobi preconditioner and the other operators take).  An iteration has four passes -- operator,
+// restriction, coarse product, update -- of a few us each up to a few hundred thousand nodes, so as
+// launches they are bound by the gaps, the ramps and the last CTAs' reductions; here a CTA an SM stays
+// for the whole solve and meets the others between passes.  The dots are block partials that every
+// CTA sums again in the same order after it has met the others, so each takes the loop's decisions
+// itself, with the same bits.  A meeting takes 1.3 us, one that sums two values 3 to 4 (its chain of
+// FP64 instructions, 64 cycles each, is what was left of 10: hence the FP32 pairs, the values side by
+// side and the division while waiting).  A step, this against the launches (ms): 8k nodes 0.251 against
+// 0.358 mixed and 0.304 against 0.402 FP64, 64k 0.471 against 0.628, 262k 1.27 against 1.60, 512k 2.42
+// against 2.71 and 7.05 against 7.43, 2M 18.2 against 21.2.
+// NW: warps a CTA, see k_cg_sweep.
+struct SweepState {
+  double alpha, beta, rz, rr, pq, target;
+  double irz;                     // 1 / rz
+  double tol, inner_rel, bnorm2;  // the solve's settings
+  int it, solve_it, go, max_iter;
+};
+
+// The sums' parts: FP64, or FP32 pairs on the FP32 path (an FP64 instruction holds the pipe for 64 cycles,
+// and the chain of a reduction is what a meeting waits for)
+template <typename P>
+struct SweepSum;
+template <>
+struct SweepSum<double> {
+  double s;
+  __device__ __forceinline__ void add(const SweepSum& o) { s += o.s; }
+  __device__ __forceinline__ void shfl_add(int off) { s += __shfl_xor_sync(0xffffffffu, s, off); }
+  __device__ __forceinline__ double value() const { return s; }
+  __device__ __forceinline__ static SweepSum of(const DotAcc<double>& d) { return {d.s}; }
+  __device__ __forceinline__ static SweepSum of(double d) { return {d}; }
+};
+template <>
+struct SweepSum<float> {
+  float hi, lo;
+  __device__ __forceinline__ void add(const SweepSum& o) { pair_add(hi, lo, o.hi, o.lo); }
+  __device__ __forceinline__ void shfl_add(int off) {
+    const float h = __shfl_xor_sync(0xffffffffu, hi, off), l = __shfl_xor_sync(0xffffffffu, lo, off);
+    pair_add(hi, lo, h, l);
+  }
+  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ static SweepSum of(const DotAcc<float>& d) { return {d.hi, d.lo}; }
+};
+template <typename P>
+__device__ __forceinline__ SweepSum<P> sweep_load(const double* p) {
+  const double d = __ldcg(p);
+  if constexpr (sizeof(P) == 8) {
+    return {d};
+  } else {
+    const long long b = __double_as_longlong(d);
+    return {__int_as_float((int)(b & 0xffffffffll)), __int_as_float((int)(b >> 32))};
+  }
+}
+template <typename P>
+__device__ __forceinline__ void sweep_store(double* p, const SweepSum<P>& x) {
+  if constexpr (sizeof(P) == 8)
+    __stcg(p, x.s);
+  else
+    __stcg(p, __longlong_as_double((long long)((unsigned long long)(unsigned)__float_as_int(x.lo) << 32 |
+                                               (unsigned)__float_as_int(x.hi))));
+}
+// a / b by Newton steps on the reciprocal of b's significand (half of the compiler's FP64 instructions)
+__device__ __forceinline__ double sweep_div(double a, double b) {
+  const long long bits = __double_as_longlong(b);
+  const int ex = (int)(bits >> 52) & 0x7ff;
+  if (ex == 0 || ex >= 0x7fe) return a / b;
+  const double m = __longlong_as_double((bits & (long long)0x800fffffffffffffull) | 0x3ff0000000000000ll);
+  double x = (double)(1.0f / (float)m);
+  x = fma(x, fma(-m, x, 1.0), x);
+  x = fma(x, fma(-m, x, 1.0), x);
+  double q = a * x;
+  q = fma(fma(-m, q, a), x, q);
+  return q * __longlong_as_double((long long)(2046 - ex) << 52);
+}
+__device__ __forceinline__ bool sweep_finite(double x) {
+  return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
+}
+
+template <int NW, typename P>
+struct SweepSmem {
+  SweepSum<P> red[3 * NW];
+  SweepState st;
+  int fail;
+  int hb[NW][12];       // gather bases of the warp's slice
+  int off[NW], nq[NW];  // the planned slice: quad offset base and quads (0: none)
+  int2 runs[NW][32];
+};
+// A pass, inlined with 16 warps a CTA (128 registers), a function of its own with 32 (64 registers: one
+// body with all of them spills)
+#define NNPP_SWEEP_PASS(name, ...) (NW <= 16 ? name<__VA_ARGS__> : name##_fn<__VA_ARGS__>)
+
+// Every CTA of the launch meets here: what the others wrote before is visible after.  The warps' sums
+// of NV values (part, lane 0) come back as totals in decide(tot), which thread 0 runs before the CTA
+// goes on; waiting() is its work while the others come.  partials has two halves, used in turn (half): a CTA can be a meeting ahead of the last
+// one's reads, not two.  False when the wait gave up.
+template <int NV, int NW, typename P, typename F, typename H>
+__device__ __forceinline__ bool sweep_meet(const EngineView& v, SweepSmem<NW, P>& sm, unsigned int& target, int& half,
+                                           const SweepSum<P> (&part)[NV > 0 ? NV : 1], F&& decide, H&& waiting) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (NV > 0 && lane == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sm.red[q * NW + warp] = part[q];
+  __syncthreads();
+  if (warp == 0) {
+    // two values: half a warp each, so that their chains run at once
+    constexpr int kSeg = NV == 2 ? 16 : 32, kRounds = NV == 2 ? 1 : NV;
+    const int sub = lane % kSeg, G = gridDim.x;
+    double* buf = v.partials + (size_t)half * 3 * G;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int q = NV == 2 ? lane / 16 : r;
+      SweepSum<P> x{};
+#pragma unroll
+      for (int w = 0; w < NW; w += kSeg)
+        if (w + sub < NW) x.add(sm.red[q * NW + w + sub]);
+#pragma unroll
+      for (int off = kSeg / 2; off > 0; off >>= 1) x.shfl_add(off);
+      if (sub == 0) sweep_store<P>(buf + q * G + blockIdx.x, x);
+    }
+    unsigned int* count = v.ticket + v.M + 4;
+    target += G;
+    int ok = 1;
+    __syncwarp();
+    if (lane == 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+      waiting();
+      unsigned int seen, polls = 0;
+      do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+      } while ((int)(seen - target) < 0 && ++polls < kWaitPolls);
+      ok = (int)(seen - target) >= 0 ? 1 : 0;
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    double tot[NV > 0 ? NV : 1];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int q = NV == 2 ? lane / 16 : r;
+      constexpr int kU = 160 / kSeg;  // a lane's parts all in flight (160 CTAs a round)
+      SweepSum<P> x{};
+      for (int i0 = sub; i0 < G; i0 += 160) {
+        SweepSum<P> y[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          y[u] = SweepSum<P>{};
+          if (i0 + kSeg * u < G) y[u] = sweep_load<P>(buf + q * G + i0 + kSeg * u);
+        }
+#pragma unroll
+        for (int d = 1; d < kU; d *= 2)
+#pragma unroll
+          for (int u = 0; u + d < kU; u += 2 * d) y[u].add(y[u + d]);
+        x.add(y[0]);
+      }
+#pragma unroll
+      for (int off = kSeg / 2; off > 0; off >>= 1) x.shfl_add(off);
+      const double t = x.value();
+      if (NV == 2) {
+        tot[0] = __shfl_sync(0xffffffffu, t, 0);
+        tot[NV - 1] = __shfl_sync(0xffffffffu, t, 16);
+      } else {
+        tot[r] = t;
+      }
+    }
+    if (lane == 0) {
+      sm.fail = ok ? 0 : 1;
+      decide(tot);
+    }
+  }
+  half ^= 1;
+  __syncthreads();
+  return sm.fail == 0;
+}
+
+// The warp walks an aggregate's nodes: f(nodes) with U nodes a lane (-1: none), in a fixed order.  The
+// aggregate's bins along x are one contiguous node range; their bounds are loaded one run a lane and
+// the warp walks the runs' concatenation.
+template <int U, typename F>
+__device__ __forceinline__ void walk_aggregate(const KParams& k, int I, int lane, int2* runs, F&& f) {
+  const int ax = I % k.cna0, ay = (I / k.cna0) % k.cna1, az = I / (k.cna0 * k.cna1);
+  const int bx0 = ax * k.cf, nx = min(bx0 + k.cf, k.nb0) - bx0;
+  const int y0 = ay * k.cf, ny = min(y0 + k.cf, k.nb1) - y0;
+  const int z0 = az * k.cf, rows = ny * (min(z0 + k.cf, k.nb2) - z0);
+#pragma unroll 1
+  for (int g = 0; g < rows; g += 32) {
+    const int nr = min(32, rows - g);
+    int lo = 0, len = 0;
+    if (lane < nr) {
+      const int b0 = bx0 + k.nb0 * ((y0 + (g + lane) % ny) + k.nb1 * (z0 + (g + lane) / ny));
+      lo = __ldg(k.bin_start + b0);
+      len = __ldg(k.bin_start + b0 + nx) - lo;
+    }
+    int pre = len;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, pre, off);
+      if (lane >= off) pre += t;
+    }
+    const int total = __shfl_sync(0xffffffffu, pre, 31);
+    __syncwarp();
+    if (lane < nr) runs[lane] = make_int2(pre - len, lo);  // (first position, first node)
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < total; base += 32 * U) {
+      int node[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int idx = base + lane + 32 * u;
+        node[u] = -1;
+        if (idx < total)
+#pragma unroll 1
+          for (int r = 0; r < nr; ++r) {
+            const int2 ru = runs[r];
+            if (idx >= ru.x) node[u] = ru.y + (idx - ru.x);
+          }
+      }
+      f(node);
+    }
+  }
+}
+
+// x_c = A_c^-1 r_c, a warp a row; the warp's sum of r_c[I] x_c[I] (lane 0)
+template <typename P, int NW>
+__device__ __forceinline__ SweepSum<P> sweep_coarse(const KParams& k, float* srv) {
+  const int lane = threadIdx.x & 31;
+  const int nq = k.cld >> 2;
+  float4* sv4 = reinterpret_cast<float4*>(srv);
+  for (int i = threadIdx.x; i < nq; i += 32 * NW) sv4[i] = reinterpret_cast<const float4*>(k.rc)[i];
+  __syncthreads();
+  constexpr int kU = NW <= 16 ? kGemvU : kGemvU / 2;
+  DotAcc<P> dot;
+#pragma unroll 1
+  for (int I = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; I < k.cn; I += gridDim.x * NW) {
+    const float4* row = reinterpret_cast<const float4*>(k.cinv + (size_t)I * k.cld);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int j0 = lane; j0 < nq; j0 += 32 * kU) {
+      float4 a[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (j0 + 32 * u < nq) a[u] = __ldg(row + j0 + 32 * u);
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (j0 + 32 * u < nq) {
+          const float4 b = sv4[j0 + 32 * u];
+          acc[0] = fmaf(a[u].x, b.x, acc[0]);
+          acc[1] = fmaf(a[u].y, b.y, acc[1]);
+          acc[2] = fmaf(a[u].z, b.z, acc[2]);
+          acc[3] = fmaf(a[u].w, b.w, acc[3]);
+        }
+    }
+    float x = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+    if (lane == 0) {
+      k.xc[I] = x;
+      dot.add(srv[I], x);
+    }
+  }
+  return SweepSum<P>::of(dot);
+}
+
+// A part of a slice's row sums: sum of w x[node] over the quads part, part + K, ..., QB quads a batch, the
+// next batch's loads in flight
+template <int K, int QB>
+__device__ __forceinline__ float sweep_row(const KParams& k, int off, int nq, int lane, int part, const int* hb,
+                                           bool live) {
+  const QuadPtr op(k.sell_cg + (size_t)(off >> 5) * kSellW, lane);
+  const float* z = k.z32;
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float4 w[QB];
+  uint2 code[QB];
+  auto load = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < QB; ++u) {
+      w[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      code[u] = make_uint2(0u, 0u);
+      if (q0 + u * K < nq) {
+        w[u] = op.weights(q0 + u * K);
+        code[u] = op.codes(q0 + u * K);
+      }
+    }
+  };
+  if (!live) return 0.0f;
+  load(part);
+#pragma unroll 1
+  for (int q0 = part; q0 < nq; q0 += QB * K) {
+    float zv[4 * QB];
+#pragma unroll
+    for (int u = 0; u < 4 * QB; ++u) zv[u] = z[code_node(hb, quad_code(code[u >> 2], u & 3))];
+    float4 wc[QB];
+#pragma unroll
+    for (int u = 0; u < QB; ++u) wc[u] = w[u];
+    if (q0 + QB * K < nq) load(q0 + QB * K);
+#pragma unroll
+    for (int u = 0; u < 4 * QB; ++u) acc[u & 3] = fmaf(quad_weight(wc[u >> 2], u & 3), zv[u], acc[u & 3]);
+  }
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+}
+template <int K>
+__device__ __forceinline__ double sweep_row64(const KParams& k, int off, int nq, int lane, int part, const int* hb,
+                                              bool live) {
+  return live ? cg_row64<K, false>(k, off, nq, lane, part, hb, k.z64) : 0.0;
+}
+
+// q = A z + beta q, p = z + beta p on a slice that K warps share (lane's row a, -1: none); adds p.q.  Every
+// warp of the CTA calls it.  EARLY: the row's own values are loaded before its sum (four registers
+// more; a slice's chain of loads is shorter).
+template <bool EARLY, typename P, int K, int NW>
+__device__ __forceinline__ void sweep_slice(const KParams& k, SweepSmem<NW, P>& sm, P* s_acc, int off, int nq, int a, P beta,
+                                            DotAcc<P>& dot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % K;
+  const bool live = a >= 0, owner = live && part == 0;
+  P *p = VecSel<P>::p(k), *q = VecSel<P>::q(k);
+  P za = P(0), da = P(0), qa = P(0), pa = P(0);
+  auto own = [&] {
+    za = VecSel<P>::z(k)[a];
+    da = __ldg(VecSel<P>::d(k) + a);
+    qa = q[a];
+    pa = p[a];
+  };
+  if (EARLY && owner) own();
+  P sum;
+  if constexpr (sizeof(P) == 4)
+    sum = sweep_row<K, EARLY && NW <= 16 ? 4 : 2>(k, off, nq, lane, part, sm.hb[warp], live);
+  else
+    sum = sweep_row64<K>(k, off, nq, lane, part, sm.hb[warp], live);
+  if (K > 1) {
+    if (part) s_acc[threadIdx.x] = sum;
+    __syncthreads();
+    if (!part)
+#pragma unroll
+      for (int h = 1; h < K; ++h) sum += s_acc[threadIdx.x + 32 * h];
+  }
+  if (owner) {
+    if (!EARLY) own();
+    const P qn = da * za - sum + beta * qa;
+    const P pn = za + beta * pa;
+    q[a] = qn;
+    p[a] = pn;
+    dot.add(pn, qn);
+  }
+  if (K > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+}
+
+// The slice's gather bases into the warp's table; the lane's row (-1: not an unknown) and the slice's place
+template <typename P, int NW>
+__device__ __forceinline__ int sweep_take(const KParams& k, SweepSmem<NW, P>& sm, const SliceDesc* slices, int sg, int* off,
+                                          int* nq) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const SliceDesc& d = slices[sg];
+  const int row0 = __ldg(&d.row0), width = __ldg(k.cg_width + sg);
+  *off = __ldg(&d.off);
+  *nq = (width + 3) >> 2;
+  if (lane < 9) sm.hb[warp][lane] = __ldg(&d.gbase[lane]);
+  __syncwarp();
+  const int a = __ldg(k.cg_rows + row0 + lane);
+  return a >= 0 && __ldg(k.freem + a) ? a : -1;
+}
+
+// the slices [s0, s1), K warps each
+template <typename P, int K, int NW>
+__device__ __forceinline__ SweepSum<P> sweep_slices(const KParams& k, SweepSmem<NW, P>& sm, P* s_acc, const SliceDesc* slices,
+                                               int s0, int s1, P beta) {
+  constexpr int kGroup = NW / K;  // slices of a CTA at a time
+  DotAcc<P> dot;
+#pragma unroll 1
+  for (int base = s0 + blockIdx.x * kGroup; base < s1; base += gridDim.x * kGroup) {
+    const int sg = base + (threadIdx.x >> 5) / K;
+    int off = 0, nq = 0, a = -1;
+    if (sg < s1) a = sweep_take<P, NW>(k, sm, slices, sg, &off, &nq);
+    sweep_slice<false, P, K>(k, sm, s_acc, off, nq, a, beta, dot);
+  }
+  dot.warp_sum();
+  return SweepSum<P>::of(dot);
+}
+template <typename P, int K, int NW>
+__device__ __noinline__ SweepSum<P> sweep_slices_fn(const KParams& k, SweepSmem<NW, P>& sm, P* s_acc, const SliceDesc* slices,
+                                               int s0, int s1, P beta) {
+  return sweep_slices<P, K, NW>(k, sm, s_acc, slices, s0, s1, beta);
+}
+
+// the passes of the solve
+__device__ __forceinline__ int sweep_agg0() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }  // one an SM first
+__device__ __forceinline__ int sweep_aggs() { return gridDim.x * (blockDim.x >> 5); }
+__device__ __forceinline__ int sweep_node0() { return blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int sweep_nodes() { return gridDim.x * blockDim.x; }
+// x_c into shared memory (after the coarse product's meeting)
+__device__ __forceinline__ void sweep_stage(const KParams& k, float* srv) {
+  for (int i = threadIdx.x; i < k.cn; i += blockDim.x) srv[i] = k.xc[i];
+  __syncthreads();
+}
+__device__ __forceinline__ void sweep_store_rc(const KParams& k, int I, float acc) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+  if ((threadIdx.x & 31) == 0) k.rc[I] = acc;
+}
+
+// the right-hand side and its restriction
+template <typename P, int NW>
+__device__ __forceinline__ void sweep_rhs(const KParams& k, SweepSmem<NW, P>& sm) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int I = sweep_agg0(); I < k.cn; I += sweep_aggs()) {
+    float acc = 0.0f;
+    walk_aggregate<4>(k, I, lane, sm.runs[threadIdx.x >> 5], [&](const int (&node)[4]) {
+      P* rin = VecSel<P>::rin(k);
+      P* p = VecSel<P>::p(k);
+      P* q = VecSel<P>::q(k);
+      P* e = VecSel<P>::e(k);
+      double r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) r[u] = node[u] >= 0 ? k.r64[node[u]] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (node[u] >= 0) {
+          const int a = node[u];
+          rin[a] = (P)r[u];
+          p[a] = q[a] = e[a] = P(0);
+          if (sizeof(P) == 4) {  // the deflated solve's right-hand side and t = A e^
+            k.r0_32[a] = (float)r[u];
+            k.t32[a] = 0.0f;
+          }
+          acc += (float)(P)r[u];
+        }
+    });
+    sweep_store_rc(k, I, acc);
+  }
+}
+
+// z = M^-1 r; deflated: r^ = r - A P x_c, z = D^-1 r^.  The warp's r.z, r.r and the undeflated r.r
+template <typename P>
+struct Dots3 {
+  SweepSum<P> rz, rr, r0;
+};
+template <typename P>
+struct Dots2 {
+  SweepSum<P> a, b;
+};
+template <typename P, int NW>
+__device__ __forceinline__ Dots3<P> sweep_first_z(const KParams& k, float* srv, bool def) {
+  sweep_stage(k, srv);
+  P* rin = VecSel<P>::rin(k);
+  P* z = VecSel<P>::z(k);
+  const P* dinv = VecSel<P>::dinv(k);
+  DotAcc<P> part[3];
+#pragma unroll 1
+  for (int a = sweep_node0(); a < k.N; a += sweep_nodes()) {
+    const P di = dinv[a];
+    P r = rin[a];
+    part[2].add(r, r);
+    P zz = P(0);
+    if (di != P(0)) {
+      if (def) {
+        r = r - (P)ap_apply(k, a, srv);
+        rin[a] = r;
+        zz = r * di;
+      } else {
+        zz = r * di + (P)srv[__ldg(k.agg + a)];
+      }
+    }
+    z[a] = zz;
+    part[0].add(r, zz);
+    part[1].add(r, r);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) part[i].warp_sum();
+  return Dots3<P>{SweepSum<P>::of(part[0]), SweepSum<P>::of(part[1]), SweepSum<P>::of(part[2])};
+}
+
+// deflated iteration: r_c = P^T q (q is 0 off the unknowns)
+template <int NW>
+__device__ __forceinline__ void sweep_restrict_q(const KParams& k, SweepSmem<NW, float>& sm) {
+  const int lane = threadIdx.x & 31;
+  const float* q = k.q32;
+#pragma unroll 1
+  for (int I = sweep_agg0(); I < k.cn; I += sweep_aggs()) {
+    float acc = 0.0f;
+    walk_aggregate<8>(k, I, lane, sm.runs[threadIdx.x >> 5], [&](const int (&node)[8]) {
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = node[u] >= 0 ? q[node[u]] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += x[u];
+    });
+    sweep_store_rc(k, I, acc);
+  }
+}
+
+// deflated iteration: w = q - A P x_c, e^ += alpha p, r^ -= alpha w, t += alpha q, z = D^-1 r^; the
+// warp's r.z and r.r
+template <int NW>
+__device__ __forceinline__ Dots2<float> sweep_update(const KParams& k, float* srv, float alpha) {
+  sweep_stage(k, srv);
+  const float *dinv = k.dinv32, *q = k.q32, *p = k.p32;
+  float *e = k.e32, *rin = k.rin32, *t = k.t32, *z = k.z32;
+  DotAcc<float> rz, rr;
+#pragma unroll 1
+  for (int a = sweep_node0(); a < k.N; a += sweep_nodes()) {
+    const float di = dinv[a];
+    if (di == 0.0f) continue;
+    const float qa = q[a], pa = p[a], ea = e[a], ra = rin[a], ta = t[a];
+    const float w = qa - ap_apply(k, a, srv);
+    e[a] = ea + alpha * pa;
+    const float r = ra - alpha * w;
+    rin[a] = r;
+    t[a] = ta + alpha * qa;
+    const float zz = r * di;
+    z[a] = zz;
+    rz.add(r, zz);
+    rr.add(r, r);
+  }
+  rz.warp_sum();
+  rr.warp_sum();
+  return Dots2<float>{SweepSum<float>::of(rz), SweepSum<float>::of(rr)};
+}
+
+// additive iteration: e += alpha p, r -= alpha q with the restriction of r; the warp's r.D^-1 r and r.r
+template <typename P, int NW>
+__device__ __forceinline__ Dots2<P> sweep_update_restrict(const KParams& k, SweepSmem<NW, P>& sm, P alpha) {
+  const int lane = threadIdx.x & 31;
+  DotAcc<P> rzf, rr;
+#pragma unroll 1
+  for (int I = sweep_agg0(); I < k.cn; I += sweep_aggs()) {
+    float acc = 0.0f;
+    walk_aggregate<2>(k, I, lane, sm.runs[threadIdx.x >> 5], [&](const int (&node)[2]) {
+      P* rin = VecSel<P>::rin(k);
+      P* p = VecSel<P>::p(k);
+      P* q = VecSel<P>::q(k);
+      P* e = VecSel<P>::e(k);
+      const P* dinv = VecSel<P>::dinv(k);
+      P r[2], d[2], pv[2], qv[2], ev[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        r[u] = d[u] = pv[u] = qv[u] = ev[u] = P(0);
+        if (node[u] >= 0) {
+          r[u] = rin[node[u]];
+          d[u] = dinv[node[u]];
+          pv[u] = p[node[u]];
+          qv[u] = q[node[u]];
+          ev[u] = e[node[u]];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (d[u] != P(0)) {
+          e[node[u]] = ev[u] + alpha * pv[u];
+          r[u] = r[u] - alpha * qv[u];
+          rin[node[u]] = r[u];
+          rzf.add(r[u], r[u] * d[u]);
+          rr.add(r[u], r[u]);
+        }
+        acc += (float)r[u];
+      }
+    });
+    sweep_store_rc(k, I, acc);
+  }
+  rzf.warp_sum();
+  rr.warp_sum();
+  return Dots2<P>{SweepSum<P>::of(rzf), SweepSum<P>::of(rr)};
+}
+
+// additive iteration: z = D^-1 r + P x_c
+template <typename P, int NW>
+__device__ __forceinline__ void sweep_z(const KParams& k, float* srv) {
+  sweep_stage(k, srv);
+  P* rin = VecSel<P>::rin(k);
+  P* z = VecSel<P>::z(k);
+  const P* dinv = VecSel<P>::dinv(k);
+  for (int a = sweep_node0(); a < k.N; a += sweep_nodes()) {
+    const P di = dinv[a];
+    z[a] = di == P(0) ? P(0) : rin[a] * di + (P)srv[__ldg(k.agg + a)];
+  }
+}
+
+// the deflated solve's end, e = e^ + Q (r0 - t): the restriction, then the correction
+template <int NW>
+__device__ __forceinline__ void sweep_last_restrict(const KParams& k, SweepSmem<NW, float>& sm) {
+  const int lane = threadIdx.x & 31;
+  const float *dinv = k.dinv32, *r0 = k.r0_32, *t = k.t32;
+#pragma unroll 1
+  for (int I = sweep_agg0(); I < k.cn; I += sweep_aggs()) {
+    float acc = 0.0f;
+    walk_aggregate<4>(k, I, lane, sm.runs[threadIdx.x >> 5], [&](const int (&node)[4]) {
+      float x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        x[u] = node[u] >= 0 && dinv[node[u]] != 0.0f ? r0[node[u]] - t[node[u]] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc += x[u];
+    });
+    sweep_store_rc(k, I, acc);
+  }
+}
+template <int NW>
+__device__ __forceinline__ void sweep_last_add(const KParams& k, float* srv) {
+  sweep_stage(k, srv);
+  const float* dinv = k.dinv32;
+  float* e = k.e32;
+  for (int a = sweep_node0(); a < k.N; a += sweep_nodes())
+    if (dinv[a] != 0.0f) e[a] = e[a] + srv[__ldg(k.agg + a)];
+}
+
+// the same passes as functions (NNPP_SWEEP_PASS)
+template <typename P, int NW>
+__device__ __noinline__ SweepSum<P> sweep_coarse_fn(const KParams& k, float* srv) {
+  return sweep_coarse<P, NW>(k, srv);
+}
+template <typename P, int NW>
+__device__ __noinline__ void sweep_rhs_fn(const KParams& k, SweepSmem<NW, P>& sm) {
+  sweep_rhs<P, NW>(k, sm);
+}
+template <typename P, int NW>
+__device__ __noinline__ Dots3<P> sweep_first_z_fn(const KParams& k, float* srv, bool def) {
+  return sweep_first_z<P, NW>(k, srv, def);
+}
+template <int NW>
+__device__ __noinline__ void sweep_restrict_q_fn(const KParams& k, SweepSmem<NW, float>& sm) {
+  sweep_restrict_q<NW>(k, sm);
+}
+template <int NW>
+__device__ __noinline__ Dots2<float> sweep_update_fn(const KParams& k, float* srv, float alpha) {
+  return sweep_update<NW>(k, srv, alpha);
+}
+template <typename P, int NW>
+__device__ __noinline__ Dots2<P> sweep_update_restrict_fn(const KParams& k, SweepSmem<NW, P>& sm, P alpha) {
+  return sweep_update_restrict<P, NW>(k, sm, alpha);
+}
+template <typename P, int NW>
+__device__ __noinline__ void sweep_z_fn(const KParams& k, float* srv) {
+  sweep_z<P, NW>(k, srv);
+}
+template <int NW>
+__device__ __noinline__ void sweep_last_restrict_fn(const KParams& k, SweepSmem<NW, float>& sm) {
+  sweep_last_restrict<NW>(k, sm);
+}
+template <int NW>
+__device__ __noinline__ void sweep_last_add_fn(const KParams& k, float* srv) {
+  sweep_last_add<NW>(k, srv);
+}
+
+template <typename P, int NW>
+__global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
+  extern __shared__ __align__(16) float srv[];  // cld floats: r_c, then x_c
+  __shared__ SweepSmem<NW, P> sm;
+  __shared__ P s_acc[32 * NW];
+  // the parameters in shared memory: a meeting empties the L1, and every pass would fetch its
+  // pointers again
+  __shared__ KParams k;
+  for (int i = threadIdx.x; i < (int)(sizeof(KParams) / 4); i += 32 * NW)
+    reinterpret_cast<int*>(&k)[i] = reinterpret_cast<const int*>(v.inst)[i];
+  __syncthreads();
+  DevState* ds = k.ds;
+  if (threadIdx.x == 0) {
+    sm.st.tol = ds->tol;
+    sm.st.inner_rel = ds->inner_rel;
+    sm.st.bnorm2 = ds->bnorm2;
+    sm.st.max_iter = ds->max_iter;
+    sm.st.solve_it = ds->solve_iters;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (*((volatile int*)&ds->outer_active) == 0) return;  // every CTA alike: only the loop around sets it
+  const bool def = deflating<P>(k);
+  unsigned int target = 0;
+  int half = 0;
+  auto none = [](const double*) {};
+  auto idle = [] {};
+  auto meet = [&] {
+    const SweepSum<P> no[1] = {};
+    return sweep_meet<0, NW, P>(v, sm, target, half, no, none, idle);
+  };
+  // restriction done: the coarse product
+  auto coarse = [&] {
+    if (!meet()) return false;
+    NNPP_SWEEP_PASS(sweep_coarse, P, NW)(k, srv);
+    return meet();
+  };
+  auto next = [&](double rz, double rr) {
+    SweepState& s = sm.st;
+    s.beta = s.rz != 0.0 ? rz * s.irz : 0.0;
+    s.rz = rz;
+    s.rr = rr;
+    s.it += 1;
+    s.solve_it += 1;
+    s.go = s.alpha != 0.0 && sweep_finite(rr) && rr > s.target && s.it < s.max_iter && s.solve_it < s.max_iter;
+  };
+  // The slices over the warps: a warp each for the rounds that fill every warp, and the last round's
+  // shared by as many warps as there are for each.  Where all of them make one such round (small cases),
+  // a warp keeps its slice: its place and the lane's row are fetched once.
+  const int all = gridDim.x * NW;
+  const int whole = v.ncslices / all * all;
+  int split = 1;
+  while (split < 8 && (v.ncslices - whole) * 2 * split <= all) split *= 2;
+  int row = -1;
+  if (whole == 0) {
+    const int sg = blockIdx.x * (NW / split) + warp / split;
+    int off = 0, nq = 0;
+    if (sg < v.ncslices) row = sweep_take<P, NW>(k, sm, v.cslices, sg, &off, &nq);
+    if (lane == 0) {
+      sm.off[warp] = off;
+      sm.nq[warp] = nq;
+    }
+    __syncwarp();
+  }
+  auto shared_slices = [&](auto kc, P beta) {
+    constexpr int K = decltype(kc)::value;
+    if (whole) return NNPP_SWEEP_PASS(sweep_slices, P, K, NW)(k, sm, s_acc, v.cslices, whole, v.ncslices, beta);
+    DotAcc<P> dot;
+    sweep_slice<true, P, K>(k, sm, s_acc, sm.off[warp], sm.nq[warp], row, beta, dot);
+    dot.warp_sum();
+    return SweepSum<P>::of(dot);
+  };
+  auto apply = [&](P beta) {
+    SweepSum<P> dot{};
+    if (whole) dot = NNPP_SWEEP_PASS(sweep_slices, P, 1, NW)(k, sm, s_acc, v.cslices, 0, whole, beta);
+    if (split == 8)
+      dot.add(shared_slices(std::integral_constant<int, 8>(), beta));
+    else if (split == 4)
+      dot.add(shared_slices(std::integral_constant<int, 4>(), beta));
+    else if (split == 2)
+      dot.add(shared_slices(std::integral_constant<int, 2>(), beta));
+    else
+      dot.add(shared_slices(std::integral_constant<int, 1>(), beta));
+    return dot;
+  };
+  NNPP_SWEEP_PASS(sweep_rhs, P, NW)(k, sm);
+  bool ok = coarse();
+  if (ok) {
+    const Dots3<P> d = NNPP_SWEEP_PASS(sweep_first_z, P, NW)(k, srv, def);
+    const SweepSum<P> t[3] = {d.rz, d.rr, d.r0};
+    ok = sweep_meet<3, NW, P>(v, sm, target, half, t, [&](const double* tot) {
+      SweepState& s = sm.st;
+      s.rz = tot[0];
+      s.rr = tot[1];
+      s.beta = s.alpha = s.pq = 0.0;
+      s.it = 0;
+      // FP64: to the final tolerance in one sweep; mixed: by inner_rel of the correction equation's
+      // residual (before the deflation), not below what the outer tolerance needs
+      const double tb = s.tol * s.tol * s.bnorm2;
+      s.target = sizeof(P) == 4 ? fmax(s.inner_rel * s.inner_rel * tot[2], 0.09 * tb) : 0.25 * tb;
+      s.go = tot[1] > s.target && s.max_iter > 0;
+    }, idle);
+  }
+  while (ok && sm.st.go) {
+    const SweepSum<P> pq = apply((P)sm.st.beta);
+    auto inverse = [&] { sm.st.irz = sweep_div(1.0, sm.st.rz); };  // next()'s division, ahead
+    if (def) {
+      if constexpr (sizeof(P) == 4) {
+        const SweepSum<P> no[1] = {};
+        if (!(ok = sweep_meet<0, NW, P>(v, sm, target, half, no, none, inverse))) break;
+        NNPP_SWEEP_PASS(sweep_restrict_q, NW)(k, sm);
+        if (!(ok = meet())) break;
+        const SweepSum<P> d[2] = {pq, NNPP_SWEEP_PASS(sweep_coarse, P, NW)(k, srv)};
+        ok = sweep_meet<2, NW, P>(v, sm, target, half, d, [&](const double* tot) {
+          SweepState& s = sm.st;  // p.P_d A p = p.q - r_c.x_c
+          s.pq = tot[0];
+          const double pw = tot[0] - tot[1];
+          s.alpha = (tot[0] > 0.0 && pw > 0.0 && sweep_finite(pw)) ? sweep_div(s.rz, pw) : 0.0;
+        }, idle);
+        if (!ok) break;
+        const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update, NW)(k, srv, (float)sm.st.alpha);
+        const SweepSum<P> t[2] = {u.a, u.b};
+        ok = sweep_meet<2, NW, P>(v, sm, target, half, t, [&](const double* tot) { next(tot[0], tot[1]); }, idle);
+      }
+    } else {
+      const SweepSum<P> d[1] = {pq};
+      ok = sweep_meet<1, NW, P>(v, sm, target, half, d, [&](const double* tot) {
+        SweepState& s = sm.st;
+        s.pq = tot[0];
+        s.alpha = (tot[0] > 0.0 && sweep_finite(tot[0])) ? sweep_div(s.rz, tot[0]) : 0.0;
+      }, inverse);
+      if (!ok) break;
+      const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update_restrict, P, NW)(k, sm, (P)sm.st.alpha);
+      if (!(ok = meet())) break;
+      SweepSum<P> t[2] = {u.a, u.b};
+      t[0].add(NNPP_SWEEP_PASS(sweep_coarse, P, NW)(k, srv));  // r.D^-1 r + r_c.x_c
+      ok = sweep_meet<2, NW, P>(v, sm, target, half, t, [&](const double* tot) { next(tot[0], tot[1]); }, idle);
+      if (!ok) break;
+      NNPP_SWEEP_PASS(sweep_z, P, NW)(k, srv);
+      ok = meet();
+    }
+  }
+  if constexpr (sizeof(P) == 4)
+    if (ok && def) {
+      NNPP_SWEEP_PASS(sweep_last_restrict, NW)(k, sm);
+      ok = coarse();
+      if (ok) NNPP_SWEEP_PASS(sweep_last_add, NW)(k, srv);
+    }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (!ok) {
+      ds->wait_timeout = 1;
+    } else if (blockIdx.x == 0) {
+      const SweepState& s = sm.st;
+      ds->rz = s.rz;
+      ds->rr = s.rr;
+      ds->alpha = s.alpha;
+      ds->beta = s.beta;
+      ds->pq = s.pq;
+      ds->inner_target = s.target;
+      ds->inner_it = s.it;
+      ds->solve_iters = s.solve_it;
+      ds->cg_iters += s.it;
+      ds->inner_active = 0;
+    }
+    // the last CTA out sets the meeting's counters back
+    __threadfence();
+    if (atomicAdd(&v.ticket[v.M + 5], 1u) == gridDim.x - 1) {
+      v.ticket[v.M + 4] = 0;
+      v.ticket[v.M + 5] = 0;
+    }
+  }
+}
+#undef NNPP_SWEEP_PASS
 
 // ------------------------------------------------------------------- warm start ---------
 // Initial guess of the potential solve from the last H solutions x_n, ..., x_{n-H+1} and
@@ -2818,7 +3648,8 @@ __device__ __forceinline__ void refine_decide(DevState* ds, double rr) {
   ds->outer_it += 1;
   ds->outer_total += 1;
   const bool conv = rr <= ds->tol * ds->tol * ds->bnorm2;
-  const bool go = !conv && ds->outer_it < ds->max_outer && ds->solve_iters < ds->max_iter && isfinite(rr);
+  const bool go = !conv && ds->outer_it < ds->max_outer && ds->solve_iters < ds->max_iter && isfinite(rr) &&
+                  !ds->wait_timeout;
   if (!go) {
     ds->cg_solves += 1;
     ds->last_relres = sqrt(rr / ds->bnorm2);
@@ -2929,7 +3760,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_ir64(EngineView v, cudaGraphCondi
       live = a >= 0 && k.freem[a];
       if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
       __syncwarp();
-      if (live) sum[0] = cg_row64<K>(k, d, k.cg_width[ss.sg - first], lane, ss.part, s_hb[warp], k.e64);
+      if (live) sum[0] = cg_row64<K>(k, d.off, (k.cg_width[ss.sg - first] + 3) >> 2, lane, ss.part, s_hb[warp], k.e64);
     }
     if (K > 1) split_sum<K, 1>(sum, s_acc);
     if (have && ss.part == 0) {
@@ -4597,6 +5428,38 @@ nnpp_status launch_cg_init_b(const Engine& e, const EngineView& v, int prec, cud
   NNPP_CUDA(cudaGetLastError());
   if (split) return prec == NNPP_MIXED ? launch_coarse_z<float>(e, v, st, hc, 1) : launch_coarse_z<double>(e, v, st, hc, 1);
   return NNPP_OK;
+}
+
+// The inner solve in one launch (k_cg_sweep): single instances with the two-level preconditioner,
+// with the gathering operator (variant 0) or in FP64.
+bool cg_sweep_applies(const Engine& e, int prec) {
+  return e.members.size() == 1 && engine_coarse(e) && (prec == NNPP_FP64 || e.spmv_variant == 0);
+}
+
+template <typename P, int NW>
+nnpp_status launch_sweep_w(const Engine& e, const EngineView& v, cudaStream_t st) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(e.sms);
+  cfg.blockDim = dim3(32 * NW);
+  cfg.dynamicSmemBytes = (size_t)cld_max(e) * sizeof(float);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  NNPP_CUDA(cudaLaunchKernelEx(&cfg, k_cg_sweep<P, NW>, v));
+  return NNPP_OK;
+}
+// Slices up to which a CTA has 16 warps: four or more share each of them, and with 128 registers the
+// passes are inlined and a warp has four quads in flight; above, 32 warps of 64 registers.  Measured, 16
+// against 32 (ms a step): 8k nodes 0.251 against 0.322, 64k (1,429 slices) 0.494 against 0.471, 262k
+// 1.40 against 1.27, 2M 24.4 against 18.2.
+constexpr long long kSweepSlices = 152 * 4;
+nnpp_status launch_cg_sweep_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {
+  const bool few = v.ncslices <= kSweepSlices;
+  if (prec == NNPP_MIXED) return few ? launch_sweep_w<float, 16>(e, v, st) : launch_sweep_w<float, 32>(e, v, st);
+  return few ? launch_sweep_w<double, 16>(e, v, st) : launch_sweep_w<double, 32>(e, v, st);
 }
 
 nnpp_status launch_cg_spmv_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {

@@ -38,7 +38,7 @@ def _check(sim, o):
 
 
 @pytest.mark.parametrize("n,N", [(10, 1), (10, 33), (10, 997), (20, 8000), (28, 21951), (38, 54871),
-                                 (56, 175615)])
+                                 (56, 175615), (64, 262143)])
 @pytest.mark.parametrize("order", ["fp64", "mixed", "switch"])
 def test_sliced_steps(gpu, orc, n, N, order):
     nn = gpu
