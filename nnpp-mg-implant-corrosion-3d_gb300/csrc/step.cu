@@ -1711,18 +1711,36 @@ __device__ __forceinline__ float ap_apply(const KParams& k, int i, const float* 
   return s;
 }
 
-// warp per aggregate, the instances one after another
+// The coarse kernels' work: kBlock / 32 aggregates (a warp each) of one instance a tile, the instances'
+// tiles in one list, so that an ensemble's small coarse spaces run side by side (eight members of
+// 20,000 to 195,000 nodes: restriction 29 us and product 22 us with every warp on one instance after
+// another).  False past the last tile.
+constexpr int kAggTile = kBlock / 32;
+__device__ __forceinline__ bool agg_tile(const EngineView& v, int t, int* inst, int* first) {
+  for (int i = 0; i < v.M; ++i) {
+    const int n = v.inst[i].coarse ? (v.inst[i].cn + kAggTile - 1) / kAggTile : 0;
+    if (t < n) {
+      *inst = i;
+      *first = t * kAggTile;
+      return true;
+    }
+    t -= n;
+  }
+  return false;
+}
+
+// warp per aggregate
 template <typename P>
 __global__ void __launch_bounds__(kBlock) k_coarse_restrict(EngineView v, int which) {
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (int inst = 0; inst < v.M; ++inst) {
+  int inst, first;
+  for (int t = blockIdx.x; agg_tile(v, t, &inst, &first); t += gridDim.x) {
     const KParams& k = v.inst[inst];
-    if (!k.coarse || !coarse_active(k, which == 2 ? 0 : which)) continue;
+    if (!coarse_active(k, which == 2 ? 0 : which)) continue;
     if (which == 2 && !deflating<P>(k)) continue;  // the deflated solve's final correction only
     const P* r = VecSel<P>::rin(k);
-    for (int I = gw; I < k.cn; I += warps) {
+    const int I = first + (threadIdx.x >> 5);
+    if (I < k.cn) {
       const int ax = I % k.cna0, ay = (I / k.cna0) % k.cna1, az = I / (k.cna0 * k.cna1);
       const int bx0 = ax * k.cf, bx1 = min(bx0 + k.cf, k.nb0);
       float acc = 0.0f;
@@ -1748,9 +1766,8 @@ template <typename P>
 __global__ void __launch_bounds__(kBlock) k_cg_update_restrict(EngineView v) {
   __shared__ int2 s_runs[kBlock / 32][32];
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (int inst = 0; inst < v.M; ++inst) {
+  int inst, first;
+  for (int t = blockIdx.x; agg_tile(v, t, &inst, &first); t += gridDim.x) {
     const KParams& k = v.inst[inst];
     if (!coarse_active(k, 1)) continue;
     P* rin = VecSel<P>::rin(k);
@@ -1759,9 +1776,9 @@ __global__ void __launch_bounds__(kBlock) k_cg_update_restrict(EngineView v) {
     P* e = VecSel<P>::e(k);
     const P* dinv = VecSel<P>::dinv(k);
     const P alpha = (P)k.ds->alpha;
-    if (!k.coarse) continue;  // engines run the split iteration only when every member has one
     const bool def = deflating<P>(k);
-    for (int I = gw; I < k.cn; I += warps) {
+    const int I = first + (threadIdx.x >> 5);
+    if (I < k.cn) {
       const int ax = I % k.cna0, ay = (I / k.cna0) % k.cna1, az = I / (k.cna0 * k.cna1);
       const int bx0 = ax * k.cf, bx1 = min(bx0 + k.cf, k.nb0);
       if (def) {
@@ -1880,11 +1897,10 @@ __global__ void __launch_bounds__(kBlock, 3) k_coarse_gemv(EngineView v, int whi
   __shared__ double sm[3 * kBlock / 32];
   __shared__ int s_last;
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (int inst = 0; inst < v.M; ++inst) {
+  int inst, first;
+  for (int t = blockIdx.x; agg_tile(v, t, &inst, &first); t += gridDim.x) {
     const KParams& k = v.inst[inst];
-    if (!k.coarse || !coarse_active(k, which == 2 ? 0 : which)) continue;
+    if (!coarse_active(k, which == 2 ? 0 : which)) continue;
     if (which == 2 && !deflating<float>(k)) continue;  // the deflated solve's final correction only
     const int n = k.cn, ld = k.cld;
     const bool dm = def_mixed && k.defl_ok && *((volatile const int*)&k.ds->defl) != 0;
@@ -1908,7 +1924,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_coarse_gemv(EngineView v, int whi
     __syncthreads();
     const float4* sr4 = reinterpret_cast<const float4*>(srv);
     const int nq = ld >> 2;  // 16-byte groups per row
-    for (int I = gw; I < n; I += warps) {
+    const int I = first + (threadIdx.x >> 5);
+    if (I < n) {
       const float4* row = reinterpret_cast<const float4*>(k.cinv + (size_t)I * ld);
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       // rounds of kGemvU 16-byte loads per lane, all in flight before their products
@@ -2177,7 +2194,9 @@ __global__ void __launch_bounds__(kBlock) k_cg_zdots(EngineView v, cudaGraphCond
 // 0.358 mixed and 0.304 against 0.402 FP64, 64k 0.471 against 0.628, 262k 1.27 against 1.60, 512k 2.42
 // against 2.71 and 7.05 against 7.43, 2M 18.2 against 21.2.
 // NW: warps a CTA, see k_cg_sweep.
+template <typename P>
 struct SweepState {
+  P alpha_p, beta_p;              // alpha and beta as the passes use them
   double alpha, beta, rz, rr, pq, target;
   double irz;                     // 1 / rz
   double tol, inner_rel, bnorm2;  // the solve's settings
@@ -2239,14 +2258,20 @@ __device__ __forceinline__ double sweep_div(double a, double b) {
   q = fma(fma(-m, q, a), x, q);
   return q * __longlong_as_double((long long)(2046 - ex) << 52);
 }
+// comparisons by the bits (an FP64 comparison takes the FP64 pipe)
 __device__ __forceinline__ bool sweep_finite(double x) {
   return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
 }
+__device__ __forceinline__ bool sweep_nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+// x > 0, finite or infinite (a NaN fails sweep_finite, which goes with it)
+__device__ __forceinline__ bool sweep_positive(double x) { return __double_as_longlong(x) > 0; }
+// a > b for finite a and b >= 0
+__device__ __forceinline__ bool sweep_above(double a, double b) { return __double_as_longlong(a) > __double_as_longlong(b); }
 
 template <int NW, typename P>
 struct SweepSmem {
   SweepSum<P> red[3 * NW];
-  SweepState st;
+  SweepState<P> st;
   int fail;
   int hb[NW][12];       // gather bases of the warp's slice
   int off[NW], nq[NW];  // the planned slice: quad offset base and quads (0: none)
@@ -2847,13 +2872,14 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
     return meet();
   };
   auto next = [&](double rz, double rr) {
-    SweepState& s = sm.st;
-    s.beta = s.rz != 0.0 ? rz * s.irz : 0.0;
+    SweepState<P>& s = sm.st;
+    s.beta = sweep_nonzero(s.rz) ? rz * s.irz : 0.0;
+    s.beta_p = (P)s.beta;
     s.rz = rz;
     s.rr = rr;
     s.it += 1;
     s.solve_it += 1;
-    s.go = s.alpha != 0.0 && sweep_finite(rr) && rr > s.target && s.it < s.max_iter && s.solve_it < s.max_iter;
+    s.go = sweep_nonzero(s.alpha) && sweep_finite(rr) && sweep_above(rr, s.target) && s.it < s.max_iter && s.solve_it < s.max_iter;
   };
   // The slices over the warps: a warp each for the rounds that fill every warp, and the last round's
   // shared by as many warps as there are for each.  Where all of them make one such round (small cases),
@@ -2900,10 +2926,11 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
     const Dots3<P> d = NNPP_SWEEP_PASS(sweep_first_z, P, NW)(k, srv, def);
     const SweepSum<P> t[3] = {d.rz, d.rr, d.r0};
     ok = sweep_meet<3, NW, P>(v, sm, target, half, t, [&](const double* tot) {
-      SweepState& s = sm.st;
+      SweepState<P>& s = sm.st;
       s.rz = tot[0];
       s.rr = tot[1];
       s.beta = s.alpha = s.pq = 0.0;
+      s.beta_p = s.alpha_p = P(0);
       s.it = 0;
       // FP64: to the final tolerance in one sweep; mixed: by inner_rel of the correction equation's
       // residual (before the deflation), not below what the outer tolerance needs
@@ -2913,7 +2940,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
     }, idle);
   }
   while (ok && sm.st.go) {
-    const SweepSum<P> pq = apply((P)sm.st.beta);
+    const SweepSum<P> pq = apply(sm.st.beta_p);
     auto inverse = [&] { sm.st.irz = sweep_div(1.0, sm.st.rz); };  // next()'s division, ahead
     if (def) {
       if constexpr (sizeof(P) == 4) {
@@ -2923,25 +2950,27 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
         if (!(ok = meet())) break;
         const SweepSum<P> d[2] = {pq, NNPP_SWEEP_PASS(sweep_coarse, P, NW)(k, srv)};
         ok = sweep_meet<2, NW, P>(v, sm, target, half, d, [&](const double* tot) {
-          SweepState& s = sm.st;  // p.P_d A p = p.q - r_c.x_c
+          SweepState<P>& s = sm.st;  // p.P_d A p = p.q - r_c.x_c
           s.pq = tot[0];
           const double pw = tot[0] - tot[1];
-          s.alpha = (tot[0] > 0.0 && pw > 0.0 && sweep_finite(pw)) ? sweep_div(s.rz, pw) : 0.0;
+          s.alpha = (sweep_positive(tot[0]) && sweep_positive(pw) && sweep_finite(pw)) ? sweep_div(s.rz, pw) : 0.0;
+          s.alpha_p = (P)s.alpha;
         }, idle);
         if (!ok) break;
-        const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update, NW)(k, srv, (float)sm.st.alpha);
+        const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update, NW)(k, srv, sm.st.alpha_p);
         const SweepSum<P> t[2] = {u.a, u.b};
         ok = sweep_meet<2, NW, P>(v, sm, target, half, t, [&](const double* tot) { next(tot[0], tot[1]); }, idle);
       }
     } else {
       const SweepSum<P> d[1] = {pq};
       ok = sweep_meet<1, NW, P>(v, sm, target, half, d, [&](const double* tot) {
-        SweepState& s = sm.st;
+        SweepState<P>& s = sm.st;
         s.pq = tot[0];
-        s.alpha = (tot[0] > 0.0 && sweep_finite(tot[0])) ? sweep_div(s.rz, tot[0]) : 0.0;
+        s.alpha = (sweep_positive(tot[0]) && sweep_finite(tot[0])) ? sweep_div(s.rz, tot[0]) : 0.0;
+        s.alpha_p = (P)s.alpha;
       }, inverse);
       if (!ok) break;
-      const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update_restrict, P, NW)(k, sm, (P)sm.st.alpha);
+      const Dots2<P> u = NNPP_SWEEP_PASS(sweep_update_restrict, P, NW)(k, sm, sm.st.alpha_p);
       if (!(ok = meet())) break;
       SweepSum<P> t[2] = {u.a, u.b};
       t[0].add(NNPP_SWEEP_PASS(sweep_coarse, P, NW)(k, srv));  // r.D^-1 r + r_c.x_c
@@ -2962,7 +2991,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
     if (!ok) {
       ds->wait_timeout = 1;
     } else if (blockIdx.x == 0) {
-      const SweepState& s = sm.st;
+      const SweepState<P>& s = sm.st;
       ds->rz = s.rz;
       ds->rr = s.rr;
       ds->alpha = s.alpha;
@@ -5139,17 +5168,22 @@ __global__ void k_adj_solve_setup(KParams k, const Rec64* snap, const double* ps
   }
 }
 
-__global__ void k_sum_c0(KParams k, int mixed, double* out) {
+// out[block]: the block's share of sum c_0, in a fixed order; with parts, the sum of those
+__global__ void k_sum_c0(KParams k, int mixed, const double* parts, int n, double* out) {
   __shared__ double sm[kBlock / 32];
   double part[1] = {0.0};
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < k.N; a += gridDim.x * blockDim.x) {
-    if (mixed)
-      part[0] += (double)k.rec32_cur[a].c[0] + (double)k.clo[a].x;
-    else
-      part[0] += k.rec64_cur[a].c[0];
+  if (parts) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) part[0] += parts[i];
+  } else {
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < k.N; a += gridDim.x * blockDim.x) {
+      if (mixed)
+        part[0] += (double)k.rec32_cur[a].c[0] + (double)k.clo[a].x;
+      else
+        part[0] += k.rec64_cur[a].c[0];
+    }
   }
   block_sum<1, kBlock>(part, sm);
-  if (threadIdx.x == 0) *out = part[0];
+  if (threadIdx.x == 0) out[blockIdx.x] = part[0];
 }
 
 }  // namespace
@@ -5227,8 +5261,13 @@ nnpp_status launch_adj_solve_setup(Handle& h, const Rec64* snap, const double* p
 
 nnpp_status launch_sum_c0(Handle& h, double* out) {
   KParams kp = make_kparams(h, h.cur);
-  // one block: a fixed summation order, so repeated runs give the same mass to the bit
-  k_sum_c0<<<1, kBlock, 0, h.st>>>(kp, h.state_prec == NNPP_MIXED ? 1 : 0, out);
+  // block parts and their sum, a fixed summation order: repeated runs give the same mass to the bit.
+  // (One block alone took 0.65 ms at 262k nodes.)
+  double* parts = h.engine->d_partials.get();
+  const int mixed = h.state_prec == NNPP_MIXED ? 1 : 0;
+  const int blocks = std::max(1, std::min((h.N + kBlock - 1) / kBlock, h.engine->sms));
+  k_sum_c0<<<blocks, kBlock, 0, h.st>>>(kp, mixed, nullptr, 0, parts);
+  k_sum_c0<<<1, kBlock, 0, h.st>>>(kp, mixed, parts, blocks, out);
   NNPP_CUDA(cudaGetLastError());
   return NNPP_OK;
 }
@@ -5396,14 +5435,19 @@ int cld_max(const Engine& e) {
   return m;
 }
 
+// CTAs of the coarse kernels: one a tile of aggregates (agg_tile), at most eight an SM
+int coarse_grid(const Engine& e) {
+  long long tiles = 0;
+  for (const Handle* h : e.members) tiles += h->coarse.valid ? (h->coarse.n + kAggTile - 1) / kAggTile : 0;
+  return (int)std::max(1ll, std::min(tiles, (long long)e.sms * 8));
+}
+
 // z = M^-1 r with the two-level preconditioner: restriction, coarse solve, z and the dots
 template <typename P>
 nnpp_status launch_coarse_z(const Engine& e, const EngineView& v, cudaStream_t st, cudaGraphConditionalHandle hc,
                             int init) {
-  int nmax = 1;
-  for (const Handle* h : e.members) nmax = std::max(nmax, h->coarse.valid ? h->coarse.n : 0);
   const int which = init ? 0 : 1;
-  const int rg = std::max(1, std::min((nmax * 32 + kBlock - 1) / kBlock, e.sms * 8));
+  const int rg = coarse_grid(e);
   k_coarse_restrict<P><<<rg, kBlock, 0, st>>>(v, which);
   k_coarse_gemv<<<rg, kBlock, (size_t)cld_max(e) * sizeof(float), st>>>(v, which, 0, 0, 0);
   k_cg_zdots<P><<<occ_grid(k_cg_zdots<P>, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v, hc, init,
@@ -5505,7 +5549,7 @@ nnpp_status launch_cg_spmv_b(const Engine& e, const EngineView& v, int prec, cud
 // (every kernel passes over instances that are not deflating)
 nnpp_status launch_cg_final_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {
   if (prec != NNPP_MIXED || !engine_coarse(e) || e.members.size() != 1) return NNPP_OK;
-  const int rg = std::max(1, std::min((cld_max(e) * 32 + kBlock - 1) / kBlock, e.sms * 8));
+  const int rg = coarse_grid(e);
   const int cg = occ_grid(k_def_final, 0, e.sms, v.nchunks);
   k_def_final<<<cg, kBlock, 0, st>>>(v, 1);
   k_coarse_restrict<float><<<rg, kBlock, 0, st>>>(v, 2);
@@ -5518,9 +5562,7 @@ nnpp_status launch_cg_final_b(const Engine& e, const EngineView& v, int prec, cu
 // update fused with the restriction, coarse product, z and the dots
 template <typename P>
 nnpp_status launch_coarse_update(const Engine& e, const EngineView& v, cudaStream_t st, cudaGraphConditionalHandle hc) {
-  int nmax = 1;
-  for (const Handle* h : e.members) nmax = std::max(nmax, h->coarse.valid ? h->coarse.n : 0);
-  const int rg = std::max(1, std::min((nmax * 32 + kBlock - 1) / kBlock, e.sms * 8));
+  const int rg = coarse_grid(e);
   k_cg_update_restrict<P><<<rg, kBlock, 0, st>>>(v);
   if (e.members.size() == 1) {
     // one instance: the dots come from the aggregates, the decisions from the coarse product's
