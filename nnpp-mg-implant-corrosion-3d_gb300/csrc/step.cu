@@ -170,6 +170,9 @@ __device__ __forceinline__ void block_pair_sum(float (&h)[NV], float (&l)[NV], d
   }
   __syncthreads();
   if (wid == 0) {
+    // value q ends in lane q, so that one conversion (the FP64 pipe) serves all of them
+    static_assert(NV <= 32, "a value a lane");
+    float mh = 0.0f, ml = 0.0f;
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       float th = 0.0f, tl = 0.0f;
@@ -178,8 +181,15 @@ __device__ __forceinline__ void block_pair_sum(float (&h)[NV], float (&l)[NV], d
         tl = smf[q * (BLK / 32) + lane].y;
       }
       pair_warp_sum(th, tl);
-      out[q] = (double)th + (double)tl;
+      const float h0 = __shfl_sync(0xffffffffu, th, 0), l0 = __shfl_sync(0xffffffffu, tl, 0);
+      if (lane == q) {
+        mh = h0;
+        ml = l0;
+      }
     }
+    const double d = (double)mh + (double)ml;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) out[q] = __shfl_sync(0xffffffffu, d, q);
   }
   __syncthreads();
 }
@@ -3031,49 +3041,66 @@ __device__ __forceinline__ int warm_history(const KParams& k) {
   return n < k.hist_m ? n : k.hist_m;
 }
 
+// 1 / sqrt(x), x > 0: two Newton steps from the FP32 root of x scaled by a power of four into [1, 4)
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  const long long bits = __double_as_longlong(x);
+  const int ex = (int)(bits >> 52);
+  if (ex == 0 || ex >= 0x7ff) return 1.0 / sqrt(x);
+  const int odd = (ex + 1) & 1;  // x = m 2^(ex - 1023 - odd), an even power
+  const double m = __longlong_as_double((bits & 0x000fffffffffffffll) | (long long)(1023 + odd) << 52);
+  double y = (double)rsqrtf((float)m);
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const double r = fma(-m * y, y, 1.0);
+    y = fma(0.5 * y, r, y);
+  }
+  return y * __longlong_as_double((long long)(1023 - (ex - 1023 - odd) / 2) << 52);
+}
+
 // Solve the scaled Galerkin system by Cholesky; differences whose pivot falls below 1e-12
 // (near-dependent) or whose A-norm is below 1e-12 of the solution's (rounding level) end
-// the basis.  Thread 0 of one CTA.
-__device__ void warm_solve(const double (&tot)[kWarmSlots], int nd, DevState* ds) {
-  double G[kWarmD][kWarmD], r[kWarmD], d[kWarmD], L[kWarmD][kWarmD], y[kWarmD];
-  int q = 0;
-  for (int i = 0; i < kWarmD; ++i)
-    for (int j = i; j < kWarmD; ++j) G[i][j] = G[j][i] = tot[q++];
-  for (int i = 0; i < kWarmD; ++i) r[i] = tot[q++];
-  const double xax = tot[q];
-  int n = 0;
-  for (int i = 0; i < nd; ++i) {
-    if (!(G[i][i] > 1e-24 * xax) || !isfinite(G[i][i])) break;
-    d[i] = sqrt(G[i][i]);
-    n = i + 1;
-  }
+// the basis.  One warp: lane 5 i + j holds the scaled entry (i, j), lane 25 + i the right-hand side's i,
+// which takes the same steps as a sixth column.  (Thread 0 alone took 45 us, a chain of some 45 divisions
+// and roots of 25 FP64 instructions that each hold the pipe for 64 cycles.)
+__device__ void warm_solve(const double* tot, int nd, DevState* ds) {
+  static_assert(kWarmD * (kWarmD + 1) <= 32, "an entry a lane");
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int D = kWarmD, kRhs = D * D, kTri = D * (D + 1) / 2;
+  const int lane = threadIdx.x & 31;
+  const bool entry = lane < kRhs, rhs = lane >= kRhs && lane < kRhs + D;
+  const int i = entry ? lane / D : rhs ? lane - kRhs : 0, j = entry ? lane % D : D;
+  auto tri = [&](int p, int q) { return p * D - p * (p - 1) / 2 + (q - p); };  // p <= q
+  double c = entry ? tot[tri(min(i, j), max(i, j))] : rhs ? tot[kTri + i] : 0.0;
+  const double gd = tot[tri(lane < D ? lane : 0, lane < D ? lane : 0)];  // lanes < D: the diagonal
+  const bool use = lane < nd && lane < D && gd > 1e-24 * tot[kTri + D] && isfinite(gd);
+  const int n = __ffs(~__ballot_sync(kAll, use)) - 1;
+  const double dinv = use ? rsqrt_newton(gd) : 1.0;
+  c *= __shfl_sync(kAll, dinv, i);
+  const double dj = __shfl_sync(kAll, dinv, entry ? j : 0);
+  if (entry) c *= dj;
   int m = 0;
-  for (int j = 0; j < n; ++j) {
-    double sj = 1.0;
-    for (int k2 = 0; k2 < j; ++k2) sj -= L[j][k2] * L[j][k2];
-    if (!(sj > 1e-12)) break;
-    L[j][j] = sqrt(sj);
-    for (int i = j + 1; i < n; ++i) {
-      double si = G[i][j] / (d[i] * d[j]);
-      for (int k2 = 0; k2 < j; ++k2) si -= L[i][k2] * L[j][k2];
-      L[i][j] = si / L[j][j];
-    }
-    m = j + 1;
+  double inv = 0.0;  // lane q: 1 / L(q, q)
+  for (int q = 0; q < n; ++q) {
+    const double sq = __shfl_sync(kAll, c, q * D + q);
+    if (!(sq > 1e-12)) break;
+    const double iv = rsqrt_newton(sq);
+    if ((entry && j == q) || (rhs && i == q)) c *= iv;
+    const double li = __shfl_sync(kAll, c, i * D + q);
+    const double lj = __shfl_sync(kAll, c, entry ? j * D + q : kRhs + q);
+    if ((entry || rhs) && i > q && j > q) c = fma(-li, lj, c);
+    if (lane == q) inv = iv;
+    m = q + 1;
   }
-  for (int i = 0; i < m; ++i) {
-    double si = r[i] / d[i];
-    for (int k2 = 0; k2 < i; ++k2) si -= L[i][k2] * y[k2];
-    y[i] = si / L[i][i];
+  for (int q = m - 1; q >= 0; --q) {
+    const double y = __shfl_sync(kAll, c, kRhs + q) * __shfl_sync(kAll, inv, q);
+    const double l = __shfl_sync(kAll, c, q * D + i);  // L(q, i)
+    if (rhs && i == q) c = y;
+    if (rhs && i < q) c = fma(-l, y, c);
   }
-  bool ok = m > 0;
-  for (int i = m - 1; i >= 0; --i) {
-    double si = y[i];
-    for (int k2 = i + 1; k2 < m; ++k2) si -= L[k2][i] * y[k2];
-    y[i] = si / L[i][i];
-    ok = ok && isfinite(y[i]);
-  }
-  for (int i = 0; i < kWarmD; ++i) ds->warm_coef[i] = (ok && i < m) ? y[i] / d[i] : 0.0;
-  ds->warm_nd = ok ? m : 0;
+  const bool ok = m > 0 && __all_sync(kAll, !(rhs && i < m) || isfinite(c));
+  const double di = __shfl_sync(kAll, dinv, i);
+  if (rhs) ds->warm_coef[i] = ok && i < m ? c * di : 0.0;
+  if (lane == 0) ds->warm_nd = ok ? m : 0;
 }
 
 // backward differences D^1..D^{H-1} of the FP32 pairs t[0..H-1] (newest first) into d;
@@ -3100,13 +3127,47 @@ __device__ __forceinline__ void load_history_pairs(const double* ring, const int
   }
 }
 
+// A warp's sums of its lanes' 32 values, value q in lane q: at each step the lanes of a pair keep half of
+// the values each (31 pair sums instead of five a value)
+__device__ __forceinline__ void pair_warp_transpose_sum(float (&h)[32], float (&l)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < off; ++q) {
+      const float sh = up ? h[q] : h[q + off], sl = up ? l[q] : l[q + off];
+      float kh = up ? h[q + off] : h[q], kl = up ? l[q + off] : l[q];
+      pair_add(kh, kl, __shfl_xor_sync(0xffffffffu, sh, off), __shfl_xor_sync(0xffffffffu, sl, off));
+      h[q] = kh;
+      l[q] = kl;
+    }
+  }
+}
+
 // The Galerkin system's dot products, on FP32 pairs (the FP64 rate of the GB300 would
 // bound this pass): the history is split into pairs, differenced and multiplied with the
-// pair operations, ~2^-46 relative per operation.
+// pair operations, ~2^-46 relative per operation.  Up to 64k nodes it is the chain of the sums and of the
+// small solve: a value a lane in every stage of the sums, a warp in the solve.  A step of 8k nodes 0.251 ms
+// with 21 sums one after another and the solve in one thread, 0.215
+// so.
 template <typename P>
-__global__ void __launch_bounds__(kBlock) k_warm_dots(EngineView v) {
-  __shared__ double sm[kWarmSlots * kBlock / 32];
+__global__ void __launch_bounds__(kBlock, 2) k_warm_dots(EngineView v) {
+  constexpr int kW = kBlock / 32;
+  static_assert(kWarmSlots <= 32 && kWarmSlots <= kReduceSlots, "a value a lane");
+  __shared__ float2 s_sum[kW][32];
+  __shared__ double s_tot[32];
   __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* parts = reinterpret_cast<float2*>(v.partials);  // item i: kReduceSlots pairs
+  // the warps' pairs summed by lane (of warp 0)
+  auto across = [&](float& th, float& tl) {
+    __syncthreads();
+    th = tl = 0.0f;
+    if (warp == 0)
+#pragma unroll
+      for (int w = 0; w < kW; ++w) pair_add(th, tl, s_sum[w][lane].x, s_sum[w][lane].y);
+  };
   for (int item = blockIdx.x; item < v.nchunks; item += gridDim.x) {
     const Chunk c = v.chunks[item];
     const KParams& k = v.inst[c.inst];
@@ -3164,15 +3225,41 @@ __global__ void __launch_bounds__(kBlock) k_warm_dots(EngineView v) {
         part[q].add_pair(x0h, x0l, b0h, b0l);
       }
     }
-    write_dot_partials<kWarmSlots, float>(v, item, part, sm);
-    if (item_done(&v.ticket[c.inst], v.chunk_count[c.inst], &s_last)) {
-      double tot[kWarmSlots];
-      reduce_dot_items<kWarmSlots, float>(v.partials, v.stride, v.chunk_first[c.inst], v.chunk_count[c.inst], tot, sm);
-      if (threadIdx.x == 0) {
-        DevState* ds = k.ds;
-        ds->warm_nd = 0;
-        if (H >= 3) warm_solve(tot, H - 1, ds);
-        v.ticket[c.inst] = 0;
+    float sh[32], sl[32], th, tl;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      sh[q] = q < kWarmSlots ? part[q < kWarmSlots ? q : 0].hi : 0.0f;
+      sl[q] = q < kWarmSlots ? part[q < kWarmSlots ? q : 0].lo : 0.0f;
+    }
+    pair_warp_transpose_sum(sh, sl);
+    s_sum[warp][lane] = make_float2(sh[0], sl[0]);
+    across(th, tl);
+    if (warp == 0 && lane < kWarmSlots) parts[(size_t)item * kReduceSlots + lane] = make_float2(th, tl);
+    const int first = v.chunk_first[c.inst], count = v.chunk_count[c.inst];
+    if (item_done(&v.ticket[c.inst], count, &s_last)) {
+      // the last CTA: a warp takes every kW-th item, its lanes a value each
+      constexpr int U = 8;
+      float ah = 0.0f, al = 0.0f;
+      for (int i = warp; i < count; i += U * kW) {
+        float2 x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          x[u] = make_float2(0.0f, 0.0f);
+          if (i + u * kW < count && lane < kWarmSlots) x[u] = __ldcg(parts + (size_t)(first + i + u * kW) * kReduceSlots + lane);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) pair_add(ah, al, x[u].x, x[u].y);
+      }
+      s_sum[warp][lane] = make_float2(ah, al);
+      across(th, tl);
+      if (warp == 0) {
+        s_tot[lane] = (double)th + (double)tl;
+        if (lane == 0) {
+          k.ds->warm_nd = 0;
+          v.ticket[c.inst] = 0;
+        }
+        __syncwarp();
+        if (H >= 3) warm_solve(s_tot, H - 1, k.ds);
       }
     }
     __syncthreads();
