@@ -9,6 +9,7 @@
 #include <climits>
 #include <cmath>
 #include <utility>
+#include <type_traits>
 #include <vector>
 
 #include "neighbours.cuh"
@@ -258,8 +259,9 @@ __global__ void k_scan_nodes(int n, const int* __restrict__ order, const int* __
 // Warp per node.  Visits the cells within one cell of the sphere's bounding box in
 // ascending hash order, keeps those that pass the reference's sphere-cube test, and
 // appends the members of each (in the sorted order) that pass the horizon test, so the
-// list equals the reference's scan over all cells (grid.h:157-196).  Pass FILL=false
-// counts (lengths without self), FILL=true writes the CSR columns.
+// list equals the reference's scan over all cells (grid.h:157-196).  kScanCount counts (lengths
+// without self), kScanFill writes the CSR columns, kScanBoth counts and writes the columns at
+// max_node_no - 1 a node.
 //
 // Both tests are decided in FP32 on positions relative to the cells' corners in units of r,
 // where the squared distance is off by less than eps (see scan_eps): below 1 - eps a test
@@ -268,7 +270,8 @@ __global__ void k_scan_nodes(int n, const int* __restrict__ order, const int* __
 // the reference's cells of ten spacings are ~1,500 FP64 instructions a warp, which at 64 cycles
 // each took 53 ms a pass at 512k nodes; in FP32, four candidates a lane in flight and a cell a
 // lane, a pass takes 3.4 ms.  Nodes in cell order: the warps of a CTA scan the same cells.
-template <bool FILL>
+enum { kScanCount, kScanFill, kScanBoth };
+template <int MODE>
 __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, double x0, double y0, double z0,
                             double cx, double cy, double cz, int mx, int my, int max_hash,
@@ -299,8 +302,8 @@ __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* _
     long long cells = 0;
     if (nx > 0 && ny > 0 && hi[2] >= lo[2]) cells = (long long)nx * ny * (hi[2] - lo[2] + 1);
     int fill = 0;
-    const int rbase = FILL ? row_ptr[i] : 0;
     const int cap = max_node_no - 1;
+    const size_t rbase = MODE == kScanFill ? (size_t)row_ptr[i] : (size_t)i * cap;
     for (long long c0 = 0; c0 < cells; c0 += 32) {
       // a cell a lane, in ascending hash order
       const long long c = c0 + lane;
@@ -365,7 +368,7 @@ __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* _
               pass = pass && cand != i;
             }
             const unsigned int bal = __ballot_sync(0xffffffffu, pass);
-            if (FILL && pass) {
+            if (MODE != kScanCount && pass) {
               const int pos = fill + __popc(bal & ((1u << lane) - 1u));
               if (pos < cap) cols[rbase + pos] = cand;
             }
@@ -374,12 +377,24 @@ __global__ void k_cell_scan(int n, const double* __restrict__ x, const double* _
         }
       }
     }
-    if (!FILL && lane == 0) {
+    if (MODE != kScanFill && lane == 0) {
       len[i] = fill;
       if (fill + 1 > max_node_no) atomicExch(err, 1);
     }
   }
 }
+
+// the rows of kScanBoth to the CSR columns, a warp a row
+__global__ void k_pack_rows(int n, int cap, const int* __restrict__ ptr, const int* __restrict__ rows, int* cols) {
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+    const int p0 = ptr[i], len = ptr[i + 1] - p0;
+    for (int j = lane; j < len; j += 32) cols[p0 + j] = rows[(size_t)i * cap + j];
+  }
+}
+// columns of the one-scan build's rows; above it (a large max_node_no) a second scan is cheaper than
+// the memory.  512k nodes, max_node_no 160: one scan and the packing 3.7 ms against 6.8 for two scans
+constexpr long long kScanRowsMax = 1ll << 29;
 
 // Variant of k_cell_scan for the allocation-free build: one pass that writes the padded
 // column-major output directly (self at column 0, grid.h:170-171), the lengths (self
@@ -670,10 +685,20 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
   k_scan_nodes<<<grid_for(N, 256), 256, 0, st>>>(N, order.get(), hash.get(), x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
                                                  1.0 / r, nodes.get());
   const float eps = scan_eps(r, cx, cy, cz);
-  k_cell_scan<false><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
-                                                 max_hash, r, eps, start.get(), nodes.get(),
-                                                 max_node_no, len.get(), nullptr, nullptr,
-                                                 err.get());
+  // one scan into rows of max_node_no - 1 columns where those are a few bytes more than the lists (up to
+  // 2 GB), packed after; two scans, the lengths first, otherwise
+  const long long cap = max_node_no - 1;
+  DBuf<int> rows;
+  const bool both = cap > 0 && cap * N <= kScanRowsMax && rows.alloc((size_t)(cap * N));
+  auto scan = [&](auto mode, int* cols) {
+    k_cell_scan<decltype(mode)::value><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my, max_hash, r,
+                                                                  eps, start.get(), nodes.get(), max_node_no, len.get(),
+                                                                  out.ptr.get(), cols, err.get());
+  };
+  if (both)
+    scan(std::integral_constant<int, kScanBoth>(), rows.get());
+  else
+    scan(std::integral_constant<int, kScanCount>(), nullptr);
   NNPP_CUDA(cudaGetLastError());
   int herr = 0;
   NNPP_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -685,10 +710,10 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
   if (nnz < 0 || nnz > (long long)INT_MAX)
     return set_error(NNPP_ERR_UNSUPPORTED, "build: more than 2^31-1 bonds");
   if (!out.col.alloc(nnz > 0 ? nnz : 1)) return set_error(NNPP_ERR_NOMEM, "neighbour columns");
-  k_cell_scan<true><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
-                                                max_hash, r, eps, start.get(), nodes.get(),
-                                                max_node_no, nullptr, out.ptr.get(),
-                                                out.col.get(), err.get());
+  if (both)
+    k_pack_rows<<<warps_grid, 256, 0, st>>>(N, (int)cap, out.ptr.get(), rows.get(), out.col.get());
+  else
+    scan(std::integral_constant<int, kScanFill>(), out.col.get());
   NNPP_CUDA(cudaGetLastError());
   DBuf<int> dml;
   if (!dml.alloc(1)) return set_error(NNPP_ERR_NOMEM, "max length");

@@ -45,3 +45,20 @@ def test_scan_ties_and_cells(gpu, orc, shape, r_cells, cell_factor):
     assert ml == ml_o
     assert np.array_equal(lengths, len_o)
     assert np.array_equal(clouds, expect)
+
+
+@pytest.mark.parametrize("N", [1, 33, 1000])
+def test_one_scan_and_two_scans_agree(gpu, N):
+    """The one-scan build (rows of max_node_no - 1 columns, packed) against the two-scan build that a
+    max_node_no too large for such rows takes: the same lists."""
+    nn = gpu
+    inp = nn.synth(1, 10, seed=2)
+    args = [inp["params"]] + [np.ascontiguousarray(inp[k][..., :N])
+                              for k in ("nodes", "bctypes", "bcvalues", "icvalues", "phase0")]
+    out = []
+    for most in (200, (1 << 29) // N + 2):
+        sim = nn.Simulation(*args)
+        sim.build_neighbours(most)
+        out.append(sim.neighbours_csr())
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
