@@ -5,7 +5,12 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <exception>
+#include <thread>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "engine.cuh"
 
@@ -198,6 +203,39 @@ nnpp_status one_view(Handle& h, const KParams& k, OneView& ov) {
 }  // namespace
 
 // ======================================================================== C ABI ==========
+namespace {
+// A large host result's pages, faulted in by a thread while the device works: the copy into pages that
+// nothing has touched yet spends its time on the faults (328 MB of lists of 512,000 nodes: 12.2 ms fresh,
+// 1.7 ms touched).  The contents do not change, and a range that cannot be populated (or a kernel without
+// the call) is left to the copy.
+class Prefault {
+ public:
+  Prefault(void* p, size_t bytes) {
+#ifdef __linux__
+    if (!p || bytes < kMin) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t a = ((uintptr_t)p + page - 1) / page * page, e = ((uintptr_t)p + bytes) / page * page;
+    if (e <= a) return;
+    try {
+      t_ = std::thread([a, e] { madvise((void*)a, e - a, kPopulateWrite); });
+    } catch (const std::exception&) {  // no thread: the copy faults the pages in
+    }
+#endif
+  }
+  void wait() {
+    if (t_.joinable()) t_.join();
+  }
+  ~Prefault() { wait(); }
+  Prefault(const Prefault&) = delete;
+  Prefault& operator=(const Prefault&) = delete;
+
+ private:
+  static constexpr size_t kMin = 16u << 20;
+  static constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
+  std::thread t_;
+};
+}  // namespace
+
 extern "C" {
 
 int nnpp_device_count(void) {
@@ -265,6 +303,7 @@ nnpp_status nnpp_build_clouds_hash(int max_node_no, double r, double dx, double 
   cudaStream_t st;
   NNPP_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   nnpp_status res = NNPP_OK;
+  Prefault pages(clouds_colmajor, max_node_no > 0 ? sizeof(int) * (size_t)max_node_no * (size_t)n_nodes : 0);
   {
     DBuf<double> xyz;
     RefLists L;
@@ -275,6 +314,7 @@ nnpp_status nnpp_build_clouds_hash(int max_node_no, double r, double dx, double 
                       cudaMemcpyHostToDevice, st);
       res = build_ref_lists(st, n_nodes, xyz.get(), xyz.get() + n_nodes, xyz.get() + 2 * (size_t)n_nodes,
                             max_node_no, r, dx, dy, dz, order_mode, L);
+      pages.wait();
       if (res == NNPP_OK) res = emit_padded(st, L, max_node_no, clouds_colmajor, cloud_lengths);
       if (res == NNPP_OK && max_cloud_length) *max_cloud_length = L.max_len;
     }
@@ -351,9 +391,11 @@ nnpp_status nnpp_build_neighbours(nnpp_handle* hp, int max_node_no, double r, do
   }
   h.built = false;
   h.implicit_work.reset();
+  Prefault pages(clouds_colmajor, max_node_no > 0 ? sizeof(int) * (size_t)max_node_no * (size_t)h.N : 0);
   NNPP_TRY(build_ref_lists(h.st, h.N, h.ux.get(), h.uy.get(), h.uz.get(), max_node_no, r, cx, cy, cz,
                            order_mode, h.ref));
   h.max_node_no = max_node_no;
+  pages.wait();
   NNPP_TRY(emit_padded(h.st, h.ref, max_node_no, clouds_colmajor, cloud_lengths));
   if (max_cloud_length) *max_cloud_length = h.ref.max_len;
   const nnpp_params& p = h.p;
