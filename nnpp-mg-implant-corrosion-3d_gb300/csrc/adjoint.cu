@@ -396,7 +396,7 @@ nnpp_status nnpp_backward(nnpp_handle* hp, const double* dL_dmass, double* grad_
         NNPP_TRY(launch_adj_transport(e, v, sn, sn1, lam.get(), mu.get(), nu.get(), acc.get(), h.st));
       // adjoint potential solve on the unknowns of step n
       NNPP_TRY(coarse_select(h, n));
-      NNPP_TRY(launch_adj_solve_setup(h, sn, psi.get()));
+      NNPP_TRY(launch_adj_solve_setup(h, sn, psi.get(), n == s1 - 1));
       h.b_override = nu.get();
       if (hm >= 3) {
         // the adjoint potentials form their own warm-start ring

@@ -222,7 +222,7 @@ nnpp_status launch_snap_state(Handle& h, Rec64* dst);
 nnpp_status launch_snap_phi(Handle& h, Rec64* dst);
 // a stored solved potential into phi64, the current records and the snapshot dst
 nnpp_status launch_load_phi(Handle& h, const double* phi, Rec64* dst);
-nnpp_status launch_adj_solve_setup(Handle& h, const Rec64* snap, const double* psi_prev);
+nnpp_status launch_adj_solve_setup(Handle& h, const Rec64* snap, const double* psi_prev, bool first);
 nnpp_status launch_record_solve(Handle& h, int slot);
 nnpp_status launch_adj_transport32(const Engine& e, const EngineView& v, Handle& h, const Rec64* snap,
                                    const Rec64* snap1, const double* lam, float4* rec, double* mu,
