@@ -259,26 +259,56 @@ __device__ __forceinline__ int seg_or(int v) {
   return v;
 }
 
+// A warp's sums of eight FP64 values a lane, all of them in every lane: the lanes of a pair keep half of
+// the values each, 9 additions (of 64 cycles) instead of 40
+__device__ __forceinline__ void warp_sums8(double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  double x[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) x[q] = v[q];
+#pragma unroll
+  for (int n = 4, off = 16; n > 0; n >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < n) {
+        const double send = up ? x[q] : x[q + n], keep = up ? x[q + n] : x[q];
+        x[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+  }
+  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+  // value q in the lanes whose bits 4, 3, 2 spell q
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = __shfl_sync(0xffffffffu, x[0], q << 2);
+}
+
+// a warp's sums of NV values, in lane 0
+template <int NV>
+__device__ __forceinline__ void warp_sums(double (&v)[NV]) {
+  if constexpr (NV == 8) {
+    warp_sums8(v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+  }
+}
+
 // Block-wide sum of NV doubles per thread into block_out[NV] (thread 0 holds the result).
 template <int NV, int BLOCK>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* smem /* NV*BLOCK/32 */) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  warp_sums<NV>(v);
+  if (lane == 0)
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double x = v[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-    if (lane == 0) smem[k * (BLOCK / 32) + wid] = x;
-  }
+    for (int k = 0; k < NV; ++k) smem[k * (BLOCK / 32) + wid] = v[k];
   __syncthreads();
   if (wid == 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double x = (lane < BLOCK / 32) ? smem[k * (BLOCK / 32) + lane] : 0.0;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-      v[k] = x;
-    }
+    for (int k = 0; k < NV; ++k) v[k] = (lane < BLOCK / 32) ? smem[k * (BLOCK / 32) + lane] : 0.0;
+    warp_sums<NV>(v);
   }
   __syncthreads();
 }

@@ -810,10 +810,30 @@ struct SplitSlice {
   int sg, part;
   __device__ __forceinline__ SplitSlice(int base) : sg(base + (threadIdx.x >> 5) / K), part((threadIdx.x >> 5) % K) {}
 };
-// the parts' sums of NV values a lane: part 0 gets the totals, in part order (sm: kBlock * NV)
+// the parts' sums of NV values a lane: part 0 gets the totals, in part order (sm: kBlock * NV).  With as
+// many values as parts each part adds a share of them (16 FP64 values of eight parts are 112 additions
+// of 64 cycles in part 0 alone).
 template <int K, int NV, typename T>
 __device__ __forceinline__ void split_sum(T (&v)[NV], T* sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if constexpr (NV >= K && K > 1) {
+    const int part = warp % K;
+    T* own = sm + (size_t)(warp - part) * NV * 32 + lane;  // part 0's values, the next part's NV * 32 on
+#pragma unroll
+    for (int q = 0; q < NV; ++q) own[(part * NV + q) * 32] = v[q];
+    __syncthreads();
+    for (int q = part; q < NV; q += K) {
+      T t = own[q * 32];
+#pragma unroll
+      for (int h = 1; h < K; ++h) t += own[(h * NV + q) * 32];
+      own[q * 32] = t;
+    }
+    __syncthreads();
+    if (part == 0)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[q] = own[q * 32];
+    return;
+  }
   if (warp % K)
 #pragma unroll
     for (int q = 0; q < NV; ++q) sm[(warp * NV + q) * 32 + lane] = v[q];
@@ -3989,7 +4009,7 @@ __device__ __forceinline__ double dissolve_switch(double c0, double csat, double
   return c0 > csat ? 1.0 : 0.0;
 }
 
-constexpr int kDiagSlots = 9;  // mass[4], solid, vol, dissolved, nonfinite, spare
+constexpr int kDiagSlots = 8;  // mass[4], solid, vol, dissolved, nonfinite
 
 // Per-step diagnostics of one instance from its reduced transport partials (thread 0).
 __device__ __forceinline__ void finish_instance(const KParams& k, const double (&tot)[kDiagSlots]) {
@@ -4646,8 +4666,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_transport64(EngineView v) {
         part[6] = k.k_diss * swv;
         part[7] = bad ? 1.0 : 0.0;
       }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) part[q] = warp_sum_d(part[q]);
+      static_assert(kDiagSlots == 8, "warp_sums8");
+      warp_sums8(part);
       slice_partials64<kDiagSlots>(v, inst, __ldg(&v.slice_first[inst]), __ldg(&v.slice_count[inst]), ss.sg, part);
     }
     if (K > 1) __syncthreads();
