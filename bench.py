@@ -635,16 +635,17 @@ def run_ours(args):
     inner = d1["cg_iterations_total"] - d0["cg_iterations_total"]
     outer = d1["outer_iterations_total"] - d0["outer_iterations_total"]
     solves = d1["cg_solves"] - d0["cg_solves"]
-    # per solve: warm-start dots + apply, phi pairs + prep; per outer iteration cg_init +
-    # refinement; per CG iteration spmv + update; with the coarse correction restrict + coarse
-    # product + z/dots after every cg_init, coarse product + z after every (restricting)
-    # update; per step the transport
-    launches = 4 * solves + 2 * outer + 2 * inner + args.steps + ((2 * inner + 3 * outer) if cn else 0)
-    # coarse checks (one phase comparison each) and rebuilds (assembly, Newton-Schulz start,
-    # at most 18 steps' 2I - T, symmetrisation, two A P passes, phase snapshot; the GEMMs are
-    # cuBLAS's)
+    # per solve: warm-start dots + apply, phi pairs + prep; per step the transport and the next
+    # guess's pass; per outer iteration the refinement and, with the two-level preconditioner and
+    # operator 0, the inner solve in one launch, otherwise cg_init, per CG iteration the operator and
+    # the update, and with the coarse correction the restriction, the coarse product and z
+    launches = 4 * solves + 2 * outer + 2 * args.steps
+    if not cn or sim.tuning()[2] != 0:
+        launches += 2 * inner + ((2 * inner + 3 * outer) if cn else 0)
+    # coarse checks (one phase comparison each) and rebuilds (A P, assembly, the direct inverse's
+    # levels, phase snapshot)
     if pk and refresh > 0:
-        launches += -(-args.steps // refresh) + 24 * (rb1 - rb0)
+        launches += -(-args.steps // refresh) + 28 * (rb1 - rb0)
 
     # end to end through the public API with host buffers (nnpp_step_host): a second handle
     # of the same workload, after the same warm-up, steps the same steps as the timed region

@@ -352,7 +352,8 @@ nnpp_status nnpp_set_checks(nnpp_handle* h, int flags);
  * since the handle was built, of which warm-started (Newton-Schulz from the previous
  * inverse); rebuilds triggered by phase changes during runs and their summed duration in
  * milliseconds (host clock, the stream drained before and after: the time a run spends on
- * them); the Newton-Schulz steps of the last rebuild.  Any pointer may be NULL.  No
+ * them); the Newton-Schulz steps of the last rebuild (0: inverted directly; the iteration is for
+ * operators too near singular for that).  Any pointer may be NULL.  No
  * counterpart in the reference (measurement). */
 nnpp_status nnpp_get_coarse_stats(nnpp_handle* h, int64_t* rebuilds, int64_t* warm_rebuilds,
                                   int64_t* run_rebuilds, double* run_rebuild_ms,
@@ -409,9 +410,10 @@ nnpp_status nnpp_time_kernel(nnpp_handle* h, int kernel_id, int precision, int r
                              double* ms_per_launch);
 
 /* The execution configuration of the handle's kernels: bins per tile, lanes per node of the
- * FP64 tile kernels, and the FP32 CG operator's variant: 0 / 3 gathers from L1/L2 (batches
- * of 16 bond columns; 0 keeps the next batch's stream in flight), 1 operator and slice windows streamed by bulk copies into shared
- * memory, 2 / 4 slice windows copied into shared memory by asynchronous copies (batches of
+ * residual entry points' tile kernels, and the FP32 CG operator's variant: 0 / 3 gathers from
+ * L1/L2 (batches of 16 / 8 bond columns, the next batch in flight; a single instance with the
+ * two-level preconditioner runs its whole inner solve with 0 in one launch), 1 operator and
+ * slice windows streamed by bulk copies into shared memory, 2 / 4 slice windows copied into shared memory by asynchronous copies (batches of
  * 8 / 16), 5 / 6 / 7 the variants 4 / 3 / 2 with bulk L2 prefetches of the operator stream
  * a few batches ahead, 8 the tile's halo (positions and the CG vector) staged in shared
  * memory, rows and columns restricted to the nodes without a Dirichlet value of the

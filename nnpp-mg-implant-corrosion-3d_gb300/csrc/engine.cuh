@@ -116,11 +116,11 @@ constexpr int kTrVariants = 2;    // FP32 transport forms (0 L1/L2 gathers, 1 ha
 struct Engine {
   std::vector<Handle*> members;
   int T = 4;                // bins per tile (autotuned)
-  int W = 8;                // lanes per node (autotuned)
+  int W = 8;                // lanes per node of the tile kernels
   bool tuned = false;
   bool eager = false;       // NNPP_EAGER=1: launch kernel by kernel, loops driven by the host
-  int spmv_variant = 0;     // FP32 CG operator: 0, 3 L1/L2 gathers (batches of 16, 0
-                            // pipelined),
+  int spmv_variant = 0;     // FP32 CG operator: 0, 3 L1/L2 gathers (batches of 16, 8; 0 also
+                            // in the one-launch inner solve),
                             // 1 bulk-copy staged, 2, 4 shared-memory windows (8, 16),
                             // 5, 6, 7: 4, 3, 2 with L2 prefetch of the operator stream,
                             // 8 tile halo in shared memory, weights recomputed
