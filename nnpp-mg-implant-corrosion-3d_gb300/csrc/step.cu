@@ -5592,12 +5592,12 @@ bool cg_sweep_applies(const Engine& e, int prec) {
 }
 
 template <typename P, int NW>
-nnpp_status launch_sweep_w(const Engine& e, const EngineView& v, cudaStream_t st) {
+nnpp_status launch_sweep_w(const Engine& e, const EngineView& v, int grid, cudaStream_t st) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(e.sms);
+  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(32 * NW);
   cfg.dynamicSmemBytes = (size_t)cld_max(e) * sizeof(float);
   cfg.stream = st;
@@ -5611,10 +5611,23 @@ nnpp_status launch_sweep_w(const Engine& e, const EngineView& v, cudaStream_t st
 // against 32 (ms a step): 8k nodes 0.251 against 0.322, 64k (1,429 slices) 0.494 against 0.471, 262k
 // 1.40 against 1.27, 2M 24.4 against 18.2.
 constexpr long long kSweepSlices = 152 * 4;
+// CTAs: every SM where the slices are more than the warps of three quarters of them; those three quarters
+// below, and half of the SMs for few slices.  A solve alone gets little or nothing slower and the solves
+// of other handles' threads run beside it.  Measured (ms a step of each handle, 1 / 8 threads): 8k nodes
+// 76 CTAs 0.284 / 0.88, 152 0.294 / 1.63; 22k 76 0.275 / 0.97, 114 0.266 / 1.29; 64k 114 0.396 / 2.48,
+// 152 0.394 / 3.10, 76 0.472 / 2.34.  (As launches that share the SMs: 0.64 / 1.03, 0.61 / 1.14 and
+// 0.76 / 2.54; from 125k nodes on eight threads' solves one after another are 10 to 16% slower than
+// launches were, 9.0 against 8.2 at 262k, one 44% faster.)
+int sweep_grid(int sms, int slices, bool few) {
+  const int part = few ? sms / 2 : sms * 3 / 4;
+  return slices > part * (few ? 16 : 32) ? sms : std::max(1, part);
+}
 nnpp_status launch_cg_sweep_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {
   const bool few = v.ncslices <= kSweepSlices;
-  if (prec == NNPP_MIXED) return few ? launch_sweep_w<float, 16>(e, v, st) : launch_sweep_w<float, 32>(e, v, st);
-  return few ? launch_sweep_w<double, 16>(e, v, st) : launch_sweep_w<double, 32>(e, v, st);
+  const int grid = sweep_grid(e.sms, v.ncslices, few);
+  if (prec == NNPP_MIXED)
+    return few ? launch_sweep_w<float, 16>(e, v, grid, st) : launch_sweep_w<float, 32>(e, v, grid, st);
+  return few ? launch_sweep_w<double, 16>(e, v, grid, st) : launch_sweep_w<double, 32>(e, v, grid, st);
 }
 
 nnpp_status launch_cg_spmv_b(const Engine& e, const EngineView& v, int prec, cudaStream_t st) {
