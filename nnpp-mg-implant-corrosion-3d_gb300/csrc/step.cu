@@ -3466,18 +3466,53 @@ __global__ void __launch_bounds__(kBlock) k_phi4(EngineView v) {
 }
 
 // prep: b, the FP64 residual r = b - A phi and the norms; the mask-only sums (diagonal,
-// Dirichlet coupling, unknown flag) are formed only when the phases changed (op_valid == 0)
-__global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphConditionalHandle hc) {
+// Dirichlet coupling, unknown flag) are formed only when the phases changed (op_valid == 0), by
+// k_prep_masks, for the instances that need them; k_prep_slices serves the others and takes every
+// instance's decision.  (One kernel for both had the mask pass's 128 registers: the usual pass, which
+// only sums phi, took 0.22 ms at 512k nodes, 0.17 and 0.003 for the other's launch alone.)  K warps share
+// a slice where a warp each leaves the chip's warps empty (see SplitSlice); the mask pass, a warp a
+// slice, adds the K parts as they do, so that a step repeated from a restored state gives the same bits.
+
+// a row's b, residual and norms from its sums (mixed path); the slice's partials
+__device__ __forceinline__ void prep_row(const EngineView& v, const KParams& k, int sg, int lane, int a, bool rowok,
+                                         bool fr, double dsum, double cpl, double swphi, double pha) {
+  float b2h = 0.0f, b2l = 0.0f, r2h = 0.0f, r2l = 0.0f;  // b.b and r.r as FP32 pairs
+  if (rowok) {
+    double b;
+    if (k.b_override) {
+      b = k.b_override[a];
+    } else {
+      double R11 = 0.0;
+      for (int s = 0; s < S; ++s) R11 += k.z[s] * conc_of<float>(k, a, s);
+      b = k.lam * R11;
+    }
+    const double bb = fr ? b : 0.0;
+    const double r = fr ? bb - (dsum * pha - swphi) : 0.0;
+    k.b64[a] = bb;
+    k.r64[a] = r;
+    const double be = bb + (fr ? cpl : 0.0);
+    pair_square(be, b2h, b2l);
+    pair_square(r, r2h, r2l);
+  }
+  pair_warp_sum(b2h, b2l);
+  pair_warp_sum(r2h, r2l);
+  if (lane == 0) {
+    store_pair(v.partials, sg, b2h, b2l);
+    store_pair(v.partials, (size_t)v.stride + sg, r2h, r2l);
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_prep_masks(EngineView v) {
   __shared__ int s_hb[kBlock / 32][12];
-  __shared__ double sm[2 * kBlock / 32];
-  __shared__ int s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // warps claim slices one at a time (slices of solid nodes, narrow and partial slices
-  // cost less than full ones)
-  for (int sg = claim_slice(v, lane); sg < v.nslices; sg = claim_slice(v, lane)) {
+  int any = 0;
+  for (int i = threadIdx.x; i < v.M; i += kBlock) any |= v.inst[i].ds->op_valid == 0;
+  if (!__syncthreads_or(any)) return;
+  for (int sg = blockIdx.x * (kBlock / 32) + warp; sg < v.nslices; sg += gridDim.x * (kBlock / 32)) {
     const SliceDesc& d = v.slices[sg];
     const KParams& k = v.inst[d.inst];
-    const bool cached = k.ds->op_valid != 0;
+    if (k.ds->op_valid != 0) continue;
     if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
     __syncwarp();
     const int a = d.row0 + lane;
@@ -3492,12 +3527,12 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
     const int* hb = s_hb[warp];
     const QuadPtr op(sell_w(k, d), lane);
     const float4* wls = reinterpret_cast<const float4*>(sell_lo_col(k, d)) + lane;
-    // sum_j w phi_j over the liquid columns as an FP32 pair in bond order (the cached pass
-    // adds the solid columns' exact zeros, so both passes give the same bits).  The mask
+    // sum_j w phi_j over the liquid columns as an FP32 pair in bond order (k_prep_slices
+    // adds the solid columns' exact zeros, so both give the same bits).  The mask
     // sums also write the row into the CG operator's slices: its bonds to possible unknowns
     // (liquid, no potential Dirichlet value), codes relative to that slice's windows, zero
     // padding, and the slice's longest row.
-    const int cpos = scan && !cached ? k.cg_pos[a] : -1;
+    const int cpos = scan ? k.cg_pos[a] : -1;
     const SliceDesc* cd = nullptr;
     CgRowWriter<float> out;
     int cby = 0, cbz = 0;
@@ -3512,29 +3547,19 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
       cby = cd->tile & 0xffff;
       cbz = cd->tile >> 16;
     }
-    float dh = 0.f, dl = 0.f, sh = 0.f, sl = 0.f, ch = 0.f, cl = 0.f;
+    float dh = 0.f, dl = 0.f, ch = 0.f, cl = 0.f;
+    float ph_[K], pl_[K];  // sum w phi in the K parts of k_prep_slices
+    for (int h = 0; h < K; ++h) ph_[h] = pl_[h] = 0.0f;
     int anyll = 0;
     if (__any_sync(0xffffffffu, scan)) {
       const int width = d.width;
       for (int c0 = 0; c0 < width; c0 += kResB) {
+        const int h = c0 / kResB % K;
+        float sh = ph_[h], sl = pl_[h];
         const int nc = min(kResB, width - c0);  // a multiple of 4
         float w[kResB], wl[kResB];
         unsigned int code[kResB];
         load_residual_quads(op, wls, c0, nc, w, wl, code);
-        if (cached) {
-          float2 f[kResB];
-#pragma unroll
-          for (int u = 0; u < kResB; ++u)
-            if (u < nc) f[u] = __ldg(reinterpret_cast<const float2*>(k.phi4 + code_node(hb, code[u])));
-#pragma unroll
-          for (int u = 0; u < kResB; ++u)
-            if (u < nc) {
-              float ph, pl;
-              pair_mul(w[u], wl[u], f[u].x, f[u].y, ph, pl);
-              pair_add(sh, sl, ph, pl);
-            }
-          continue;
-        }
         float4 f[kResB];
 #pragma unroll
         for (int u = 0; u < kResB; ++u)
@@ -3556,6 +3581,8 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
               out.add(w[u], wl[u], (unsigned int)((r << 12) | (m - cd->gbase[r])));
             }
           }
+        ph_[h] = sh;
+        pl_[h] = sl;
       }
     }
     if (cpos >= 0) {
@@ -3563,50 +3590,89 @@ __global__ void __launch_bounds__(kBlock) k_prep_slices(EngineView v, cudaGraphC
       out.finish(cd->width);
       atomicMax(&k.cg_width[cpos >> 5], out.n);
     }
-    float b2h = 0.0f, b2l = 0.0f, r2h = 0.0f, r2l = 0.0f;  // b.b and r.r as FP32 pairs
+    const bool fr = scan && anyll;
+    const double dsum = (double)dh + (double)dl, cpl = (double)ch + (double)cl;
     if (rowok) {
-      double b;
-      if (k.b_override) {
-        b = k.b_override[a];
-      } else {
-        double R11 = 0.0;
-        for (int s = 0; s < S; ++s) R11 += k.z[s] * conc_of<float>(k, a, s);
-        b = k.lam * R11;
-      }
-      const double pha = (double)fa.x + (double)fa.y;
-      const double swphi = scan ? (double)sh + (double)sl : 0.0;
-      bool fr;
-      double dsum, cpl;
-      if (cached) {
-        fr = k.freem[a] != 0;
-        dsum = k.dsum64[a];
-        cpl = k.cpl64[a];
-      } else {
-        dsum = scan ? (double)dh + (double)dl : 0.0;
-        cpl = scan ? (double)ch + (double)cl : 0.0;
-        fr = scan && anyll;
-        k.freem[a] = fr ? 1 : 0;
-        k.dsum64[a] = fr ? dsum : 1.0;
-        k.cpl64[a] = fr ? cpl : 0.0;
-        k.dinv64[a] = fr ? 1.0 / dsum : 0.0;
-        k.d32[a] = fr ? (float)dsum : 1.0f;
-        k.dinv32[a] = fr ? (float)(1.0 / dsum) : 0.0f;
-      }
-      const double bb = fr ? b : 0.0;
-      const double r = fr ? bb - (dsum * pha - swphi) : 0.0;
-      k.b64[a] = bb;
-      k.r64[a] = r;
-      const double be = bb + (fr ? cpl : 0.0);
-      pair_square(be, b2h, b2l);
-      pair_square(r, r2h, r2l);
+      k.freem[a] = fr ? 1 : 0;
+      k.dsum64[a] = fr ? dsum : 1.0;
+      k.cpl64[a] = fr ? cpl : 0.0;
+      k.dinv64[a] = fr ? 1.0 / dsum : 0.0;
+      k.d32[a] = fr ? (float)dsum : 1.0f;
+      k.dinv32[a] = fr ? (float)(1.0 / dsum) : 0.0f;
     }
-    pair_warp_sum(b2h, b2l);
-    pair_warp_sum(r2h, r2l);
-    if (lane == 0) {
-      store_pair(v.partials, sg, b2h, b2l);
-      store_pair(v.partials, (size_t)v.stride + sg, r2h, r2l);
-    }
+    float sh = ph_[0], sl = pl_[0];
+    for (int h = 1; h < K; ++h) pair_add(sh, sl, ph_[h], pl_[h]);
+    prep_row(v, k, sg, lane, a, rowok, fr, dsum, cpl, (double)sh + (double)sl, (double)fa.x + (double)fa.y);
     __syncwarp();
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kBlock, 4) k_prep_slices(EngineView v, cudaGraphConditionalHandle hc) {
+  __shared__ int s_hb[kBlock / 32][12];
+  __shared__ double sm[2 * kBlock / 32];
+  __shared__ float2 s_part[K > 1 ? kBlock : 1];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % K;
+  // K == 1: warps claim slices one at a time (slices of solid nodes, narrow and partial slices
+  // cost less than full ones)
+  constexpr int kAtOnce = SplitSlice<K>::kSlices;
+  for (int base = K == 1 ? claim_slice(v, lane) : (int)blockIdx.x * kAtOnce; base < v.nslices;
+       base = K == 1 ? claim_slice(v, lane) : base + (int)gridDim.x * kAtOnce) {
+    const int sg = K == 1 ? base : min(base + warp / K, v.nslices - 1);
+    const SliceDesc& d = v.slices[sg];
+    const KParams& k = v.inst[d.inst];
+    // the others are k_prep_masks's
+    const bool mine = (K == 1 || base + warp / K < v.nslices) && k.ds->op_valid != 0;
+    if (K == 1 && !mine) continue;
+    if (lane < 9) s_hb[warp][lane] = d.gbase[lane];
+    __syncwarp();
+    const int a = d.row0 + lane;
+    const bool rowok = mine && lane < d.nrows;
+    const bool fr = rowok && k.freem[a] != 0;
+    const int* hb = s_hb[warp];
+    float sh = 0.f, sl = 0.f;
+    if (__any_sync(0xffffffffu, fr)) {
+      const QuadPtr op(sell_w(k, d), lane);
+      const float4* wls = reinterpret_cast<const float4*>(sell_lo_col(k, d)) + lane;
+      const int width = d.width;
+      for (int c0 = kResB * part; c0 < width; c0 += kResB * K) {
+        const int nc = min(kResB, width - c0);  // a multiple of 4
+        float w[kResB], wl[kResB];
+        unsigned int code[kResB];
+        load_residual_quads(op, wls, c0, nc, w, wl, code);
+        float2 f[kResB];
+#pragma unroll
+        for (int u = 0; u < kResB; ++u)
+          if (u < nc) f[u] = __ldg(reinterpret_cast<const float2*>(k.phi4 + code_node(hb, code[u])));
+#pragma unroll
+        for (int u = 0; u < kResB; ++u)
+          if (u < nc) {
+            float ph, pl;
+            pair_mul(w[u], wl[u], f[u].x, f[u].y, ph, pl);
+            pair_add(sh, sl, ph, pl);
+          }
+      }
+    }
+    if (K > 1) {
+      s_part[threadIdx.x] = make_float2(sh, sl);
+      __syncthreads();
+      if (part == 0)
+#pragma unroll
+        for (int h = 1; h < K; ++h) pair_add(sh, sl, s_part[threadIdx.x + 32 * h].x, s_part[threadIdx.x + 32 * h].y);
+    }
+    double dsum = 1.0, cpl = 0.0, pha = 0.0;
+    if (fr && part == 0) {
+      const float2 fa = __ldg(reinterpret_cast<const float2*>(k.phi4 + a));
+      dsum = k.dsum64[a];
+      cpl = k.cpl64[a];
+      pha = (double)fa.x + (double)fa.y;
+    }
+    if (mine && part == 0) prep_row(v, k, sg, lane, a, rowok, fr, dsum, cpl, (double)sh + (double)sl, pha);
+    if (K > 1)
+      __syncthreads();
+    else
+      __syncwarp();
   }
   if (take_last_ticket(&v.ticket[v.M + 1], &s_last)) {
     for (int i = 0; i < v.M; ++i) {
@@ -5514,7 +5580,14 @@ nnpp_status launch_prep_b(const Engine& e, const EngineView& v, int prec, cudaSt
                           cudaGraphConditionalHandle hc, double* F11_out) {
   if (prec == NNPP_MIXED && !F11_out) {
     k_phi4<float><<<occ_grid(k_phi4<float>, 0, e.sms, v.nchunks), kBlock, 0, st>>>(v);
-    k_prep_slices<<<claim_grid(k_prep_slices, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, hc);
+    dispatch_split(split_warps(e.sms, v.nslices, 8), [&](auto kc) {
+      constexpr int K = decltype(kc)::value;
+      k_prep_masks<K><<<occ_grid(k_prep_masks<K>, 0, e.sms, (v.nslices + 7) / 8), kBlock, 0, st>>>(v);
+      if (K > 1)
+        k_prep_slices<K><<<split_grid<K>(k_prep_slices<K>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, hc);
+      else
+        k_prep_slices<K><<<claim_grid(k_prep_slices<K>, 0, e.sms, v.nslices), kBlock, 0, st>>>(v, hc);
+    });
     NNPP_CUDA(cudaGetLastError());
     return NNPP_OK;
   }
