@@ -635,11 +635,11 @@ def run_ours(args):
     inner = d1["cg_iterations_total"] - d0["cg_iterations_total"]
     outer = d1["outer_iterations_total"] - d0["outer_iterations_total"]
     solves = d1["cg_solves"] - d0["cg_solves"]
-    # per solve: warm-start dots + apply, phi pairs + prep; per step the transport and the next
+    # per solve: warm-start dots + apply, phi pairs, mask sums and prep; per step the transport and the next
     # guess's pass; per outer iteration the refinement and, with the two-level preconditioner and
     # operator 0, the inner solve in one launch, otherwise cg_init, per CG iteration the operator and
     # the update, and with the coarse correction the restriction, the coarse product and z
-    launches = 4 * solves + 2 * outer + 2 * args.steps
+    launches = 5 * solves + 2 * outer + 2 * args.steps
     if not cn or sim.tuning()[2] != 0:
         launches += 2 * inner + ((2 * inner + 3 * outer) if cn else 0)
     # coarse checks (one phase comparison each) and rebuilds (A P, assembly, the direct inverse's
