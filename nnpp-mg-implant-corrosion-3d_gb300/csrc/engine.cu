@@ -1,5 +1,5 @@
 // engine.cu -- batched execution: work lists over one or many instances, the autotuner
-// (bins per tile T, lanes per node W), CUDA-graph capture of the step with device-side loop
+// (bins per tile T, CG operator variant), CUDA-graph capture of the step with device-side loop
 // control (conditional while nodes) and the run loop.
 #include <algorithm>
 #include <cstdlib>

@@ -3,23 +3,23 @@
 // Dirichlet main.cpp:676-712, clamp main.cpp:805-837, phase flip main.cpp:914-922, volume
 // main.cpp:944-949).
 //
-// Work is a list of tiles (bond kernels) or node chunks (vector kernels) over all instances
-// of a batch; each CTA loops over the list (persistent grid).  A tile kernel stages the
-// tile's halo into shared memory and reaches every neighbour through a 16-bit slot, so the
-// per-bond stream is 2 bytes (+ the stored weight where one is used).
+// Work is a list of slices of 32 rows (bond kernels), node chunks (vector kernels) or tiles (the
+// residual entry and the FP64 adjoint) over all instances of a batch; each CTA loops over the list
+// (persistent grid).  A slice streams its rows' bonds in quads of columns, weights and 16-bit codes;
+// a tile kernel stages the tile's halo into shared memory and reaches every neighbour through a
+// 16-bit slot.
 //
 // Precision:
-//   FP64  : FP64 records and stored FP64 weights, FP64 Jacobi-preconditioned CG.
-//   mixed : transport in FP32 with stored FP32 weights (computed in FP64), per-lane FP32
-//           accumulation and a compensated (TwoSum) cross-lane reduction per node;
+//   FP64  : FP64 records and stored FP64 weights, FP64 CG.
+//   mixed : transport in FP32 with stored FP32 weights (computed in FP64);
 //           concentrations kept as compensated FP32 pairs (hi + lo), the saturation test on
-//           hi + lo in FP64; potential: FP64 residual b - A phi (stored FP64 weights) with
-//           FP32 CG corrections whose operator recomputes the weights in FP32 from
-//           tile-relative coordinates.
+//           hi + lo in FP64; potential: residual b - A phi in FP32 pairs (the FP64 weights as
+//           pairs) into FP64, with FP32 CG corrections.
 //
 // Reductions: every work item writes one partial per value; the CTA that completes an
 // instance's last item reduces that instance's partials in item order (deterministic), and
-// the last instance to finish sets the graph's loop condition (any instance still active).
+// the last instance to finish sets the graph's loop condition (any instance still active).  The
+// one-launch inner solve (k_cg_sweep) instead has every CTA sum the CTAs' parts.
 #include <cmath>
 #include <cstring>
 
