@@ -14,6 +14,7 @@
 // dependent pivots each, one CTA a block, the block in registers.
 #include <algorithm>
 
+#include "coarse_index.h"
 #include "coarse_inverse.cuh"
 
 namespace nnpp {
@@ -244,15 +245,15 @@ __global__ void __launch_bounds__(256) k_eliminate(int m, int planes, int s, flo
 //   ODD == 1: j = s (2 u + 1) >= i, from the transposes written by ODD == 0 (+ D_i^-1 for
 //             j = i), and its transpose.
 template <int ODD>
-__global__ void __launch_bounds__(256) k_grow(int m, int planes, int s, const float* d, const float* wl, const float* wr,
-                                              int nj, float* x) {
+__global__ void __launch_bounds__(256) k_grow(int m, int planes, GrowPass pass, const float* d, const float* wl,
+                                              const float* wr, float* x) {
   __shared__ TileSm sm;
-  const int t = (int)blockIdx.z / nj, u = (int)blockIdx.z - t * nj;
-  const int i = s * (2 * t + 1), j = ODD ? s * (2 * u + 1) : 2 * s * u;
+  const GrowPass::Block blk = pass.block((int)blockIdx.x);
+  const int s = pass.s, i = blk.i, j = blk.j;
   if (ODD && j < i) return;
   const size_t mm = (size_t)m * m;
   const size_t n = (size_t)planes * m;
-  const int row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+  const int row0 = blk.row_tile * kTile, col0 = blk.col_tile * kTile;
   float acc[4][4] = {};
   tile_mma<false, false>(sm, wl + i * mm, m, x + (size_t)(i - s) * m * n + (size_t)j * m, (int)n, m, m, m, row0, col0, acc);
   if (i + s < planes)
@@ -332,8 +333,9 @@ nnpp_status coarse_direct_inverse(CoarseBlocks& b, const int na[3], const float*
   k_first_block<<<std::max(1, std::min((m * m + 255) / 256, 152)), 256, 0, st>>>(m, n, b.d.get(), x);
   for (s /= 2; s >= 1; s /= 2) {
     const int odd = (L - 1 - s) / (2 * s) + 1, kept = (L - 1) / (2 * s) + 1;
-    k_grow<0><<<dim3(nt, nt, odd * kept), 256, 0, st>>>(m, L, s, b.d.get(), b.wl.get(), b.wr.get(), kept, x);
-    k_grow<1><<<dim3(nt, nt, odd * odd), 256, 0, st>>>(m, L, s, b.d.get(), b.wl.get(), b.wr.get(), odd, x);
+    const GrowPass even = {s, odd, kept, 0, (int)nt}, odds = {s, odd, odd, 1, (int)nt};
+    k_grow<0><<<(unsigned)even.blocks(), 256, 0, st>>>(m, L, even, b.d.get(), b.wl.get(), b.wr.get(), x);
+    k_grow<1><<<(unsigned)odds.blocks(), 256, 0, st>>>(m, L, odds, b.d.get(), b.wl.get(), b.wr.get(), x);
   }
   k_inverse_out<<<std::min(n, 152 * 8), 256, 0, st>>>(g, n, ld, x, rowabs, b.bad.get(), inv);
   NNPP_CUDA(cudaGetLastError());
