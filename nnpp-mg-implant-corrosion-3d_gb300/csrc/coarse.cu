@@ -82,8 +82,10 @@ __device__ __forceinline__ bool node_liquid(const KParams& k, int i, int mixed) 
   return (mixed ? k.rec32_cur[i].phase : (float)k.rec64_cur[i].phase) == 0.0f;
 }
 
-// What the bond walk needs of a node in one word: its aggregate's place (10 bits an axis), liquid
-// and potential-Dirichlet flags.
+// What the bond walk needs of a node in one word: its aggregate's place (10 bits an axis: build_tiles, which
+// runs before any coarse operator, refuses more than kMaxAxisBins bins an axis), liquid and
+// potential-Dirichlet flags.
+static_assert(kMaxAxisBins <= 1024, "a place's fields are 10 bits an axis");
 constexpr unsigned int kTagLiquid = 1u << 30, kTagDir = 1u << 31;
 __global__ void k_node_tags(KParams k, int mixed, int na0, int na1, unsigned int* tag) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k.N; i += gridDim.x * blockDim.x) {

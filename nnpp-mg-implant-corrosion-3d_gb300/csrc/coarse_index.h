@@ -13,8 +13,8 @@ namespace nnpp {
 
 // The blocks of one pass of the inverse's growth over a level of stride s: plane pairs (i, j),
 // i = s (2 t + 1) for t < rows and j = s (2 u + first) for u < cols, times the tiles x tiles tiles of a
-// plane's block.  They are one list along gridDim.x (2^31 - 1 blocks): a long, thin domain has up to 3000
-// planes and so 1500 x 1500 pairs, and gridDim.z ends at 65535, which 512 planes pass.
+// plane's block.  They are one list along gridDim.x (2^31 - 1 blocks): a long, thin domain has up to 1024
+// planes (kMaxAxisBins) and so 512 x 512 pairs, and gridDim.z ends at 65535, which 512 planes pass.
 struct GrowPass {
   int s, rows, cols, first, tiles;
   struct Block {

@@ -167,7 +167,9 @@ nnpp_status engine_warm(Engine& e, int prec);    // tune, upload parameters, bui
 nnpp_status engine_params(Engine& e);            // re-upload the members' KParams
 void engine_destroy_graphs(Engine& e);
 
-// tiles.cu: tile descriptors, 16-bit halo slots and FP32 position records of one instance
+// tiles.cu: tile descriptors, 16-bit halo slots and FP32 position records of one instance; refuses
+// (NNPP_ERR_UNSUPPORTED) more than kMaxAxisBins bins along an axis
+constexpr int kMaxAxisBins = 1024;
 nnpp_status build_tiles(Handle& h, int T, std::vector<TileDesc>& tiles, std::vector<SliceDesc>& slices,
                         int inst, int* halo_max, int* bond_max, bool* windows_fit);
 // the CG operator's slices of one instance (bin rows' nodes without a potential Dirichlet

@@ -288,7 +288,7 @@ nnpp_status build_tiles(Handle& h, int T, std::vector<TileDesc>& tiles, std::vec
                         int inst, int* halo_max, int* bond_max, bool* windows_fit) {
   const Layout& L = h.lay;
   const int N = h.N;
-  if (L.nb[0] > 1024 || L.nb[1] > 1024 || L.nb[2] > 1024)
+  if (L.nb[0] > kMaxAxisBins || L.nb[1] > kMaxAxisBins || L.nb[2] > kMaxAxisBins)
     return set_error(NNPP_ERR_UNSUPPORTED, "tiles: more than 1024 bins per axis");
   Grid3 g;
   g.nb[0] = L.nb[0];

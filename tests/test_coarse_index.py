@@ -1,5 +1,5 @@
-"""The coarse operator's index arithmetic (csrc/coarse_index.h) at its limits, on the host: an aggregate
-grid has at most 3000 aggregates, so up to 3000 planes along one axis."""
+"""The coarse operator's index arithmetic (csrc/coarse_index.h) at its limits, on the host: up to
+1024 planes of aggregates along one axis (the bins an axis may have), and beyond."""
 import ctypes
 import os
 import subprocess

@@ -69,3 +69,24 @@ def test_more_than_512_planes(gpu, orc, axis):
     shape = [4, 4, 4]
     shape[axis] = 1560
     _solve_and_step(gpu, orc, tuple(shape), 4 * 512)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_1024_bins_along_an_axis(gpu, orc, axis):
+    """3 x 3 x 3086 nodes: 1024 one-bin aggregates on one axis, the most that the lists take (and what the
+    coarse operator's node words hold, 10 bits an axis)."""
+    shape = [3, 3, 3]
+    shape[axis] = 3086
+    _solve_and_step(gpu, orc, tuple(shape), 1024)
+
+
+def test_more_bins_are_refused(gpu):
+    """3 x 3 x 3100 nodes: 1028 bins on one axis are an error before any coarse operator is formed."""
+    nn = gpu
+    for axis in range(3):
+        shape = [3, 3, 3]
+        shape[axis] = 3100
+        sim = nn.Simulation(*_wire(nn, tuple(shape)))
+        with pytest.raises(nn.NNPPError) as e:
+            sim.build_neighbours()
+        assert e.value.status == 6
