@@ -675,48 +675,56 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
     NNPP_TRY(scan_ints(st, count.get(), start.get(), max_hash, nullptr));
   }
   // Step 5 (grid.h:143-196): count, then fill
-  DBuf<int> len, err;
-  if (!len.alloc(N) || !err.alloc(1) || !out.ptr.alloc(N + 1))
-    return set_error(NNPP_ERR_NOMEM, "scan buffers");
-  NNPP_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
-  const int warps_grid = grid_for((long long)N * 32, 256, 152 * 64);
+  DBuf<int> len, err, dml;
   DBuf<ScanNode> nodes;
-  if (!nodes.alloc(N)) return set_error(NNPP_ERR_NOMEM, "scan buffers");
+  if (!len.alloc(N) || !err.alloc(1) || !dml.alloc(1) || !out.ptr.alloc(N + 1) || !nodes.alloc(N))
+    return set_error(NNPP_ERR_NOMEM, "scan buffers");
+  const int warps_grid = grid_for((long long)N * 32, 256, 152 * 64);
   k_scan_nodes<<<grid_for(N, 256), 256, 0, st>>>(N, order.get(), hash.get(), x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
                                                  1.0 / r, nodes.get());
   const float eps = scan_eps(r, cx, cy, cz);
-  // one scan into rows of max_node_no - 1 columns where those are a few bytes more than the lists (up to
-  // 2 GB), packed after; two scans, the lengths first, otherwise
-  const long long cap = max_node_no - 1;
-  DBuf<int> rows;
-  const bool both = cap > 0 && cap * N <= kScanRowsMax && rows.alloc((size_t)(cap * N));
   auto scan = [&](auto mode, int* cols) {
     k_cell_scan<decltype(mode)::value><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my, max_hash, r,
                                                                   eps, start.get(), nodes.get(), max_node_no, len.get(),
                                                                   out.ptr.get(), cols, err.get());
   };
-  if (both)
-    scan(std::integral_constant<int, kScanBoth>(), rows.get());
-  else
-    scan(std::integral_constant<int, kScanCount>(), nullptr);
-  NNPP_CUDA(cudaGetLastError());
-  int herr = 0;
-  NNPP_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
-  NNPP_CUDA(cudaStreamSynchronize(st));
-  if (herr)
-    return set_error(NNPP_ERR_CAPACITY, "Not enough room to store clouds. Increase max_node_no.");
+  // one scan into rows of max_node_no - 1 columns where those are a few bytes more than the lists (up to
+  // 2 GB), packed after; two scans, the lengths first, otherwise and where the memory does not hold rows and
+  // lists at once
+  const long long cap = max_node_no - 1;
   long long nnz = 0;
-  NNPP_TRY(scan_ints(st, len.get(), out.ptr.get(), N, &nnz));
-  if (nnz < 0 || nnz > (long long)INT_MAX)
-    return set_error(NNPP_ERR_UNSUPPORTED, "build: more than 2^31-1 bonds");
-  if (!out.col.alloc(nnz > 0 ? nnz : 1)) return set_error(NNPP_ERR_NOMEM, "neighbour columns");
-  if (both)
-    k_pack_rows<<<warps_grid, 256, 0, st>>>(N, (int)cap, out.ptr.get(), rows.get(), out.col.get());
-  else
-    scan(std::integral_constant<int, kScanFill>(), out.col.get());
-  NNPP_CUDA(cudaGetLastError());
-  DBuf<int> dml;
-  if (!dml.alloc(1)) return set_error(NNPP_ERR_NOMEM, "max length");
+  auto lists = [&](int* rows) -> nnpp_status {
+    NNPP_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
+    if (rows)
+      scan(std::integral_constant<int, kScanBoth>(), rows);
+    else
+      scan(std::integral_constant<int, kScanCount>(), nullptr);
+    NNPP_CUDA(cudaGetLastError());
+    int herr = 0;
+    NNPP_CUDA(cudaMemcpyAsync(&herr, err.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+    NNPP_CUDA(cudaStreamSynchronize(st));
+    if (herr)
+      return set_error(NNPP_ERR_CAPACITY, "Not enough room to store clouds. Increase max_node_no.");
+    NNPP_TRY(scan_ints(st, len.get(), out.ptr.get(), N, &nnz));
+    if (nnz < 0 || nnz > (long long)INT_MAX)
+      return set_error(NNPP_ERR_UNSUPPORTED, "build: more than 2^31-1 bonds");
+    if (!out.col.alloc(nnz > 0 ? nnz : 1)) return set_error(NNPP_ERR_NOMEM, "neighbour columns");
+    if (rows)
+      k_pack_rows<<<warps_grid, 256, 0, st>>>(N, (int)cap, out.ptr.get(), rows, out.col.get());
+    else
+      scan(std::integral_constant<int, kScanFill>(), out.col.get());
+    NNPP_CUDA(cudaGetLastError());
+    return NNPP_OK;
+  };
+  DBuf<int> rows;
+  const bool both = cap > 0 && cap * N <= kScanRowsMax && rows.alloc((size_t)(cap * N));
+  nnpp_status res = lists(both ? rows.get() : nullptr);
+  if (both && res == NNPP_ERR_NOMEM) {
+    rows.reset();
+    clear_error();
+    res = lists(nullptr);
+  }
+  NNPP_TRY(res);
   NNPP_CUDA(cudaMemsetAsync(dml.get(), 0, sizeof(int), st));
   k_max_int<<<grid_for(N, 256), 256, 0, st>>>(len.get(), N, dml.get());
   int ml = 0;

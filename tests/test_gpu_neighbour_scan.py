@@ -62,3 +62,28 @@ def test_one_scan_and_two_scans_agree(gpu, N):
         out.append(sim.neighbours_csr())
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
+
+
+def test_build_where_rows_and_lists_do_not_fit_together(gpu):
+    """103,823 nodes of up to 4,168 neighbours with 2.8 GB of device memory left: the one-scan build's rows
+    take 2.08 GB and the lists 1.4, so the rows are given back and the two-scan build runs.  (The test's
+    own allocation is what fills the device.)"""
+    nn = gpu
+    torch = pytest.importorskip("torch")
+    n, most = 47, 5001
+    g = np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij")).reshape(3, -1).astype(np.float64)
+    args = (most, 10.0, 10.0, 10.0, 10.0, np.ascontiguousarray(g))
+    _, expect, ml = nn.build_clouds_hash(*args, want_clouds=False)
+    bonds = int(expect.sum()) - expect.size
+    rows = 4 * (most - 1) * g.shape[1]
+    left = int(2.8e9)
+    assert rows < left < rows + 4 * bonds - 200e6 and 4 * bonds < left - 500e6
+    torch.cuda.synchronize()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+    try:
+        _, lengths, ml2 = nn.build_clouds_hash(*args, want_clouds=False)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert ml2 == ml
+    assert np.array_equal(lengths, expect)
