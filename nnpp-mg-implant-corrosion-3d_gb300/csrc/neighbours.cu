@@ -248,9 +248,10 @@ __global__ void k_scan_nodes(int n, const int* __restrict__ order, const int* __
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const int i = order[k], m = hash[i];
     ScanNode v;
-    v.x = (float)((x[i] - (x0 + (double)(m % mx) * cx)) * inv_r);
-    v.y = (float)((y[i] - (y0 + (double)((m / mx) % my) * cy)) * inv_r);
-    v.z = (float)((z[i] - (z0 + (double)(m / mx / my) * cz)) * inv_r);
+    // the corners rounded as the scan rounds them (far from the origin a contracted sum is another corner)
+    v.x = (float)((x[i] - __dadd_rn(x0, __dmul_rn((double)(m % mx), cx))) * inv_r);
+    v.y = (float)((y[i] - __dadd_rn(y0, __dmul_rn((double)((m / mx) % my), cy))) * inv_r);
+    v.z = (float)((z[i] - __dadd_rn(z0, __dmul_rn((double)(m / mx / my), cz))) * inv_r);
     v.id = i;
     out[k] = v;
   }
@@ -571,12 +572,18 @@ nnpp_status check_hash_grid(const double bb[6], double cx, double cy, double cz,
 // Bound of the error of k_cell_scan's squared distances (units of r) near 1.  With cells of c
 // radii, the node's position relative to a visited cell's corner is at most 1 + 3 c, a
 // candidate's at most c, their difference is rounded once more: each coordinate is off by less
-// than u (3 + 7 c), u = 2^-24; 2 sqrt(3) of that, its square and the square sum's own three
-// roundings bound the squared distance's error (with a factor of about two to spare).  Large
-// cells make it exceed 1: every test is then the FP64 one.
-float scan_eps(double r, double cx, double cy, double cz) {
-  const double c = std::max(cx, std::max(cy, cz)) / r;
-  const double u = 1.0 / 16777216.0, d = u * (4.0 + 14.0 * c);
+// than u (3 + 7 c), u = 2^-24.  Corners, rounded alike in both kernels, cancel from differences of
+// positions, but a cell's far face is rounded once more, by up to 2 v m for coordinates of up to m
+// radii, v = 2^-53, which far from the origin is the larger part (taken as 8 v m).  2 sqrt(3) of that,
+// its square and the square sum's own three roundings bound the squared distance's error (with a factor
+// of about two to spare on the first part).  Large cells or coordinates make it exceed 1: every test is
+// then the FP64 one.
+float scan_eps(double r, double cx, double cy, double cz, const double bb[6]) {
+  const double w = std::max(cx, std::max(cy, cz)), c = w / r;
+  double m = 0.0;
+  for (int q = 0; q < 6; ++q) m = std::max(m, std::fabs(bb[q]));
+  m = (m + w) / r;
+  const double u = 1.0 / 16777216.0, v = u * u / 32.0, d = u * (4.0 + 14.0 * c) + 8.0 * v * m;
   return (float)std::min(1e6, 4.0 * d + 4.0 * d * d + 16.0 * u);
 }
 
@@ -682,7 +689,7 @@ nnpp_status build_ref_lists(cudaStream_t st, int N, const double* x, const doubl
   const int warps_grid = grid_for((long long)N * 32, 256, 152 * 64);
   k_scan_nodes<<<grid_for(N, 256), 256, 0, st>>>(N, order.get(), hash.get(), x, y, z, x0, y0, z0, cx, cy, cz, mx, my,
                                                  1.0 / r, nodes.get());
-  const float eps = scan_eps(r, cx, cy, cz);
+  const float eps = scan_eps(r, cx, cy, cz, out.bbox);
   auto scan = [&](auto mode, int* cols) {
     k_cell_scan<decltype(mode)::value><<<warps_grid, 256, 0, st>>>(N, x, y, z, x0, y0, z0, cx, cy, cz, mx, my, max_hash, r,
                                                                   eps, start.get(), nodes.get(), max_node_no, len.get(),

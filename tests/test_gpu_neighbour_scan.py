@@ -47,6 +47,24 @@ def test_scan_ties_and_cells(gpu, orc, shape, r_cells, cell_factor):
     assert np.array_equal(clouds, expect)
 
 
+@pytest.mark.parametrize("offset", [0.0, 2.0 ** 20, 2.0 ** 38])
+def test_scan_far_from_the_origin(gpu, orc, offset):
+    """Ties on a lattice far from the origin (every coordinate exact).  The cell side is chosen so that at
+    2^38 three sides in FP64 lie halfway between two coordinates: the fourth column's corner then differs
+    by a coordinate's last place, 1.6e-4 radii, with the product rounded or not."""
+    nn = gpu
+    dx = 0.125
+    side = float.fromhex("0x1.a2d2aaaaaaaaap-2")
+    g = np.stack(np.meshgrid(*[np.arange(n) for n in (11, 10, 9)], indexing="ij")).reshape(3, -1).astype(np.float64) * dx
+    g = np.ascontiguousarray(g[:, np.random.default_rng(4).permutation(g.shape[1])] + offset)
+    cell = (side, 4.1 * dx, 3.28 * dx)
+    clouds, lengths, ml = nn.build_clouds_hash(1024, 3.0 * dx, *cell, g)
+    ml_o, len_o, expect = _oracle_lists(nn, orc, g, 3.0 * dx, cell)
+    assert ml == ml_o
+    assert np.array_equal(lengths, len_o)
+    assert np.array_equal(clouds, expect)
+
+
 @pytest.mark.parametrize("N", [1, 33, 1000])
 def test_one_scan_and_two_scans_agree(gpu, N):
     """The one-scan build (rows of max_node_no - 1 columns, packed) against the two-scan build that a
