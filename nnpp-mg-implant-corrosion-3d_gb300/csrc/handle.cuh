@@ -250,7 +250,7 @@ struct Handle {
   const double* b_override = nullptr;  // set during adjoint solves
   int grid = 0;                 // CTAs of the per-handle elementwise kernels
   Engine* engine = nullptr;     // single-instance engine (owned)
-  std::shared_ptr<void> implicit_work;  // nnpp_forward_implicit's buffers for these lists
+  std::shared_ptr<void> implicit_work;  // nnpp_forward_implicit's buffers for these lists (see implicit.cu)
   // adjoint checkpoints: the full device state at a step
   struct Ckpt {
     DBuf<Rec32> rec32;

@@ -780,7 +780,7 @@ nnpp_status apply(cudaStream_t st, const ImpCtxT<NS>& c, const double* v, double
 
 // build_slices: asynchronous on st but for one read of the slot count
 nnpp_status build_slices(cudaStream_t st, int N, const int* ptr, const int* col, const double* x, const double* y,
-                         const double* z, double delta, double dx, double dV, int nf, Sliced& sl) {
+                         const double* z, double delta, double dx, double dV, Sliced& sl) {
   sl.n = (N + 31) / 32;
   DBuf<int> width;
   if (!width.alloc(sl.n) || !sl.off.alloc(sl.n + 1)) return set_error(NNPP_ERR_NOMEM, "implicit step: slices");
@@ -789,11 +789,18 @@ nnpp_status build_slices(cudaStream_t st, int N, const int* ptr, const int* col,
   long long cols = 0;
   NNPP_TRY(scan_ints(st, width.get(), sl.off.get(), sl.n, &cols));
   sl.slots = 32 * std::max<long long>(cols, 1);
-  if (!sl.col.alloc(sl.slots) || !sl.w.alloc(sl.slots) || !sl.toff.alloc((size_t)nf * sl.slots))
+  if (!sl.col.alloc(sl.slots) || !sl.w.alloc(sl.slots))
     return set_error(NNPP_ERR_NOMEM, "implicit step: slices");
   k_imp_weights<<<grid_for((long long)sl.n * 32, kTB), kTB, 0, st>>>(N, ptr, col, x, y, z, delta, dx, dV, sl.n,
                                                                      sl.off.get(), sl.col.get(), sl.w.get());
   NNPP_CUDA(cudaGetLastError());
+  return NNPP_OK;
+}
+
+// the arrays that only a step needs, the largest: the Arnoldi basis and the off-diagonals of nf fields
+nnpp_status alloc_step(Work& wk, int nf) {
+  if (!wk.V.alloc((size_t)(kRestart + 1) * nf * wk.N) || !wk.sl.toff.alloc((size_t)nf * wk.sl.slots))
+    return set_error(NNPP_ERR_NOMEM, "implicit step: Arnoldi basis and off-diagonals");
   return NNPP_OK;
 }
 
@@ -891,6 +898,12 @@ __global__ void k_imp_negate(size_t n, const double* a, double* b) {
 
 }  // namespace
 
+// Bytes of a step's arrays (alloc_step) up to which nnpp_forward_implicit leaves them with the handle for
+// its next call; larger ones (from some 85,000 nodes on; 3 GB at 512,000) are freed on return, since other
+// runs and handles need the memory, and allocating them again is little of a step that long: 125k nodes
+// 30.2 ms a call of one step against 29.5 with the arrays kept, 512k 136.0 against 134.1.
+constexpr size_t kKeepStepBytes = (size_t)512 << 20;
+
 // the four-species step's buffers
 static nnpp_status make_work(Handle& h, Work& wk) {
   const nnpp_params& p = h.p;
@@ -900,12 +913,12 @@ static nnpp_status make_work(Handle& h, Work& wk) {
   wk.N = N;
   if (!wk.u0.alloc(FN) || !wk.u1.alloc(FN) || !wk.F.alloc(FN) ||
       !wk.b.alloc(FN) || !wk.x.alloc(FN) || !wk.t.alloc(FN) || !wk.diag.alloc(FN) ||
-      !wk.V.alloc((size_t)(kRestart + 1) * FN) || !wk.part.alloc((size_t)kDotBlocks * (kRestart + 1) * F5) ||
+      !wk.part.alloc((size_t)kDotBlocks * (kRestart + 1) * F5) ||
       !wk.red.alloc(F5) || !wk.gm.alloc(1) || !wk.dir.alloc(FN) || !wk.bc.alloc(FN) || !wk.phase.alloc(N))
     return set_error(NNPP_ERR_NOMEM, "forward_implicit buffers");
   NNPP_CUDA(cudaMemsetAsync(wk.gm.get(), 0, sizeof(GmState), st));
   NNPP_TRY(build_slices(st, N, h.ref.ptr.get(), h.ref.col.get(), h.ux.get(), h.uy.get(), h.uz.get(), p.delta, p.dx,
-                        p.dx * p.dy * p.dz, F5, wk.sl));
+                        p.dx * p.dy * p.dz, wk.sl));
   // Dirichlet flags and values in the reference's order (main.cpp:676-712)
   std::vector<unsigned char> dir(FN, 0);
   std::vector<double> bc(FN, 0.0);
@@ -937,14 +950,23 @@ extern "C" nnpp_status nnpp_forward_implicit(nnpp_handle* hp, int n_steps, int64
   const int N = h.N;
   const size_t FN = (size_t)F5 * N;
   cudaStream_t st = h.st;
-  // buffers, sliced rows with their weights and Dirichlet values (the reference's node order): made by
-  // the first call, kept by the handle until its lists are rebuilt
+  // vectors, sliced rows with their weights and Dirichlet values (the reference's node order): made by
+  // the first call, kept by the handle until its lists are rebuilt; a step's arrays as kKeepStepBytes says
   if (!h.implicit_work) {
     auto made = std::make_shared<Work>();
     NNPP_TRY(make_work(h, *made));
     h.implicit_work = made;
   }
   Work& wk = *std::static_pointer_cast<Work>(h.implicit_work);
+  struct StepArrays {
+    Work& wk;
+    ~StepArrays() {
+      if (wk.V.bytes() + wk.sl.toff.bytes() <= kKeepStepBytes) return;
+      wk.V.reset();
+      wk.sl.toff.reset();
+    }
+  } step_arrays{wk};
+  NNPP_TRY(alloc_step(wk, F5));
   // the handle's state (FP64, user order)
   NNPP_TRY(store_state(h, wk.u0.get(), wk.u0.get() + (size_t)S * N, wk.phase.get()));
   DevState ds;
@@ -1135,7 +1157,7 @@ extern "C" nnpp_status nnpp_chem_create(nnpp_chem** out, int n_nodes, const doub
   ok = ok && c->xyz.alloc(3 * (size_t)N) && c->ptr.alloc(N + 1) &&
        dcol.alloc(col.size()) && c->hz.alloc((size_t)ml * N) && c->hl.alloc(N) && wk.u0.alloc(FN) &&
        wk.u1.alloc(FN) && wk.F.alloc(FN) && wk.b.alloc(FN) && wk.x.alloc(FN) && wk.t.alloc(FN) &&
-       wk.diag.alloc(FN) && wk.V.alloc((size_t)(kRestart + 1) * FN) &&
+       wk.diag.alloc(FN) &&
        wk.part.alloc((size_t)kDotBlocks * (kRestart + 1) * kChemNF) && wk.red.alloc(kChemNF) && wk.gm.alloc(1) &&
        wk.dir.alloc(FN) && wk.bc.alloc(FN) && wk.phase.alloc(N);
   if (!ok) {
@@ -1172,7 +1194,8 @@ extern "C" nnpp_status nnpp_chem_create(nnpp_chem** out, int n_nodes, const doub
   if (rs == NNPP_OK) {
     const double dx = data2[3], dy = data2[4], dz = data2[5], delta = data2[6];
     rs = build_slices(st, N, c->ptr.get(), dcol.get(), c->xyz.get(), c->xyz.get() + N, c->xyz.get() + 2 * (size_t)N,
-                      delta, dx, dx * dy * dz, kChemNF, wk.sl);
+                      delta, dx, dx * dy * dz, wk.sl);
+    if (rs == NNPP_OK) rs = alloc_step(wk, kChemNF);
     if (rs == NNPP_OK && cudaStreamSynchronize(st) != cudaSuccess) rs = set_error(NNPP_ERR_CUDA, "chem_create: weights");
   }
   if (rs != NNPP_OK) {
