@@ -896,7 +896,7 @@ nnpp_status nnpp_set_tuning(nnpp_handle* hp, int bins_per_tile, int lanes_per_no
                      "tile halo and code block within a CTA's shared memory");
   e.W = W;
   e.spmv_variant = cg_operator;
-  e.tuned = true;
+  e.tuned = e.pinned = true;
   NNPP_TRY(engine_params(e));
   return NNPP_OK;
 }

@@ -399,6 +399,12 @@ nnpp_status prepare_run(Engine& e, int prec) {
       if (h.st != e.st) NNPP_CUDA(cudaStreamSynchronize(h.st));  // built on the member's stream
     }
   }
+  // a handle tuned under the diagonal preconditioner: the one-launch solve has operator 0 (512k nodes 2.33 ms
+  // a step, 2.71 as launches)
+  if (engine_coarse(e) && e.members.size() == 1 && !e.pinned && e.spmv_variant != 0) {
+    e.spmv_variant = 0;
+    engine_destroy_graphs(e);
+  }
   const bool split = engine_coarse(e);
   if (split != e.coarse_graphs) {
     engine_destroy_graphs(e);

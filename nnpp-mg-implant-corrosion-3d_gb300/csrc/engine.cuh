@@ -118,6 +118,7 @@ struct Engine {
   int T = 4;                // bins per tile (autotuned)
   int W = 8;                // lanes per node of the tile kernels
   bool tuned = false;
+  bool pinned = false;      // by nnpp_set_tuning, which the engine does not change
   bool eager = false;       // NNPP_EAGER=1: launch kernel by kernel, loops driven by the host
   int spmv_variant = 0;     // FP32 CG operator: 0, 3 L1/L2 gathers (batches of 16, 8; 0 also
                             // in the one-launch inner solve),
