@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(128) k_residuals_grouped(ChemParams c, int N, 
           t[kSp] = fma(w, sub(Un1[(size_t)kSp * N + n], phi1_i), t[kSp]);
           t[kSp + 1] = add(t[kSp + 1], v);
         } else {
-          const int cls = pi != 0 && pn != 0 ? 1 : 0;
+          const int cls = pi == 1 && pn == 1 ? 1 : 0;  // any other value: mixed, as in k_residuals_full
 #pragma unroll
           for (int k = 0; k < kSp; ++k) {
             if (k > 0 && cls) continue;  // solid-solid bonds carry only Mg

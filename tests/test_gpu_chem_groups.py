@@ -42,3 +42,24 @@ def test_grouped_residual_sizes(gpu, orc, n, N, ratio):
     for k in range(11):
         assert np.abs(F[k] - Fr[k]).max() <= 1e-12 * np.abs(Fr[k]).max(), k
     assert np.array_equal(F[10] == 0.0, Fr[10] == 0.0)
+
+
+@pytest.mark.parametrize("n", [12, 62])
+def test_grouped_residual_phases_other_than_solid_and_liquid(gpu, orc, n):
+    """The reference tests phases for 1 and for 0: a bond of any other value is neither solid-solid nor
+    liquid-liquid.  Both forms of the grouped kernel."""
+    nn = gpu
+    g = np.load(GOLDEN)
+    d2, dc, d11 = chem_case.reactive_data2(g["data2"]), g["datac"], g["datac11"]
+    nodes, phase, Un1, Un, r, cell = chem_case.case_inputs(nn.synth, 1, n, 4, g["data2"])
+    N = nodes.shape[1]
+    phase = phase.copy()
+    phase[np.random.default_rng(2).permutation(N)[:N // 4]] = 2
+    clouds, lengths, ml = nn.build_clouds_hash(160, r, cell, cell, cell, nodes)
+    F = nn.residuals_full(nodes, clouds[:, :ml], lengths, Un1, Un, phase, chem_case.VOLN1REL, d2, dc, d11)
+    ptr = np.zeros(N + 1, dtype=np.int64)
+    ptr[1:] = np.cumsum(lengths)
+    cols = clouds[:, :ml][np.arange(ml)[None, :] < lengths[:, None]].astype(np.int32)
+    Fr = orc.residuals_full(nodes, ptr, cols, Un1, Un, phase, chem_case.VOLN1REL, d2, dc, d11)
+    for k in range(11):
+        assert np.abs(F[k] - Fr[k]).max() <= 1e-12 * np.abs(Fr[k]).max(), k
