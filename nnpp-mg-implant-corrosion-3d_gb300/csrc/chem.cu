@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "dbuf.cuh"
+#include "fp64_steps.cuh"
 
 namespace nnpp {
 namespace {
@@ -100,14 +101,9 @@ __device__ __forceinline__ double rpow(double rs, double xi, double e, int ie) {
   return dvd(1.0, pow(xi, e));
 }
 
-// a / dt: the quotient from the reciprocal and one correction by its remainder (three FP64
-// instructions against the two dozen of a division; the correction leaves it within a rounding
-// of the quotient), the division itself where dt's reciprocal is out of range
+// a / dt: three FP64 instructions, the division itself where dt's reciprocal is out of range
 __device__ __forceinline__ double over_dt(double a, const ChemParams& c) {
-  if (c.rdt == 0.0) return dvd(a, c.dt);
-  const double q = mul(a, c.rdt);
-  if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;  // infinite or NaN: no remainder
-  return fma(fma(-q, c.dt, a), c.rdt, q);
+  return c.rdt == 0.0 ? dvd(a, c.dt) : div_corrected(a, c.dt, c.rdt);
 }
 
 // The fields of node i from its bond sums (sums[k] = sum_KRk1 + sum_KRk2, s11 the potential's): the
@@ -282,21 +278,6 @@ __global__ void k_residuals_full(ChemParams c, int N, const double* __restrict__
     for (int k = 0; k < kSp; ++k) sums[k] = -add(mul(c.sg1[k], S1[k]), mul(c.sg2[k], S2[k]));
     finish_node(c, N, i, pi, iface != 0, flag != 0, sums, -mul(c.KS11, S11), Un1, Un, F);
   }
-}
-
-// 1 / sqrt(x) from a single-precision start y0 (22 bits) and Householder's third-order step
-// y0 + y0 e (1/2 + 3/8 e), e = 1 - x y0^2: the error falls to e^3 and stays at the FP64 rounding.
-// The conversions move bits, so that only the step's five operations use the FP64 pipe; values
-// that FP32 does not hold take CUDA's rsqrt.
-__device__ __forceinline__ double rsqrt_step(double x) {
-  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
-  const unsigned int ex = hi >> 20;  // the sign is clear
-  if (ex < 1023u - 100u || ex > 1023u + 100u) return rsqrt(x);
-  const float f = __uint_as_float(((ex - 1023u + 127u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
-  const unsigned int g = __float_as_uint(rsqrtf(f));
-  const double y = __hiloint2double((int)((((g >> 23) - 127u + 1023u) << 20) | ((g & 0x7fffffu) >> 3)), (int)(g << 29));
-  const double e = fma(-mul(x, y), y, 1.0);
-  return fma(mul(e, fma(e, 0.375, 0.5)), y, y);
 }
 
 // The residual for s = 0 and liquid diffusivities that are not zero, charges in the model's groups

@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "engine.cuh"
+#include "fp64_steps.cuh"
 #include "tma.cuh"
 
 namespace nnpp {
@@ -2275,19 +2276,6 @@ __device__ __forceinline__ void sweep_store(double* p, const SweepSum<P>& x) {
     __stcg(p, __longlong_as_double((long long)((unsigned long long)(unsigned)__float_as_int(x.lo) << 32 |
                                                (unsigned)__float_as_int(x.hi))));
 }
-// a / b by Newton steps on the reciprocal of b's significand (half of the compiler's FP64 instructions)
-__device__ __forceinline__ double sweep_div(double a, double b) {
-  const long long bits = __double_as_longlong(b);
-  const int ex = (int)(bits >> 52) & 0x7ff;
-  if (ex == 0 || ex >= 0x7fe) return a / b;
-  const double m = __longlong_as_double((bits & (long long)0x800fffffffffffffull) | 0x3ff0000000000000ll);
-  double x = (double)(1.0f / (float)m);
-  x = fma(x, fma(-m, x, 1.0), x);
-  x = fma(x, fma(-m, x, 1.0), x);
-  double q = a * x;
-  q = fma(fma(-m, q, a), x, q);
-  return q * __longlong_as_double((long long)(2046 - ex) << 52);
-}
 // comparisons by the bits (an FP64 comparison takes the FP64 pipe)
 __device__ __forceinline__ bool sweep_finite(double x) {
   return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
@@ -2971,7 +2959,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
   }
   while (ok && sm.st.go) {
     const SweepSum<P> pq = apply(sm.st.beta_p);
-    auto inverse = [&] { sm.st.irz = sweep_div(1.0, sm.st.rz); };  // next()'s division, ahead
+    auto inverse = [&] { sm.st.irz = div_newton(1.0, sm.st.rz); };  // next()'s division, ahead
     if (def) {
       if constexpr (sizeof(P) == 4) {
         const SweepSum<P> no[1] = {};
@@ -2983,7 +2971,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
           SweepState<P>& s = sm.st;  // p.P_d A p = p.q - r_c.x_c
           s.pq = tot[0];
           const double pw = tot[0] - tot[1];
-          s.alpha = (sweep_positive(tot[0]) && sweep_positive(pw) && sweep_finite(pw)) ? sweep_div(s.rz, pw) : 0.0;
+          s.alpha = (sweep_positive(tot[0]) && sweep_positive(pw) && sweep_finite(pw)) ? div_newton(s.rz, pw) : 0.0;
           s.alpha_p = (P)s.alpha;
         }, idle);
         if (!ok) break;
@@ -2996,7 +2984,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_cg_sweep(EngineView v) {
       ok = sweep_meet<1, NW, P>(v, sm, target, half, d, [&](const double* tot) {
         SweepState<P>& s = sm.st;
         s.pq = tot[0];
-        s.alpha = (sweep_positive(tot[0]) && sweep_finite(tot[0])) ? sweep_div(s.rz, tot[0]) : 0.0;
+        s.alpha = (sweep_positive(tot[0]) && sweep_finite(tot[0])) ? div_newton(s.rz, tot[0]) : 0.0;
         s.alpha_p = (P)s.alpha;
       }, inverse);
       if (!ok) break;
@@ -3059,22 +3047,6 @@ __device__ __forceinline__ int warm_history(const KParams& k) {
   if (k.hist_m < 3 || !k.extrapolate) return 0;
   const int n = k.ds->hist_n;
   return n < k.hist_m ? n : k.hist_m;
-}
-
-// 1 / sqrt(x), x > 0: two Newton steps from the FP32 root of x scaled by a power of four into [1, 4)
-__device__ __forceinline__ double rsqrt_newton(double x) {
-  const long long bits = __double_as_longlong(x);
-  const int ex = (int)(bits >> 52);
-  if (ex == 0 || ex >= 0x7ff) return 1.0 / sqrt(x);
-  const int odd = (ex + 1) & 1;  // x = m 2^(ex - 1023 - odd), an even power
-  const double m = __longlong_as_double((bits & 0x000fffffffffffffll) | (long long)(1023 + odd) << 52);
-  double y = (double)rsqrtf((float)m);
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double r = fma(-m * y, y, 1.0);
-    y = fma(0.5 * y, r, y);
-  }
-  return y * __longlong_as_double((long long)(1023 - (ex - 1023 - odd) / 2) << 52);
 }
 
 // Solve the scaled Galerkin system by Cholesky; differences whose pivot falls below 1e-12
