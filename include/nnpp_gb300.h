@@ -285,10 +285,10 @@ nnpp_status nnpp_forward(nnpp_handle* h, int n_steps, int precision);
  * together on the GPU (one pass over the bonds serves all five).  newton_iterations and
  * krylov_iterations (GMRES iterations summed over fields and steps) may be NULL.  The state,
  * flip steps and diagnostics continue as after nnpp_forward; the step is the reference's, so
- * it is stable at time steps far above the explicit limit.  Between calls the handle keeps, until its lists
- * are rebuilt or it is destroyed, 330 bytes of device memory a node and 12 a bond (rows padded to the longest of 32)
- * and, while they take no more than 512 MB together, the Arnoldi basis (1,240 bytes a node) and the tangents'
- * off-diagonals (40 a bond). */
+ * it is stable at time steps far above the explicit limit.  Between calls the handle keeps,
+ * until its lists are rebuilt or it is destroyed, 330 bytes of device memory a node and 12 a
+ * bond (rows padded to the longest of 32) and, while they take no more than 512 MB together,
+ * the Arnoldi basis (1,240 bytes a node) and the tangents' off-diagonals (40 a bond). */
 nnpp_status nnpp_forward_implicit(nnpp_handle* h, int n_steps, int64_t* newton_iterations,
                                   int64_t* krylov_iterations);
 
@@ -416,9 +416,10 @@ nnpp_status nnpp_time_kernel(nnpp_handle* h, int kernel_id, int precision, int r
  * residual entry points' tile kernels, and the FP32 CG operator's variant: 0 / 3 gathers from
  * L1/L2 (batches of 16 / 8 bond columns, the next batch in flight; a single instance with the
  * two-level preconditioner runs its whole inner solve with 0 in one launch), 1 operator and
- * slice windows streamed by bulk copies into shared memory, 2 / 4 slice windows copied into shared memory by asynchronous copies (batches of
- * 8 / 16), 5 / 6 / 7 the variants 4 / 3 / 2 with bulk L2 prefetches of the operator stream
- * a few batches ahead, 8 the tile's halo (positions and the CG vector) staged in shared
+ * slice windows streamed by bulk copies into shared memory, 2 / 4 slice windows copied into
+ * shared memory by asynchronous copies (batches of 8 / 16), 5 / 6 / 7 variant 4, gathers in
+ * batches of 16 and variant 2 with bulk L2 prefetches of the operator stream a few batches
+ * ahead, 8 the tile's halo (positions and the CG vector) staged in shared
  * memory, rows and columns restricted to the nodes without a Dirichlet value of the
  * potential, 2-byte neighbour codes streamed and the bond weights recomputed from the
  * positions.  Chosen by the autotuner on the first run (0 / -1 before); nnpp_set_tuning pins

@@ -123,7 +123,7 @@ struct Engine {
   int spmv_variant = 0;     // FP32 CG operator: 0, 3 L1/L2 gathers (batches of 16, 8; 0 also
                             // in the one-launch inner solve),
                             // 1 bulk-copy staged, 2, 4 shared-memory windows (8, 16),
-                            // 5, 6, 7: 4, 3, 2 with L2 prefetch of the operator stream,
+                            // 5, 6, 7: 4, gathers (16), 2 with L2 prefetch of the stream,
                             // 8 tile halo in shared memory, weights recomputed
   int tr_variant = 0;       // FP32 transport: 0 neighbour records gathered from L1/L2 (the
                             // faster), 1 the tile's halo records staged in shared memory

@@ -642,8 +642,8 @@ __device__ __forceinline__ int code_node(const int* hb, unsigned int code) {
 // q = A z + beta q, p = z + beta p (so that q = A p), partial p.q -> alpha.
 // FP32, on the CG operator's slices (32 of a bin row's nodes without a potential Dirichlet
 // value; each row holds only its bonds to possible unknowns, in bond order, zero-padded to
-// the slice's longest; codes and weights column-major: one coalesced load per bond column),
-// one lane per row.  WIN: the warp first copies the slice's window (the z values of its 9 window rows)
+// the slice's longest, in quads of bond columns: a 16-byte and an 8-byte load a lane bring four
+// bonds), one lane per row.  WIN: the warp first copies the slice's window (the z values of its 9 window rows)
 // into its shared-memory buffer with asynchronous 16-byte copies and gathers from there (the
 // code's low 12 bits are the position in the window); otherwise it gathers from L1/L2.
 // PF > 0: lane 0 keeps bulk L2 prefetches of the warp's operator stream PF batches ahead of
@@ -3317,7 +3317,7 @@ __global__ void __launch_bounds__(kBlock) k_warm_apply(EngineView v) {
 
 // ---------------------------------------------------- potential residuals on the slices ----
 // Mixed path: the prep and the refinement residual as slice kernels over the sliced operator
-// (one lane per row, bond columns streamed in batches of 8, neighbour values gathered through
+// (one lane per row, two quads of bond columns a batch, neighbour values gathered through
 // L1/L2), with the FP64 weight carried as the FP32 pair (sell, sell_lo) and FP32-pair
 // arithmetic (TwoProd, TwoSum) along each row.  Slice partials, one global ticket; the last
 // CTA makes every instance's decisions.
@@ -4317,7 +4317,6 @@ __device__ __forceinline__ void transport_slice(const EngineView& v, int sg, int
       store_pair(v.partials, 5 * st + sg, ph_hi[4], ph_lo[4]);
       store_pair(v.partials, 6 * st + sg, ph_hi[5], ph_lo[5]);
       store_pair(v.partials, 7 * st + sg, (float)n_bad, 0.0f);
-      store_pair(v.partials, 8 * st + sg, 0.0f, 0.0f);
     }
   }
 }
@@ -5448,10 +5447,11 @@ nnpp_status prepare_kernels(int H, int B, int lanes) {
 }
 
 // FP32 CG operator variants without the staged ring (the autotuner's list): 0 L1/L2 gathers
-// in batches of 16, pipelined (the next batch's weights and codes in flight while the current
-// one gathers), 64 registers (32 warps per SM); 2 shared-memory windows, pipelined batches
-// of 8; 3 L1/L2 gathers in batches of 16 (40 warps per SM); 4 shared-memory windows, batches
-// of 16; 5, 6, 7: 4, 3, 2 with bulk L2 prefetches of the operator stream 3, 3, 4 batches ahead
+// in batches of 16 bond columns, pipelined (the next batch's weights and codes in flight while the
+// current one gathers), 79 registers (three CTAs an SM); 2 shared-memory windows, pipelined batches
+// of 8; 3 L1/L2 gathers in pipelined batches of 8, 48 registers (five CTAs an SM); 4 shared-memory
+// windows, batches of 16; 5, 6, 7: 4, gathers in batches of 16 and 2 with bulk L2 prefetches of the
+// operator stream 3, 3, 4 batches ahead
 template <int W>
 void launch_spmv_gather(int variant, const EngineView& v, int sms, cudaStream_t st) {
   switch (variant) {
