@@ -5661,8 +5661,8 @@ constexpr long long kSweepSlices = 152 * 4;
 // of other handles' threads run beside it.  Measured (ms a step of each handle, 1 / 8 threads): 8k nodes
 // 76 CTAs 0.284 / 0.88, 152 0.294 / 1.63; 22k 76 0.275 / 0.97, 114 0.266 / 1.29; 64k 114 0.396 / 2.48,
 // 152 0.394 / 3.10, 76 0.472 / 2.34.  (As launches that share the SMs: 0.64 / 1.03, 0.61 / 1.14 and
-// 0.76 / 2.54; from 125k nodes on eight threads' solves one after another are 10 to 16% slower than
-// launches were, 9.0 against 8.2 at 262k, one 44% faster.)
+// 0.76 / 2.54; from 125k nodes on eight threads' solves one after another are 5 to 16% slower than
+// launches were, 8.4 to 9.0 against 8.1 to 8.2 at 262k, one alone 1.09 against 1.64.)
 int sweep_grid(int sms, int slices, bool few) {
   const int part = few ? sms / 2 : sms * 3 / 4;
   return slices > part * (few ? 16 : 32) ? sms : std::max(1, part);
