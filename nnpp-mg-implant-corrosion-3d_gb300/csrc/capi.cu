@@ -102,6 +102,7 @@ struct StateBackup {
   DBuf<Rec64> rec64;
   DBuf<int> flip;
   DevState ds;
+  long long rebuilds;  // of the coarse operator
 };
 
 nnpp_status backup(Handle& h, StateBackup& b) {
@@ -122,12 +123,20 @@ nnpp_status backup(Handle& h, StateBackup& b) {
     NNPP_CUDA(cudaMemcpyAsync(b.xh.get(), h.xh.get(), h.xh.bytes(), cudaMemcpyDeviceToDevice, h.st));
     NNPP_CUDA(cudaMemcpyAsync(b.bh.get(), h.bh.get(), h.bh.bytes(), cudaMemcpyDeviceToDevice, h.st));
   }
+  b.rebuilds = h.coarse.rebuilds;
   NNPP_TRY(read_state(h, &b.ds));
   return NNPP_OK;
 }
 
 nnpp_status restore(Handle& h, StateBackup& b) {
   const size_t N = h.N;
+  // what the evaluation may have formed for its own phases: the operator's arrays (unknowns, diagonal, CG
+  // rows) and, where it was due, the coarse operator
+  b.ds.op_valid = 0;
+  if (h.coarse.rebuilds != b.rebuilds) {
+    b.ds.defl = 0;
+    h.coarse.stale = true;
+  }
   h.cur = b.cur;
   h.state_prec = b.prec;
   NNPP_CUDA(cudaMemcpyAsync(h.phi64.get(), b.phi.get(), sizeof(double) * N, cudaMemcpyDeviceToDevice, h.st));
